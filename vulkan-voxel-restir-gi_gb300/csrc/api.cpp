@@ -1091,7 +1091,6 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.jmeta = F.jmeta;
     a.hit_cap = (uint32_t)std::min<size_t>(2 * P, 0xFFFFFFF0u);
     a.counters = F.counters;
-    a.hit_count = a.counters + CNT_HITS;
     a.nlive = F.nlive;
     a.rec = F.rec;
     a.xv = F.xv;
@@ -1238,7 +1237,6 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
         at.hitval = Q.t_hitval;
         at.jmeta = Q.t_jmeta;
         at.hit_cap = 2 * a.train_cap;
-        at.hit_count = a.counters + CNT_HITS_TRAIN;
         // As on the main path, training bounce b's light-pdf walk runs on a
         // stream of its own beside bounce b + 1; bounce b + 2, which refills
         // the job buffers of parity b & 1, waits for it.

@@ -346,11 +346,70 @@ __device__ __forceinline__ void slab4(float4 NX, float4 FX, float4 NY, float4 FY
     cswap(tk[1], rk[1], tk[2], rk[2]);
 }
 
+// Work distribution of the persistent walks.  A returning atomicAdd by one
+// lane per warp on one word takes 0.66 ns chip-wide and, with every warp of
+// the chip queueing for it, 3.2 us each (311 K of them in 205 us).  So a warp
+// does not fetch at every refill: it owns a range of the queue and refills its
+// lanes from it.  Its first 32 entries are its static share (no atomic; a warp
+// past the queue's end leaves at once), then it takes chunks that shrink with
+// what is left (a quarter of its even share, 32 to 256 entries), so that the
+// last warps finish together.  The closest hits of a 640x480 frame's bounces:
+// 40 + 94 + 62 -> 33 + 70 + 45 us; of a 1080p frame's 125 + 332 + 382 -> 132 +
+// 269 + 361 us (chunks of at most 32: 134 + 274 + 358; at 3840x2160 548 + 1307
+// + 1657 us against 638 + 1376 + 1812 with 32).
+struct WarpRange {
+    uint32_t cur, end, last;  // the entries [cur, end) in hand; the end of the last chunk taken
+    bool more;                // the queue may hold entries past it
+};
+constexpr uint32_t CHUNK_MAX = 256;
+
+__device__ __forceinline__ WarpRange range_first(uint32_t n_in) {
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), all = gridDim.x * (blockDim.x >> 5);
+    WarpRange r;
+    r.cur = min(32u * w, n_in);
+    r.end = min(32u * w + 32u, n_in);
+    r.last = 32u * all;
+    r.more = r.last < n_in;
+    return r;
+}
+
+// the next chunk (all lanes; fetch counts the entries past the static shares)
+__device__ __forceinline__ void range_next(WarpRange &r, uint32_t n_in, uint32_t *fetch) {
+    const uint32_t all = gridDim.x * (blockDim.x >> 5);
+    const uint32_t size = min(((n_in - r.last) / (128u * all) + 1u) * 32u, CHUNK_MAX);
+    uint32_t base = 0;
+    if ((threadIdx.x & 31u) == 0) base = atomicAdd(fetch, size);
+    base = 32u * all + __shfl_sync(0xffffffffu, base, 0);
+    r.cur = min(base, n_in);
+    r.last = r.end = min(base + size, n_in);
+    r.more = r.end < n_in;
+}
+
+// Adds each warp's totals to N u64 counters, one atomic per CTA and counter:
+// the CTA's last warp to finish publishes the sums (s_sum: N + 1 words of
+// shared memory, zeroed before the walk).
+template <int N>
+__device__ __forceinline__ void publish_totals(uint32_t *s_sum, uint32_t *counters, const int (&at)[N],
+                                               const uint32_t (&v)[N]) {
+    if ((threadIdx.x & 31u) != 0) return;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+        if (v[k]) atomicAdd(s_sum + k, v[k]);
+    __threadfence_block();
+    if (atomicAdd(s_sum + N, 1u) != (blockDim.x >> 5) - 1u) return;
+    __threadfence_block();
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t t = atomicAdd(s_sum + k, 0u);
+        if (t) atomicAdd(reinterpret_cast<unsigned long long *>(counters + at[k]), (unsigned long long)t);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // k_trace: closest hit over the voxel faces (replaces getIntersectionInfo,
 // raytrace.rs:354-388).  Persistent warps; each lane owns one ray and, when
-// its traversal ends, takes a new ray from the bounce queue (warp-aggregated
-// fetch once a.refill_trace lanes are idle), so a warp does not wait for its
+// its traversal ends, takes a new ray from its warp's range of the bounce queue
+// (once a.refill_trace lanes are idle), so a warp does not wait for its
 // longest ray.  The result is independent of traversal order: ties on t go
 // to the smaller (instance, triangle) key and boxes are culled only when
 // strictly beyond the current best t.  In a batched frame each lane reads the
@@ -358,7 +417,7 @@ __device__ __forceinline__ void slab4(float4 NX, float4 FX, float4 NY, float4 FY
 // ---------------------------------------------------------------------------
 template <bool BATCH, bool MESH>
 __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs a, uint32_t b) {
-    const int lane = threadIdx.x & 31;
+    __shared__ uint32_t s_sum[4];
     const int REFILL = (int)a.refill_trace;
     const uint32_t n_in = (b == 0) ? a.n0 : a.counters[a.qsel ? CNT_TQUEUE : CNT_QUEUE + b];
     const uint32_t *qin = a.qsel ? a.tq : a.queue[(b + 1) & 1];
@@ -369,7 +428,10 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs
     const float4 *tris = a.v0.sc.tri_rec;
     uint32_t nblk = a.v0.sc.n_blk_rec;
     int root = a.v0.sc.geo_root;
-    bool has = false, exhausted = false;
+    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    WarpRange range = range_first(n_in);
+    bool has = false;
     uint32_t p = 0, steps = 0, traced = 0, n_nodes = 0, n_leaves = 0;
     f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oi = f3{0, 0, 0};
     float best_t = 0.0f, hb1 = 0.0f, hb2 = 0.0f;
@@ -383,14 +445,13 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs
     int2 stack[TRAV_STACK];
     while (true) {
         const uint32_t need = __ballot_sync(FULL, !has);
-        if (!exhausted && need && (__popc(need) >= REFILL || need == FULL)) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(fetch, (uint32_t)__popc(need));
-            base = __shfl_sync(FULL, base, 0);
-            if (base + (uint32_t)__popc(need) >= n_in) exhausted = true;
+        if ((range.cur < range.end || range.more) && need && (__popc(need) >= REFILL || need == FULL)) {
+            if (range.cur == range.end) range_next(range, n_in, fetch);
+            const uint32_t base = range.cur;
+            range.cur = min(base + (uint32_t)__popc(need), range.end);
             if (!has) {
                 const uint32_t idx = base + (uint32_t)__popc(need & lanemask_lt());
-                if (idx < n_in && (b == 0 ? bounce0_pixel<BATCH>(a, idx, p) : (p = qin[idx], true))) {
+                if (idx < range.end && (b == 0 ? bounce0_pixel<BATCH>(a, idx, p) : (p = qin[idx], true))) {
                     has = true;
                     traced++;
                     const ViewDev &V = view_of<BATCH>(a, p);
@@ -417,11 +478,16 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs
                 }
             }
         }
-        if (!__any_sync(FULL, has)) break;
-        if (has) {
-            bool done = (node == EMPTY_ROOT);
-            // descend through 4-wide inner nodes to the next leaf
-            while (!done && node >= 0) {
+        if (!__any_sync(FULL, has)) {
+            if (range.cur < range.end || range.more) continue;
+            break;
+        }
+        // descend through 4-wide inner nodes to the next leaf
+        bool done = has && (node == EMPTY_ROOT);
+        while (true) {
+            const bool inner = has && !done && node >= 0;
+            if (!__any_sync(FULL, inner)) break;
+            if (inner) {
                 const float4 *w = wide + 8 * (size_t)node;
                 const float4 NX = __ldg(w + px), FX = __ldg(w + (px ^ 1)), NY = __ldg(w + py);
                 const float4 FY = __ldg(w + (py ^ 1)), NZ = __ldg(w + pz), FZ = __ldg(w + (pz ^ 1));
@@ -448,6 +514,8 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs
                     done = true;
                 }
             }
+        }
+        if (has && (done || node < 0)) {
             if (MESH && !done && (uint32_t)(~node) >= nblk) {  // leaf: one world-space mesh triangle
                 const float4 *tr = tris + 3 * (size_t)((uint32_t)(~node) - nblk);
                 const float4 A = __ldg(tr), B = __ldg(tr + 1), C = __ldg(tr + 2);
@@ -500,11 +568,7 @@ __global__ void __launch_bounds__(128) k_trace(const __grid_constant__ FrameArgs
         n_nodes += __shfl_xor_sync(FULL, n_nodes, off);
         n_leaves += __shfl_xor_sync(FULL, n_leaves, off);
     }
-    if (lane == 0 && traced) {
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_RAYS), (unsigned long long)traced);
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_NODES), (unsigned long long)n_nodes);
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_LEAVES), (unsigned long long)n_leaves);
-    }
+    publish_totals<3>(s_sum, a.counters, {CNT_RAYS, CNT_NODES, CNT_LEAVES}, {traced, n_nodes, n_leaves});
 }
 
 // Shading of one path vertex (raytrace.rs:405-577): the hit's material
@@ -844,15 +908,12 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 const int4 hv = stash_hit, rc = stash_rc;
                 const int half = stash_half;
                 const size_t rb = (size_t)b * 2 * P;
-                if (anyj) {
-                    a.rec[rb + p] = make_float4(E.x, E.y, E.z, 0.0f);
-                    a.rec[rb + P + p] = make_float4(R.x, R.y, R.z, 0.0f);
-                } else {
-                    const float q = 0.0f * mis + (1.0f - mis) * inv2pi;
-                    const float w = pdf / q;
-                    a.rec[rb + p] = make_float4(E.x, E.y, E.z, w);
-                    a.rec[rb + P + p] = make_float4(R.x, R.y, R.z, q);
-                }
+                // the record without a light hit; a light-pdf job whose ray crosses
+                // lights gets its q and w from k_hit_eval / k_hit_sum
+                const float q = 0.0f * mis + (1.0f - mis) * inv2pi;
+                const float w = pdf / q;
+                a.rec[rb + p] = make_float4(E.x, E.y, E.z, w);
+                a.rec[rb + P + p] = make_float4(R.x, R.y, R.z, q);
                 if (b == 0) {
                     a.xv[p] = make_float4(new_o.x, new_o.y, new_o.z, 0.0f);
                     a.nv[p] = make_float4(n.x, n.y, n.z, 0.0f);
@@ -928,13 +989,14 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
 // The nee_pdf pass (nee_pdf.rs:281-337) for the queued rays, in three passes
 // so that each runs with coherent lanes:
 //   k_anyhit     every light triangle the ray crosses in [1e-4, 1000] is
-//                collected (persistent warps, per-lane job replacement), in
-//                ascending (instance, leaf) order; rays that cross none get
-//                their record here;
+//                collected in ascending (instance, leaf) order; a ray that
+//                crosses none (69% at 1080p) keeps the record its shading
+//                wrote for that case;
 //   k_hit_eval   one thread per hit: computeNeePdf (nee_pdf.rs:240-279) with
-//                its reverse walk up the light BVH;
-//   k_hit_sum    one thread per job: the sum in key order, then q and
-//                w = bsdf_pdf / q complete the bounce record.
+//                its reverse walk up the light BVH; a job's only hit (26% of
+//                the jobs) completes the bounce record: q and w = bsdf_pdf / q;
+//   k_hit_sum    one thread per job with several hits (5%): the sum in key
+//                order, then the record.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void finish_job(const FrameArgs &a, uint32_t b, uint32_t p, float pdf, float nee) {
     const float inv2pi = 1.0f / (2.0f * PI_F);
@@ -946,10 +1008,39 @@ __device__ __forceinline__ void finish_job(const FrameArgs &a, uint32_t b, uint3
     reinterpret_cast<float *>(a.rec + rb + a.P + p)[3] = q;
 }
 
+// a job's hits in ascending key order
+struct HitList {
+    uint64_t key[LIGHT_LIST];
+    float b1[LIGHT_LIST], b2[LIGHT_LIST];
+};
+__device__ __forceinline__ void hit_insert(HitList &L, int &nh, uint64_t key, float b1, float b2, uint32_t *err) {
+    if (nh >= LIGHT_LIST) {
+        atomicOr(err, ERR_LIGHT_LIST);
+        return;
+    }
+    int j = nh++;
+    while (j > 0 && L.key[j - 1] > key) {
+        L.key[j] = L.key[j - 1];
+        L.b1[j] = L.b1[j - 1];
+        L.b2[j] = L.b2[j - 1];
+        j--;
+    }
+    L.key[j] = key;
+    L.b1[j] = b1;
+    L.b2[j] = b2;
+}
+
+// Light-hit collection.  Every crossed light counts, so the order of the walk
+// is free: the walk visits inner nodes only and puts the lamps it reaches
+// aside; they are tested when the warp's walks have ended (or a lane's list is
+// full), and the hits of the jobs that ended take their slots with one atomic
+// per warp.  (Tested where they were found, with one atomic per job, the pass
+// ran 7.6 of 32 lanes per instruction.)
+constexpr int LAMP_LIST = 12;  // lamps a lane puts aside; a node adds up to 4
+
 template <bool CAPTURE, bool BATCH>
 __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ FrameArgs a, uint32_t b) {
-    // walk statistics, per lane: lamp nodes fetched, lamp blocks tested, light hits
-    __shared__ uint32_t s_stat[3][128];
+    __shared__ uint32_t s_sum[4];
     const int lane = threadIdx.x & 31;
     const int REFILL = (int)a.refill_any;
     const uint32_t n_in = a.counters[CNT_AQUEUE + b];
@@ -960,30 +1051,27 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
     const float4 *tris = a.v0.sc.tri_rec;
     int root = a.v0.sc.lamp_root;
     const float tmin = EPS_NEE, tmax = 1000.0f;
-    bool has = false, exhausted = false;
-    uint32_t p = 0, idx = 0, steps = 0;
+    bool has = false;
+    uint32_t p = 0, idx = 0, steps = 0, n_nodes = 0, n_leaves = 0, n_hits = 0;
     f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oi = f3{0, 0, 0};
-    float pdf = 0.0f;
-    int node = 0, sp = 0, nh = 0;
+    int node = EMPTY_ROOT, sp = 0, nh = 0, nl = 0;  // node < 0: the walk has ended
     int px = 0, py = 2, pz = 4;  // near-plane float4 per axis, picked by the ray's direction signs
-    int stack[TRAV_STACK];
-    uint64_t keys[LIGHT_LIST];
-    float b1s[LIGHT_LIST], b2s[LIGHT_LIST];
+    int stack[TRAV_STACK], lamps[LAMP_LIST];
+    HitList hits;
     if (blockIdx.x == 0 && threadIdx.x == 0 && n_in)
         atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_ANY), (unsigned long long)n_in);
-    s_stat[0][threadIdx.x] = 0;
-    s_stat[1][threadIdx.x] = 0;
-    s_stat[2][threadIdx.x] = 0;
+    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    WarpRange range = range_first(n_in);
     while (true) {
         const uint32_t need = __ballot_sync(FULL, !has);
-        if (!exhausted && need && (__popc(need) >= REFILL || need == FULL)) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&a.counters[CNT_AFETCH + b], (uint32_t)__popc(need));
-            base = __shfl_sync(FULL, base, 0);
-            if (base + (uint32_t)__popc(need) >= n_in) exhausted = true;
+        if ((range.cur < range.end || range.more) && need && (__popc(need) >= REFILL || need == FULL)) {
+            if (range.cur == range.end) range_next(range, n_in, &a.counters[CNT_AFETCH + b]);
+            const uint32_t base = range.cur;
+            range.cur = min(base + (uint32_t)__popc(need), range.end);
             if (!has) {
                 idx = base + (uint32_t)__popc(need & lanemask_lt());
-                if (idx < n_in) {
+                if (idx < range.end) {
                     has = true;
                     p = a.aqueue[b & 1][idx];
                     if constexpr (BATCH) {
@@ -994,10 +1082,8 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                         tris = V.sc.tri_rec;
                         root = V.sc.lamp_root;
                     }
-                    const float4 ro = a.ajob[b & 1][2 * (size_t)idx], rd = a.ajob[b & 1][2 * (size_t)idx + 1];
-                    o = ld3(ro);
-                    d = ld3(rd);
-                    pdf = rd.w;
+                    o = ld3(a.ajob[b & 1][2 * (size_t)idx]);
+                    d = ld3(a.ajob[b & 1][2 * (size_t)idx + 1]);
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
                     oi = f3{-o.x * inv.x, -o.y * inv.y, -o.z * inv.z};
                     px = signbit(inv.x) ? 1 : 0;
@@ -1006,17 +1092,23 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                     node = root;
                     sp = 0;
                     nh = 0;
+                    nl = 0;
                     steps = 0;
+                    if (root < 0 && root != EMPTY_ROOT) {  // one lamp, no inner node
+                        lamps[nl++] = ~root;
+                        node = EMPTY_ROOT;
+                    }
                 }
             }
         }
-        if (!__any_sync(FULL, has)) break;
-        if (has) {
-            bool done = (node == EMPTY_ROOT);
-            // 4-wide lamp nodes: every crossed light counts, so children are
-            // visited in slot order (no sorting); the first hit child is taken,
-            // the others pushed
-            while (!done && node >= 0) {
+        if (!__any_sync(FULL, has)) {
+            if (range.cur < range.end || range.more) continue;
+            break;
+        }
+        while (true) {
+            const bool inner = has && node >= 0 && nl <= LAMP_LIST - 4;
+            if (!__any_sync(FULL, inner)) break;
+            if (inner) {
                 const float4 *w = wide + 8 * (size_t)node;
                 const float4 NX = __ldg(w + px), FX = __ldg(w + (px ^ 1)), NY = __ldg(w + py);
                 const float4 FY = __ldg(w + (py ^ 1)), NZ = __ldg(w + pz), FZ = __ldg(w + (pz ^ 1));
@@ -1034,7 +1126,9 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                     const float tf = fmin3(__fmaf_rn(fx[i], inv.x, oi.x), __fmaf_rn(fy[i], inv.y, oi.y),
                                            fminf(__fmaf_rn(fz[i], inv.z, oi.z), tmax));
                     if (tn <= tf) {  // (an unused slot's inverted box is never entered)
-                        if (next == EMPTY_ROOT) {
+                        if (rf[i] < 0) {
+                            lamps[nl++] = ~rf[i];
+                        } else if (next == EMPTY_ROOT) {
                             next = rf[i];
                         } else if (sp < TRAV_STACK) {
                             stack[sp++] = rf[i];
@@ -1043,107 +1137,81 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                         }
                     }
                 }
-                if (next != EMPTY_ROOT) node = next;
-                else if (sp == 0) done = true;
-                else node = stack[--sp];
-                if (++steps > TRAV_GUARD) {
+                if (next == EMPTY_ROOT && sp > 0) next = stack[--sp];
+                node = next;
+                if (++steps > TRAV_GUARD) {  // only reachable with a malformed layout
                     atomicOr(err, ERR_GUARD);
-                    done = true;
+                    node = EMPTY_ROOT;
                 }
-            }
-            if (!done) {  // leaf: one lamp block; each emissive face hit names one light triangle
-                s_stat[1][threadIdx.x]++;
-                const int4 r = __ldg(recs + (~node));
-                const int wx = rec_wx(r), wy = rec_wy(r), wz = rec_wz(r);
-                const uint32_t ii = rec_inst(r);
-                if (r.z < 0) {  // a mesh light triangle: (leaf, world-space triangle record) in the table
-                    const uint32_t leaf = __ldg(table + r.w), t = __ldg(table + r.w + 1);
-                    const float4 *q = tris + 3 * (size_t)t;
-                    TriHit th;
-                    if (tri_test(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2)), o, d, tmin, tmax, th)) {
-                        const uint64_t key = ((uint64_t)ii << 32) | leaf;
-                        if (nh < LIGHT_LIST) {
-                            int j = nh++;
-                            while (j > 0 && keys[j - 1] > key) {
-                                keys[j] = keys[j - 1];
-                                b1s[j] = b1s[j - 1];
-                                b2s[j] = b2s[j - 1];
-                                j--;
-                            }
-                            keys[j] = key;
-                            b1s[j] = th.b1;
-                            b2s[j] = th.b2;
-                        } else {
-                            atomicOr(err, ERR_LIGHT_LIST);
-                        }
-                    }
-                }
-                for (uint32_t fm = r.z < 0 ? 0u : (uint32_t)r.z; fm; fm &= fm - 1u) {
-                    const int f = __ffs(fm) - 1;
-                    FaceHit fh;
-                    if (!face_test(wx, wy, wz, f, o, d, inv, tmin, tmax, fh)) continue;
-                    const uint32_t leaf = __ldg(table + r.w + 2 * f + fh.half);
-                    if (leaf == INVALID) continue;
-                    const uint64_t key = ((uint64_t)ii << 32) | leaf;
-                    if (nh < LIGHT_LIST) {
-                        int j = nh++;
-                        while (j > 0 && keys[j - 1] > key) {
-                            keys[j] = keys[j - 1];
-                            b1s[j] = b1s[j - 1];
-                            b2s[j] = b2s[j - 1];
-                            j--;
-                        }
-                        keys[j] = key;
-                        b1s[j] = fh.b1;
-                        b2s[j] = fh.b2;
-                    } else {
-                        atomicOr(err, ERR_LIGHT_LIST);
-                    }
-                }
-                if (sp == 0) done = true;
-                else node = stack[--sp];
-            }
-            if (done) {
-                s_stat[0][threadIdx.x] += steps;
-                s_stat[2][threadIdx.x] += (uint32_t)nh;
-                uint32_t hb = 0;
-                if (nh > 0) {
-                    hb = atomicAdd(a.hit_count, (uint32_t)nh);
-                    if (hb + (uint32_t)nh > a.hit_cap) {
-                        atomicOr(err, ERR_LIGHT_LIST);
-                        nh = 0;
-                    }
-                }
-                if (nh == 0) {
-                    finish_job(a, b, p, pdf, 0.0f);
-                    if (CAPTURE) a.c_nee[(size_t)b * a.P + p] = 0.0f;
-                } else {
-                    for (int j = 0; j < nh; j++) {
-                        a.hitbuf[2 * (size_t)(hb + j)] =
-                            make_uint4(p, (uint32_t)(keys[j] >> 32), (uint32_t)keys[j], __float_as_uint(b1s[j]));
-                        a.hitbuf[2 * (size_t)(hb + j) + 1] = make_uint4(__float_as_uint(b2s[j]), idx, 0u, 0u);
-                    }
-                }
-                a.jmeta[idx] = make_uint2(hb, (uint32_t)nh);
-                has = false;
             }
         }
+        while (has && nl > 0) {  // one lamp; each emissive face hit names one light triangle
+            n_leaves++;
+            const int4 r = __ldg(recs + lamps[--nl]);
+            const int wx = rec_wx(r), wy = rec_wy(r), wz = rec_wz(r);
+            const uint64_t ikey = (uint64_t)rec_inst(r) << 32;
+            if (r.z < 0) {  // a mesh light triangle: (leaf, world-space triangle record) in the table
+                const uint32_t leaf = __ldg(table + r.w), t = __ldg(table + r.w + 1);
+                const float4 *q = tris + 3 * (size_t)t;
+                TriHit th;
+                if (tri_test(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2)), o, d, tmin, tmax, th))
+                    hit_insert(hits, nh, ikey | leaf, th.b1, th.b2, err);
+                continue;
+            }
+            for (uint32_t fm = (uint32_t)r.z; fm; fm &= fm - 1u) {
+                const int f = __ffs(fm) - 1;
+                FaceHit fh;
+                if (!face_test(wx, wy, wz, f, o, d, inv, tmin, tmax, fh)) continue;
+                const uint32_t leaf = __ldg(table + r.w + 2 * f + fh.half);
+                if (leaf != INVALID) hit_insert(hits, nh, ikey | leaf, fh.b1, fh.b2, err);
+            }
+        }
+        const bool done = has && node < 0;
+        const uint32_t cnt = done ? (uint32_t)nh : 0u;
+        const uint32_t multi = __ballot_sync(FULL, cnt > 1);
+        if (__any_sync(FULL, cnt > 0)) {
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int k = 1; k < 32; k <<= 1) {
+                const uint32_t up = __shfl_up_sync(FULL, incl, k);
+                if (lane >= k) incl += up;
+            }
+            unsigned long long at = 0;
+            if (lane == 31)
+                at = atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_HITS + 2 * b),
+                               ((unsigned long long)__popc(multi) << 32) | incl);
+            at = __shfl_sync(FULL, at, 31);
+            const uint32_t hb = (uint32_t)at + incl - cnt;
+            const bool fits = hb + cnt <= a.hit_cap;
+            if (!fits) atomicOr(err, ERR_LIGHT_LIST);
+            for (uint32_t j = 0; j < cnt && hb + j < a.hit_cap; j++) {
+                a.hitbuf[2 * (size_t)(hb + j)] =
+                    make_uint4(p, (uint32_t)(hits.key[j] >> 32), (uint32_t)hits.key[j], __float_as_uint(hits.b1[j]));
+                a.hitbuf[2 * (size_t)(hb + j) + 1] = make_uint4(__float_as_uint(hits.b2[j]), idx, fits ? cnt : 0u, 0u);
+            }
+            // the jobs with several hits, for the sum (a job past the hit
+            // buffer's end has none to sum)
+            if (cnt > 1)
+                a.jmeta[(uint32_t)(at >> 32) + __popc(multi & lanemask_lt())] = make_uint2(hb, fits ? cnt : 0u);
+            n_hits += cnt;
+        }
+        if (done) {
+            n_nodes += steps;
+            has = false;
+        }
     }
-    const uint32_t n_nodes = __reduce_add_sync(FULL, s_stat[0][threadIdx.x]);
-    const uint32_t n_leaves = __reduce_add_sync(FULL, s_stat[1][threadIdx.x]);
-    const uint32_t n_hits = __reduce_add_sync(FULL, s_stat[2][threadIdx.x]);
-    if (lane == 0 && n_nodes) {
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_ANODES), (unsigned long long)n_nodes);
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_ALEAVES), (unsigned long long)n_leaves);
-        atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_AHITS), (unsigned long long)n_hits);
-    }
+    n_nodes = __reduce_add_sync(FULL, n_nodes);
+    n_leaves = __reduce_add_sync(FULL, n_leaves);
+    n_hits = __reduce_add_sync(FULL, n_hits);
+    publish_totals<3>(s_sum, a.counters, {CNT_ANODES, CNT_ALEAVES, CNT_AHITS}, {n_nodes, n_leaves, n_hits});
 }
 
-template <bool BATCH>
+template <bool CAPTURE, bool BATCH>
 __global__ void __launch_bounds__(128) k_hit_eval(const __grid_constant__ FrameArgs a, uint32_t b) {
-    const uint32_t n = min(*a.hit_count, a.hit_cap);
+    const uint32_t n = min(a.counters[CNT_HITS + 2 * b], a.hit_cap);
     for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
         const uint4 A = a.hitbuf[2 * (size_t)h], B = a.hitbuf[2 * (size_t)h + 1];
+        if (B.z == 0) continue;  // of a job that did not fit the hit buffer
         const uint32_t p = A.x;
         const float4 ro = a.ajob[b & 1][2 * (size_t)B.y], rd = a.ajob[b & 1][2 * (size_t)B.y + 1];
         const DevScene &sc = view_of<BATCH>(a, p).sc;
@@ -1157,20 +1225,27 @@ __global__ void __launch_bounds__(128) k_hit_eval(const __grid_constant__ FrameA
             const float4 *q = sc.tri_rec + 3 * (size_t)((uint32_t)fw & 0x7FFFFFFFu);
             n3 = tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2))).n;
         }
-        a.hitval[h] = nee_pdf_of(sc, ld3(ro), n3, ld3(rd), A.y, A.z, __uint_as_float(A.w), __uint_as_float(B.x));
+        const float v = nee_pdf_of(sc, ld3(ro), n3, ld3(rd), A.y, A.z, __uint_as_float(A.w), __uint_as_float(B.x));
+        if (B.z > 1) {
+            a.hitval[h] = v;
+        } else {
+            const float nee = 0.0f + v;  // the sum from 0 in key order
+            finish_job(a, b, p, rd.w, nee);
+            if (CAPTURE) a.c_nee[(size_t)b * a.P + p] = nee;
+        }
     }
 }
 
 template <bool CAPTURE>
 __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameArgs a, uint32_t b) {
-    const uint32_t n_in = a.counters[CNT_AQUEUE + b];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x) {
+    const uint32_t n = a.counters[CNT_HITS + 2 * b + 1];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint2 m = a.jmeta[i];
         if (m.y == 0) continue;
-        const uint32_t p = a.aqueue[b & 1][i];
+        const uint32_t p = a.hitbuf[2 * (size_t)m.x].x, idx = a.hitbuf[2 * (size_t)m.x + 1].y;
         float nee = 0.0f;
         for (uint32_t j = 0; j < m.y; j++) nee += a.hitval[m.x + j];
-        finish_job(a, b, p, a.ajob[b & 1][2 * (size_t)i + 1].w, nee);
+        finish_job(a, b, p, a.ajob[b & 1][2 * (size_t)idx + 1].w, nee);
         if (CAPTURE) a.c_nee[(size_t)b * a.P + p] = nee;
     }
 }
@@ -1309,11 +1384,11 @@ vrg_status launch_light_pdf(cudaStream_t s, const FrameArgs &a, uint32_t b, uint
     if (batch) k_anyhit<false, true><<<ga, 128, 0, s>>>(a, b);
     else if (a.capture) k_anyhit<true, false><<<ga, 128, 0, s>>>(a, b);
     else k_anyhit<false, false><<<ga, 128, 0, s>>>(a, b);
-    if (batch) k_hit_eval<true><<<gs, 128, 0, s>>>(a, b);
-    else k_hit_eval<false><<<gs, 128, 0, s>>>(a, b);
+    if (batch) k_hit_eval<false, true><<<gs, 128, 0, s>>>(a, b);
+    else if (a.capture) k_hit_eval<true, false><<<gs, 128, 0, s>>>(a, b);
+    else k_hit_eval<false, false><<<gs, 128, 0, s>>>(a, b);
     if (a.capture) k_hit_sum<true><<<gs, 128, 0, s>>>(a, b);
     else k_hit_sum<false><<<gs, 128, 0, s>>>(a, b);
-    VRG_CUDA_TRY(cudaMemsetAsync(a.hit_count, 0, 4, s));
     VRG_CUDA_TRY(cudaGetLastError());
     return VRG_OK;
 }

@@ -18,14 +18,14 @@ constexpr int CNT_AFETCH = 32;   // [32..39] any-hit work-fetch cursor of bounce
 constexpr int CNT_SFETCH = 40;   // [40..47] shading work-fetch cursor of bounce b
 constexpr int CNT_NODES = 50;    // u64 at words 50-51: inner nodes fetched by k_trace
 constexpr int CNT_LEAVES = 52;   // u64 at words 52-53: leaf records tested by k_trace
-constexpr int CNT_HITS = 54;     // light hits collected by k_anyhit for the current bounce
-constexpr int CNT_HITS_TRAIN = 55;  // the same for a cache frame's training branch (its own job and hit buffers)
+constexpr int CNT_HITS = 64;     // [64..79] per bounce b, one u64: light hits collected by k_anyhit (word 64 + 2b)
+                                 // and jobs with several (word 65 + 2b)
 constexpr int CNT_ANODES = 56;   // u64 at words 56-57: 4-wide lamp nodes fetched by k_anyhit
 constexpr int CNT_ALEAVES = 58;  // u64 at words 58-59: lamp-block records tested by k_anyhit
 constexpr int CNT_AHITS = 60;    // u64 at words 60-61: light hits collected by k_anyhit
 constexpr int CNT_INFER = 48;    // radiance-cache queries of the frame
 constexpr int CNT_TRAIN = 49;    // radiance-cache training paths of the frame
-constexpr int CNT_WORDS = 64;
+constexpr int CNT_WORDS = 80;
 constexpr int MAX_BOUNCES = 8;
 
 // One camera view of one scene.  A frame renders either one view (the
@@ -81,11 +81,10 @@ struct FrameArgs {
     // the pixel, and a copy of its ray (origin | face, direction | bsdf pdf)
     uint32_t *aqueue[2];
     float4 *ajob[2];              // 2 float4 per job
-    uint4 *hitbuf;                // light hits: (pixel, instance, leaf, b1 bits), then (b2 bits, 0, 0, 0)
+    uint4 *hitbuf;                // light hits: (pixel, instance, leaf, b1 bits), then (b2 bits, job, the job's hits, 0)
     float *hitval;                // light-sampling pdf of each hit
-    uint2 *jmeta;                 // per any-hit job: (first hit, hit count)
+    uint2 *jmeta;                 // per any-hit job with several hits: (first hit, hit count)
     uint32_t hit_cap;
-    uint32_t *hit_count;          // the hits collected for the current bounce (a counter word)
     int4 *hits;                   // closest hit per pixel: (~record or -1, face|half<<3, b1, b2)
     uint32_t *counters;
     uint8_t *nlive;
