@@ -234,20 +234,67 @@ __global__ void k_tri_records(const InstBuild *inst, uint32_t n_inst, uint32_t n
     }
 }
 
-// The light-BLAS nodes of an instance whose transform is not a translation,
-// with min and max replaced by the transform applied to them: the v000 and
-// v111 of nodeImportance (raytrace.rs:184-185, nee_pdf.rs:127-128), computed
-// once here so the light walks move these nodes by a zero translation
-__global__ void k_xform_light_nodes(const vrg_bvh_node *in, uint32_t n, float4 r0, float4 r1, float4 r2,
-                                    vrg_bvh_node *out) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    vrg_bvh_node nd = in[j];
-    const f3 a = xf_rows(r0, r1, r2, f3{nd.min[0], nd.min[1], nd.min[2]});
-    const f3 b = xf_rows(r0, r1, r2, f3{nd.max[0], nd.max[1], nd.max[2]});
-    nd.min[0] = a.x; nd.min[1] = a.y; nd.min[2] = a.z;
-    nd.max[0] = b.x; nd.max[1] = b.y; nd.max[2] = b.z;
-    out[j] = nd;
+// min and max of a light node under its instance's transform: the v000 and
+// v111 of nodeImportance (raytrace.rs:184-185, nee_pdf.rs:127-128)
+__device__ __forceinline__ void light_box(const vrg_bvh_node &n, const InstBuild *I, f3 &lo, f3 &hi) {
+    lo = f3{n.min[0], n.min[1], n.min[2]};
+    hi = f3{n.max[0], n.max[1], n.max[2]};
+    f3 t = f3{0.0f, 0.0f, 0.0f};
+    if (I && (I->flags & INST_XFORM)) {
+        const float4 r0 = make_float4(I->m[0], I->m[1], I->m[2], I->m[3]);
+        const float4 r1 = make_float4(I->m[4], I->m[5], I->m[6], I->m[7]);
+        const float4 r2 = make_float4(I->m[8], I->m[9], I->m[10], I->m[11]);
+        lo = xf_rows(r0, r1, r2, lo);
+        hi = xf_rows(r0, r1, r2, hi);
+    } else if (I) {
+        t = f3{I->off[0], I->off[1], I->off[2]};
+    }
+    lo = add3(lo, t);
+    hi = add3(hi, t);
+}
+
+// the light tree's walk layout (DevScene::light_pair, light_par), one thread
+// per node of [top level | BLASes]; a node writes its children's parents
+__global__ void k_light_pairs(const vrg_bvh_node *tl, uint32_t n_tl, const InstBuild *inst, uint32_t n_inst,
+                              uint32_t n_total, float4 *pair, uint32_t *par) {
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n_total) return;
+    const InstBuild *I = nullptr;  // null: a node of the top level
+    const vrg_bvh_node *root = tl;
+    uint32_t base = 0;
+    if (g >= n_tl) {
+        I = &inst[inst_of(inst, n_inst, g, [](const InstBuild &J) { return J.wbase; })];
+        root = I->bl;
+        base = I->wbase;
+    }
+    const vrg_bvh_node &nd = root[g - base];
+    if (g == 0) par[0] = INVALID;
+    f3 lo[2] = {}, hi[2] = {};
+    float power[2] = {0.0f, 0.0f};
+    int ref[2] = {EMPTY_ROOT, EMPTY_ROOT};
+    if (nd.left_node_idx != INVALID) {
+        const uint32_t ch[2] = {nd.left_node_idx, nd.right_node_idx_or_prim_idx};
+        for (uint32_t s = 0; s < 2; s++) {
+            const vrg_bvh_node &c = root[ch[s]];
+            const bool leaf = c.left_node_idx == INVALID;
+            light_box(c, I, lo[s], hi[s]);
+            power[s] = c.power;
+            if (leaf) ref[s] = ~(int)(I ? ch[s] : c.right_node_idx_or_prim_idx);
+            else ref[s] = (int)(base + ch[s]);
+            par[base + ch[s]] = (g << 1) | s;
+            if (!I && leaf) par[inst[c.right_node_idx_or_prim_idx].wbase] = (g << 1) | s;
+        }
+    } else if (!I) {
+        const InstBuild &J = inst[nd.right_node_idx_or_prim_idx];
+        light_box(J.bl[0], &J, lo[0], hi[0]);
+        power[0] = J.bl[0].power;
+        if (g == 0) par[J.wbase] = INVALID;  // the only light instance
+    }
+    float4 *q = pair + LIGHT_PAIR * (size_t)g;
+    q[0] = make_float4(lo[0].x, lo[1].x, lo[0].y, lo[1].y);
+    q[1] = make_float4(lo[0].z, lo[1].z, hi[0].x, hi[1].x);
+    q[2] = make_float4(hi[0].y, hi[1].y, hi[0].z, hi[1].z);
+    q[3] = make_float4(power[0], power[1], __int_as_float(ref[0]), __int_as_float(ref[1]));
 }
 
 // world-space light-triangle records of every instance, one thread per light
@@ -564,8 +611,7 @@ struct CommitPrep {
     uint32_t max_levels = 0;
     DevBufPtr buf;
     uint8_t *B = nullptr;
-    uint64_t o_gw = 0, o_gr = 0, o_tr = 0, o_lr = 0, o_tln = 0, o_inst = 0, o_gb = 0, o_lb = 0, o_xln = 0;
-    uint64_t xf_light_nodes = 0;     // light-BLAS nodes of the instances with a transform that is not a translation
+    uint64_t o_gw = 0, o_gr = 0, o_tr = 0, o_lr = 0, o_tln = 0, o_inst = 0, o_gb = 0, o_lb = 0, o_lp = 0, o_lpar = 0;
     uint32_t tl_prim_off = 0, tl_node_off = 0;  // in the shared top-level build
     uint64_t lamp_off = 0;                      // in the shared lamp build
     uint32_t n_lamps = 0;
@@ -703,7 +749,6 @@ vrg_status commit_prepare(Scene *sc, CommitPrep &cp) {
         l.refbase = l.rbase;
         light_nodes += cs.n_light ? 2 * (uint64_t)cs.n_light - 1 : 0;
         cp.light_recs += cs.n_light;
-        if (!sc->inst_tonly[i] && cs.n_light) cp.xf_light_nodes += 2 * (uint64_t)cs.n_light - 1;
         cp.max_levels = std::max(cp.max_levels, o->levels);
     }
     cp.n_light_nodes_all = light_nodes;
@@ -717,7 +762,8 @@ vrg_status commit_prepare(Scene *sc, CommitPrep &cp) {
     cp.o_gw = o; o += al(cp.n_geo_wide * 128);
     cp.o_gr = o; o += al(cp.geo_recs * 16);
     cp.o_tr = o; o += al(cp.tri_recs * 48);
-    cp.o_xln = o; o += al(cp.xf_light_nodes * sizeof(vrg_bvh_node));
+    cp.o_lp = o; o += al((cp.n_light_tl + light_nodes) * LIGHT_PAIR * 16);
+    cp.o_lpar = o; o += al((cp.n_light_tl + light_nodes) * 4);
     cp.o_lr = o; o += al(cp.light_recs * 16);
     cp.o_tln = o; o += al((uint64_t)(cp.n_light_tl + cp.n_geo_tl) * sizeof(vrg_bvh_node));
     cp.o_inst = o; o += al((uint64_t)ni * sizeof(InstDev));
@@ -814,34 +860,22 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
     uint8_t *B = cp.B;
     // instance table (prim2node, scene.rs:282-287)
     std::vector<InstDev> idev(ni);
-    uint64_t xln = 0;
     for (uint32_t i = 0; i < ni; i++) {
         const Object *ob = sc->inst_objs[i];
-        for (int a = 0; a < 3; a++) idev[i].off[a] = sc->inst_off[i][a];
-        idev[i].light_bvh_tl_idx = 0;
-        idev[i].light_bl = ob->light_nodes;
+        const bool xf_light = !sc->inst_tonly[i] && ob->sum.n_light;  // (its light nodes carry the transform)
+        for (int a = 0; a < 3; a++) idev[i].off[a] = xf_light ? 0.0f : sc->inst_off[i][a];
+        idev[i].light_tl = 0;
         idev[i].light_leaf_tri = ob->light_leaf_tri;
         idev[i].flags = cp.gb[i].flags;
         idev[i].tri_base = cp.gb[i].tbase;
         idev[i].uv = ob->mesh_uv;
-        if (!sc->inst_tonly[i] && ob->sum.n_light) {
-            // the light walks read this instance's nodes already transformed
-            const uint32_t nn = 2 * ob->sum.n_light - 1;
-            const float *m = sc->inst_xf[i].data();
-            vrg_bvh_node *dst = (vrg_bvh_node *)(B + cp.o_xln) + xln;
-            k_xform_light_nodes<<<(nn + 127) / 128, 128, 0, s>>>(
-                ob->light_nodes, nn, make_float4(m[0], m[1], m[2], m[3]), make_float4(m[4], m[5], m[6], m[7]),
-                make_float4(m[8], m[9], m[10], m[11]), dst);
-            VRG_CUDA_TRY(cudaGetLastError());
-            idev[i].light_bl = dst;
-            idev[i].off[0] = idev[i].off[1] = idev[i].off[2] = 0.0f;
-            xln += nn;
-        }
+        idev[i].light_base = cp.lb[i].wbase;
+        idev[i].light_leaf = ob->sum.n_light == 1 ? 1u : 0u;
     }
     if (cp.n_light_inst)
         for (uint32_t j = 0; j < cp.n_light_tl; j++)
             if (sc->h_light_tl[j].left_node_idx == INVALID)
-                idev[sc->h_light_tl[j].right_node_idx_or_prim_idx].light_bvh_tl_idx = j;
+                idev[sc->h_light_tl[j].right_node_idx_or_prim_idx].light_tl = j;
     if (ni) {
         VRG_CUDA_TRY(cudaMemcpyAsync(B + cp.o_inst, idev.data(), ni * sizeof(InstDev), cudaMemcpyHostToDevice, s));
         VRG_CUDA_TRY(cudaMemcpyAsync(B + cp.o_gb, cp.gb.data(), ni * sizeof(InstBuild), cudaMemcpyHostToDevice, s));
@@ -852,6 +886,12 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
         k_wide4<<<(uint32_t)((cp.n_geo_wide + 255) / 256), 256, 0, s>>>(d_tl + cp.n_light_tl, cp.n_geo_tl, d_gb, ni,
                                                                        (uint32_t)cp.n_geo_wide,
                                                                        (float4 *)(B + cp.o_gw));
+        VRG_CUDA_TRY(cudaGetLastError());
+    }
+    if (cp.n_light_inst) {
+        const uint32_t n = (uint32_t)(cp.n_light_tl + cp.n_light_nodes_all);
+        k_light_pairs<<<(n + 127) / 128, 128, 0, s>>>(d_tl, cp.n_light_tl, d_lb, ni, n, (float4 *)(B + cp.o_lp),
+                                                      (uint32_t *)(B + cp.o_lpar));
         VRG_CUDA_TRY(cudaGetLastError());
     }
     if (cp.geo_recs) {
@@ -874,7 +914,11 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
     D.tri_rec = (const float4 *)(B + cp.o_tr);
     D.n_blk_rec = (uint32_t)cp.geo_recs;
     D.n_tri_rec = (uint32_t)cp.tri_recs;
-    D.light_tl = d_tl;
+    D.light_pair = (const float4 *)(B + cp.o_lp);
+    D.light_par = (const uint32_t *)(B + cp.o_lpar);
+    const vrg_bvh_node &lr = sc->h_light_tl[0];
+    D.light_root = !cp.n_light_inst ? EMPTY_ROOT
+                   : lr.left_node_idx != INVALID ? 0 : ~(int)lr.right_node_idx_or_prim_idx;
     D.inst = (const InstDev *)(B + cp.o_inst);
     D.mats = (const vrg_material *)sc->ctx->d_mats->ptr;
     D.n_inst = ni;

@@ -27,27 +27,6 @@ __constant__ Frame c_frames[12];
 
 namespace {
 
-struct NodeV {
-    uint32_t left, right;
-    f3 mn;
-    float power;
-    f3 mx;
-    uint32_t parent;
-};
-
-__device__ __forceinline__ NodeV ldnode(const vrg_bvh_node *n) {
-    const float2 *p = reinterpret_cast<const float2 *>(n);
-    float2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3), e = __ldg(p + 4);
-    NodeV r;
-    r.left = __float_as_uint(a.x);
-    r.right = __float_as_uint(a.y);
-    r.mn = f3{b.x, b.y, c.x};
-    r.power = c.y;
-    r.mx = f3{d.x, d.y, e.x};
-    r.parent = __float_as_uint(e.y);
-    return r;
-}
-
 // The shading point's part of nodeImportance, the same for every node of a
 // walk, worked out once per walk (the descent and the reverse walk are
 // bound by instruction issue; this took the 1080p frame from 1.114 to 1.086
@@ -78,42 +57,69 @@ __device__ __forceinline__ ImpPt imp_point(f3 point, f3 normal) {
     return P;
 }
 
+// Packed binary32 arithmetic, one rounding per component: fused
+// multiply-adds only.  (A packed product followed by a packed sum is
+// contracted into one by the assembler, with .rn and without -fmad, so sums
+// of products stay scalar.)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+// (x*x + y*y) + z*z per component
+__device__ __forceinline__ float2 sq3(float2 x, float2 y, float2 z) {
+    return make_float2(dot3(f3{x.x, y.x, z.x}, f3{x.x, y.x, z.x}), dot3(f3{x.y, y.y, z.y}, f3{x.y, y.y, z.y}));
+}
+
 // nodeImportance (raytrace.rs:181-208: uint visibility, EPS 1e-3;
-// nee_pdf.rs:125-152: float visibility, EPS 1e-4).  v000 and v111 are the
-// instance transform applied to the node's min and max; the 8 corners are the
-// axis-aligned box they span (as in the reference, not the transformed box).
-// An instance moves its light-BLAS nodes by the translation off here; an
-// instance with any other transform has its nodes' min and max transformed
-// once at commit (its off is 0), which gives the same importance bits.
+// nee_pdf.rs:125-152: float visibility, EPS 1e-4) of both children of light
+// node g.  The 8 corners are the axis-aligned box that v000 and v111 span (as
+// in the reference, not the transformed box).  The centre's 0.5 * (v000 +
+// v111) is exact, so the fused subtraction of the point rounds as the
+// separate one does.
+struct LightPair {
+    float2 imp;      // importance of (left, right)
+    int left, right; // refs
+};
 template <bool NEE>
-__device__ __forceinline__ float node_importance(const ImpPt &P, const float off[3], const NodeV &n) {
+__device__ __forceinline__ LightPair light_pair(const DevScene &sc, const ImpPt &P, uint32_t g) {
+    const float4 *q = sc.light_pair + LIGHT_PAIR * (size_t)g;
+    const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
+    const float2 lx = make_float2(a.x, a.y), ly = make_float2(a.z, a.w), lz = make_float2(b.x, b.y);
+    const float2 hx = make_float2(b.z, b.w), hy = make_float2(c.x, c.y), hz = make_float2(c.z, c.w);
     const f3 point = P.point, normal = P.normal;
-    f3 v000 = f3{n.mn.x + off[0], n.mn.y + off[1], n.mn.z + off[2]};
-    f3 v111 = f3{n.mx.x + off[0], n.mx.y + off[1], n.mx.z + off[2]};
-    f3 e = sub3(v111, v000);
-    f3 cc = sub3(lscl3(0.5f, add3(v000, v111)), point);
-    float dist_sq = fmaxf(dot3(e, e), dot3(cc, cc));
     const float eps = NEE ? EPS_NEE : EPS_TRACE;
+    const float2 half = make_float2(0.5f, 0.5f);
+    const float2 ee = sq3(sub2(hx, lx), sub2(hy, ly), sub2(hz, lz));
+    const float2 cc = sq3(__ffma2_rn(half, __fadd2_rn(lx, hx), make_float2(-point.x, -point.x)),
+                          __ffma2_rn(half, __fadd2_rn(ly, hy), make_float2(-point.y, -point.y)),
+                          __ffma2_rn(half, __fadd2_rn(lz, hz), make_float2(-point.z, -point.z)));
+    const float dl = fmaxf(ee.x, cc.x), dr = fmaxf(ee.y, cc.y);
+    float vl, vr;  // the visible share of the corners
     if (P.ax >= 0) {
+        // voxel-face normal: the corners' two distances along its axis, 4
+        // corners each; (v - pa) * sign rounds as v - pa
         const int ax = P.ax & 3;
-        float dlo = cmp3(v000, ax) - P.pa, dhi = cmp3(v111, ax) - P.pa;
-        if (P.ax & 4) { dlo = -dlo; dhi = -dhi; }
-        const uint32_t visible = (dlo >= eps ? 4u : 0u) + (dhi >= eps ? 4u : 0u);
-        if (!NEE) return n.power / dist_sq * ((float)visible / 8.0f);
-        return n.power / dist_sq * ((float)visible * 0.125f);  // = the sum of 0.125 terms, exact
-    }
-    f3 c[8] = {v000, f3{v000.x, v000.y, v111.z}, f3{v000.x, v111.y, v000.z}, f3{v000.x, v111.y, v111.z},
-               f3{v111.x, v000.y, v000.z}, f3{v111.x, v000.y, v111.z}, f3{v111.x, v111.y, v000.z}, v111};
-    if (!NEE) {
-        uint32_t visible = 0;
+        const float sg = (P.ax & 4) ? -1.0f : 1.0f;
+        const float2 lo = ax == 0 ? lx : (ax == 1 ? ly : lz), hi = ax == 0 ? hx : (ax == 1 ? hy : hz);
+        const float2 s2 = make_float2(sg, sg), o2 = make_float2(-sg * P.pa, -sg * P.pa);
+        const float2 u = __ffma2_rn(lo, s2, o2), v = __ffma2_rn(hi, s2, o2);
+        vl = (u.x >= eps ? 0.5f : 0.0f) + (v.x >= eps ? 0.5f : 0.0f);
+        vr = (u.y >= eps ? 0.5f : 0.0f) + (v.y >= eps ? 0.5f : 0.0f);
+    } else {
+        float n[2] = {0.0f, 0.0f};
 #pragma unroll
-        for (int k = 0; k < 8; k++) visible += (dot3(sub3(c[k], point), normal) >= eps) ? 1u : 0u;
-        return n.power / dist_sq * ((float)visible / 8.0f);
-    }
-    float visible = 0.0f;
+        for (int s = 0; s < 2; s++) {
+            const float x[2] = {s ? lx.y : lx.x, s ? hx.y : hx.x}, y[2] = {s ? ly.y : ly.x, s ? hy.y : hy.x},
+                        z[2] = {s ? lz.y : lz.x, s ? hz.y : hz.x};
 #pragma unroll
-    for (int k = 0; k < 8; k++) visible += 0.125f * ((dot3(sub3(c[k], point), normal) >= eps) ? 1.0f : 0.0f);
-    return n.power / dist_sq * visible;
+            for (int k = 0; k < 8; k++)
+                n[s] += dot3(sub3(f3{x[(k >> 2) & 1], y[(k >> 1) & 1], z[k & 1]}, point), normal) >= eps ? 0.125f : 0.0f;
+        }
+        vl = n[0];
+        vr = n[1];
+    }
+    LightPair R;
+    R.imp = make_float2(d.x / dl * vl, d.y / dr * vr);
+    R.left = __float_as_int(d.z);
+    R.right = __float_as_int(d.w);
+    return R;
 }
 
 struct Descent {
@@ -129,40 +135,37 @@ __device__ Descent light_descent(const DevScene &sc, f3 point, f3 normal, uint32
     R.inst = 0;
     R.leaf = 0;
     R.importance = 0.0f;
-    const vrg_bvh_node *root = sc.light_tl;
-    NodeV node = ldnode(&root[0]);
-    if (node.left == INVALID && node.right == INVALID) return R;
+    int ref = sc.light_root;
+    if (ref == EMPTY_ROOT) return R;
     const ImpPt P = imp_point(point, normal);
     float importance = 0.0f;
-    float off[3] = {0.0f, 0.0f, 0.0f};
-    uint32_t inst = INVALID, node_idx = 0;
     bool top = true;
     for (int guard = 0; guard < 256; guard++) {
-        if (top && node.left == INVALID) {
-            inst = node.right;
-            const InstDev &I = sc.inst[inst];
-            off[0] = I.off[0]; off[1] = I.off[1]; off[2] = I.off[2];
+        if (ref < 0) {
+            if (!top) {
+                R.success = true;
+                R.leaf = (uint32_t)~ref;
+                R.importance = importance;
+                return R;
+            }
+            // an instance: on with its BLAS root, whose importance counts
+            // when the top level's was 0
+            R.inst = (uint32_t)~ref;
             top = false;
-            root = I.light_bl;
-            node = ldnode(&root[0]);
-            node_idx = 0;
-            if (importance == 0.0f) importance = node_importance<false>(P, off, node);
+            const InstDev &I = sc.inst[R.inst];
+            if (importance == 0.0f) importance = light_pair<false>(sc, P, I.light_tl).imp.x;
+            ref = (int)I.light_base;
+            if (I.light_leaf) {
+                ref = ~0;
+                continue;
+            }
         }
-        if (!top && node.left == INVALID) {
-            R.success = true;
-            R.inst = inst;
-            R.leaf = node_idx;
-            R.importance = importance;
-            return R;
-        }
-        uint32_t li = node.left, ri = node.right;
-        NodeV left = ldnode(&root[li]), right = ldnode(&root[ri]);
-        float lI = node_importance<false>(P, off, left);
-        float rI = node_importance<false>(P, off, right);
-        float tot = lI + rI;
-        const float ln = lI / tot;  // the shader's right ratio is never read
-        if (mm_rand(seed) < ln) { node = left; node_idx = li; importance = lI; }
-        else { node = right; node_idx = ri; importance = rI; }
+        const LightPair c = light_pair<false>(sc, P, (uint32_t)ref);
+        const float tot = c.imp.x + c.imp.y;
+        const float ln = c.imp.x / tot;  // the shader's right ratio is never read
+        const bool left = mm_rand(seed) < ln;
+        ref = left ? c.left : c.right;
+        importance = left ? c.imp.x : c.imp.y;
         seed = mm_combine(seed, 0);
     }
     return R;
@@ -170,37 +173,14 @@ __device__ Descent light_descent(const DevScene &sc, f3 point, f3 normal, uint32
 
 // reverseTraverseBvh (nee_pdf.rs:154-228)
 __device__ float reverse_walk(const DevScene &sc, f3 point, f3 normal, uint32_t ii, uint32_t leaf) {
-    const InstDev &I = sc.inst[ii];
-    const vrg_bvh_node *root = I.light_bl;
     float probability = 1.0f;
-    float off[3] = {I.off[0], I.off[1], I.off[2]};
-    bool top = false;
-    NodeV node = ldnode(&root[leaf]);
-    uint32_t node_idx = leaf;
     const ImpPt P = imp_point(point, normal);
-    for (int guard = 0; guard < 256; guard++) {
-        uint32_t old = node_idx;
-        if (node.parent == INVALID) {
-            if (top) return probability;
-            top = true;
-            root = sc.light_tl;
-            old = I.light_bvh_tl_idx;
-            NodeV tl_leaf = ldnode(&root[I.light_bvh_tl_idx]);
-            if (tl_leaf.parent == INVALID) return probability;
-            node_idx = tl_leaf.parent;
-            node = ldnode(&root[node_idx]);
-            off[0] = off[1] = off[2] = 0.0f;
-        } else {
-            node_idx = node.parent;
-            node = ldnode(&root[node_idx]);
-        }
-        NodeV left = ldnode(&root[node.left]), right = ldnode(&root[node.right]);
-        float lI = node_importance<true>(P, off, left);
-        float rI = node_importance<true>(P, off, right);
-        float tot = lI + rI;
-        float ln = lI / tot, rn = rI / tot;
-        if (old == node.left) probability *= ln;
-        else probability *= rn;
+    uint32_t up = __ldg(sc.light_par + sc.inst[ii].light_base + leaf);
+    for (int guard = 0; guard < 256 && up != INVALID; guard++) {
+        const uint32_t g = up >> 1, right = up & 1u;
+        up = __ldg(sc.light_par + g);
+        const float2 imp = light_pair<true>(sc, P, g).imp;
+        probability *= (right ? imp.y : imp.x) / (imp.x + imp.y);
     }
     return probability;
 }

@@ -243,15 +243,31 @@ constexpr uint32_t INST_XFORM = 2u;   // a transform other than a translation
 
 struct InstDev {
     float off[3];                     // the translation (0 with INST_XFORM)
-    uint32_t light_bvh_tl_idx;        // prim2node (scene.rs:282-287)
-    const vrg_bvh_node *light_bl;     // light BLAS nodes (object space; with INST_XFORM their min and
-                                      // max already transformed, the v000 / v111 of nodeImportance)
+    uint32_t light_tl;                // prim2node (scene.rs:282-287): its leaf of the light top level
     const uint32_t *light_leaf_tri;   // per light BLAS node: chunk lx | ly<<5 | lz<<10 | face<<15 | half<<18,
                                       // mesh: its triangle index
+    const float *uv;                  // mesh: vertex uvs, 6 floats per triangle
     uint32_t flags;                   // INST_*
     uint32_t tri_base;                // mesh: its first world-space triangle record (DevScene::tri_rec)
-    const float *uv;                  // mesh: vertex uvs, 6 floats per triangle
+    uint32_t light_base;              // its light BLAS's first node in DevScene::light_pair / light_par
+    uint32_t light_leaf;              // 1: its light BLAS is a single leaf
 };
+
+// The light tree as its two walks read it, over the combined index space
+// [top level | every instance's BLAS] (world space; node j of instance k is
+// InstDev::light_base + j).  Per inner node, 64 bytes, its two children side
+// by side (L, R):
+//   0 (min.x L R, min.y L R)  1 (min.z L R, max.x L R)  2 (max.y L R, max.z L R)
+//   3 (power L R, ref L R)
+// min and max are nodeImportance's v000 and v111 (the instance transform
+// applied to the node's min and max).  A ref >= 0 is an inner node; a leaf is
+// ~instance in the top level, ~(BLAS node) below.  A top-level leaf's own
+// slot holds its instance's BLAS root as L.  light_par: parent << 1 | (is the
+// right child), INVALID at the top; a BLAS root's parent is its top-level
+// leaf's.  Both children's importance then takes four 16-byte loads of one
+// 64-byte line instead of ten 8-byte loads of two 40-byte nodes, and packed
+// arithmetic (f32x2) for the pair; the way up follows light_par alone.
+constexpr int LIGHT_PAIR = 4;  // float4 per node
 
 // The instance transform applied to a point: a translation exactly (p + t),
 // any other row-major 3x4 [R|t] as ((r0*x + r1*y) + r2*z) + t per row — the
@@ -340,7 +356,9 @@ struct DevScene {
     const int4 *lamp_rec;     // per lamp block: x/y packed coords + instance, z emissive face mask, w table base
     const uint32_t *lamp_table;  // 12 per lamp block: light-BLAS leaf of (face, half), INVALID if none
     int lamp_root;
-    const vrg_bvh_node *light_tl;  // reference-format light TL BVH (dummy node if no light)
+    const float4 *light_pair;      // the light tree (LIGHT_PAIR float4 per node) and its parents
+    const uint32_t *light_par;
+    int light_root;                // >= 0 inner node 0, < 0 ~instance (one light instance), EMPTY_ROOT no light
     const InstDev *inst;
     const vrg_material *mats;
     uint32_t n_inst;
