@@ -15,6 +15,7 @@ namespace vrg {
 
 vrg_status upload_frames(cudaStream_t s);
 vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, cudaEvent_t ev_trace, uint32_t max_rays);
+vrg_status launch_frame_begin(cudaStream_t s, const FrameArgs &a, uint32_t max_entries);
 vrg_status launch_light_pdf(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
 vrg_status launch_resolve(cudaStream_t s, const FrameArgs &a);
 vrg_status launch_spatial(cudaStream_t s, const FrameArgs &a, const CUtensorMap *res_map);
@@ -160,6 +161,24 @@ VRG_API vrg_status vrg_context_destroy(vrg_context *ctx) {
     return VRG_OK;
 }
 
+// the device copy of a material table: the table, then reflectivity / pi per
+// material, which the Lambertian branch of the shading divides out per vertex
+// in the reference
+static vrg_status upload_materials(vrg_context *ctx, const std::vector<vrg_material> &mats, DevBufPtr &out) {
+    static_assert(sizeof(vrg_material) == 48 && offsetof(vrg_material, emission) == 16, "read as float4 pairs");
+    const size_t n = mats.size(), tab = n * sizeof(vrg_material);
+    std::vector<float4> lam(n);
+    for (size_t i = 0; i < n; i++)
+        lam[i] = make_float4(mats[i].reflectivity[0] / PI_F, mats[i].reflectivity[1] / PI_F,
+                             mats[i].reflectivity[2] / PI_F, 0.0f);
+    VRG_TRY(dev_alloc(ctx->stream, tab + n * sizeof(float4), out));
+    VRG_CUDA_TRY(cudaMemcpyAsync(out->ptr, mats.data(), tab, cudaMemcpyHostToDevice, ctx->stream));
+    VRG_CUDA_TRY(cudaMemcpyAsync((uint8_t *)out->ptr + tab, lam.data(), n * sizeof(float4), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+    VRG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    return VRG_OK;
+}
+
 VRG_API vrg_status vrg_material_table_set(vrg_context *ctx, const vrg_material *mats, uint32_t n) {
     if (!ctx || !mats || n == 0 || n % 6 || n / 6 > 255) {
         set_error("material table needs a multiple of 6 entries, at most 6*255");
@@ -176,9 +195,7 @@ VRG_API vrg_status vrg_material_table_set(vrg_context *ctx, const vrg_material *
     ctx->atlas_w = ctx->atlas_h = 0;
     ctx->d_srgb = nullptr;
     DevBufPtr b;
-    VRG_TRY(dev_alloc(ctx->stream, n * sizeof(vrg_material), b));
-    VRG_CUDA_TRY(cudaMemcpyAsync(b->ptr, mats, n * sizeof(vrg_material), cudaMemcpyHostToDevice, ctx->stream));
-    VRG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    VRG_TRY(upload_materials(ctx, ctx->mats, b));
     ctx->d_mats = b;
     return VRG_OK;
 }
@@ -220,11 +237,9 @@ VRG_API vrg_status vrg_texture_atlas_set(vrg_context *ctx, const uint8_t *rgba8,
     const size_t atlas_bytes = (size_t)n_slots * 3 * map * 4, lut_off = (atlas_bytes + 255) & ~(size_t)255;
     DevBufPtr ab, mb;
     VRG_TRY(dev_alloc(ctx->stream, lut_off + sizeof(lut), ab));
-    VRG_TRY(dev_alloc(ctx->stream, mats.size() * sizeof(vrg_material), mb));
+    VRG_TRY(upload_materials(ctx, mats, mb));
     VRG_CUDA_TRY(cudaMemcpyAsync(ab->ptr, rgba8, atlas_bytes, cudaMemcpyHostToDevice, ctx->stream));
     VRG_CUDA_TRY(cudaMemcpyAsync((uint8_t *)ab->ptr + lut_off, lut, sizeof(lut), cudaMemcpyHostToDevice, ctx->stream));
-    VRG_CUDA_TRY(cudaMemcpyAsync(mb->ptr, mats.data(), mats.size() * sizeof(vrg_material), cudaMemcpyHostToDevice,
-                                 ctx->stream));
     VRG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     ctx->mats = mats;
     ctx->d_mats = mb;
@@ -510,11 +525,22 @@ static void drop_graphs(vrg_renderer *r) {
 static vrg_status renderer_alloc(vrg_renderer *r) {
     const size_t P = (size_t)r->P;
     const uint32_t nb = r->nb_max;
+    // the views' primary-ray tables (one view: the renderer's own extent)
+    const uint32_t n_tab = r->n_views ? r->n_views : 1;
+    r->vtoff.resize(n_tab);
+    r->tab_entries = 0;
+    r->tab_max = 0;
+    for (uint32_t v = 0; v < n_tab; v++) {
+        const uint32_t n = r->n_views ? r->vw[v] + r->vh[v] : r->W + r->H;
+        r->vtoff[v] = r->tab_entries;
+        r->tab_entries += n;
+        r->tab_max = std::max(r->tab_max, n);
+    }
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     size_t o = 0;
     // the arrays of a frame's bounces, one set per frame in flight
     struct SetOff {
-        size_t ro, rd, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, nv, xs, ns;
+        size_t ro, rd, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, nv, xs, ns, rt;
     } so[Renderer::SETS];
     const int sets = (int)r->n_sets;
     for (int k = 0; k < sets; k++) {
@@ -538,6 +564,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
         q.nv = o; o += al(P * 16);
         q.xs = o; o += al(P * 16);
         q.ns = o; o += al(P * 16);
+        q.rt = o; o += al(r->tab_entries * 16);
     }
     size_t o_pl = o; o += al(P * 16);
     size_t o_sp = o; o += al(P * 80);
@@ -570,6 +597,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
         F.nv = (float4 *)(B + q.nv);
         F.xs = (float4 *)(B + q.xs);
         F.ns = (float4 *)(B + q.ns);
+        F.ray_tab = (float4 *)(B + q.rt);
     }
     r->plain = (float4 *)(B + o_pl);
     r->spatial = (float4 *)(B + o_sp);
@@ -1046,6 +1074,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     memset(&a, 0, sizeof(a));
     a.P = (uint32_t)P;
     a.tiles_x = (r->W + 7) / 8;
+    a.tile_magic = div_magic(a.tiles_x);
     a.n0 = r->n_views ? (uint32_t)P : a.tiles_x * ((r->H + 3) / 4) * 32u;
     a.nb = nb_total;
     a.nb_render = pr->num_bounces;
@@ -1192,7 +1221,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
         VRG_CUDA_TRY(cudaEventRecord(r->ev_updated, r->aux));
         updated = true;
     }
-    VRG_CUDA_TRY(cudaMemsetAsync(a.counters, 0, CNT_WORDS * 4, bs));
+    VRG_TRY(launch_frame_begin(bs, a, r->tab_max));
     if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[0], s));
     // Bounce b's light-pdf walk runs on the light-pdf stream beside bounce
     // b + 1's closest hit and shading.  Ordering: the walk of b waits for the
@@ -1443,6 +1472,9 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
     a.v0.pix_off = 0;
     a.v0.pix_end = (uint32_t)P;
     a.v0.frame = r->frame;
+    a.v0.w_magic = div_magic(r->W);
+    a.v0.ray_x = r->fs[frame_set(r)].ray_tab;
+    a.v0.ray_y = a.v0.ray_x + r->W;
     a.v0.temporal_seed = pr->temporal_seed;
     a.v0.spatial_seed = pr->spatial_seed;
     if (out && !out->host) {  // device outputs are written in place
@@ -1552,6 +1584,9 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
         d.pix_off = (uint32_t)r->voff[v];
         d.pix_end = (uint32_t)(r->voff[v] + (uint64_t)r->vw[v] * r->vh[v]);
         d.frame = r->frame;
+        d.w_magic = div_magic(d.W);
+        d.ray_x = r->fs[frame_set(r)].ray_tab + r->vtoff[v];
+        d.ray_y = d.ray_x + d.W;
         d.temporal_seed = w.temporal_seed;
         d.spatial_seed = w.spatial_seed;
     }

@@ -207,7 +207,8 @@ __device__ __forceinline__ void spatial_pixel(const FrameArgs &a, uint32_t p, co
         // neighbours are taken within the pixel's own view
         const ViewDev &V = view_of<BATCH>(a, p);
         const uint32_t lp = p - V.pix_off;
-        const uint32_t qx = lp % V.W, qy = lp / V.W;
+        uint32_t qx, qy;
+        div_mod(lp, V.W, V.w_magic, qy, qx);
         const uint32_t ps = mm_combine(V.spatial_seed, lp);
         Res Rs = load_res_src(src, p, qx, qy);
         const f3 Sx_v = Rs.x_v, Sn_v = Rs.n_v;

@@ -921,6 +921,7 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
                    : lr.left_node_idx != INVALID ? 0 : ~(int)lr.right_node_idx_or_prim_idx;
     D.inst = (const InstDev *)(B + cp.o_inst);
     D.mats = (const vrg_material *)sc->ctx->d_mats->ptr;
+    D.lambert = lambert_of(sc->ctx);
     D.n_inst = ni;
     // geometry root: the TL root, or with one object its BLAS root / single record
     if (cp.n_geo_tl == 0) {
@@ -1099,6 +1100,7 @@ DevScene frame_scene(const Scene *sc) {
     DevScene D = sc->dev;
     const Context *ctx = sc->ctx;
     D.mats = ctx->d_mats ? (const vrg_material *)ctx->d_mats->ptr : nullptr;
+    D.lambert = lambert_of(ctx);
     D.atlas = ctx->d_atlas ? (const uchar4 *)ctx->d_atlas->ptr : nullptr;
     D.srgb = ctx->d_srgb;
     D.atlas_w = ctx->atlas_w;

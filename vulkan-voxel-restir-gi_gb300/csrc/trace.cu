@@ -16,6 +16,7 @@
 // next queues with one warp ballot + one atomic per warp.  State per pixel
 // stays in SoA float4 arrays; the per-bounce record (E, w=pdf/q) (R, q) feeds
 // the backward radiance recurrence of the resolve kernel.
+#include <cstring>
 #include <mutex>
 
 #include "vrg_frame.cuh"
@@ -23,7 +24,10 @@
 
 namespace vrg {
 
-__constant__ Frame c_frames[12];
+// Per (face, half): (normal, corner bits of the triangle's vertices: 3 x 3
+// bits), tangent, bitangent.  In global memory, not constant memory: the lanes
+// of a warp shade different faces, and constant loads serialize over them.
+__device__ float4 d_faces[12 * 3];
 
 namespace {
 
@@ -256,26 +260,36 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 // raygen (raygen.rs:84-111): pixel corner, jitter multiplied by 0.00
-// lp: the pixel's index within its view
-__device__ __forceinline__ void raygen(const ViewDev &V, uint32_t lp, f3 &o, f3 &d) {
-    uint32_t x = lp % V.W, y = lp / V.W;
-    float u = 2.0f * (float)x / (float)V.W - 1.0f;
-    float v = 2.0f * (float)y / (float)V.H - 1.0f;
-    float aspect = (float)V.W / (float)V.H;
+__device__ __forceinline__ f3 ray_col(const ViewDev &V, uint32_t x) {
+    const float u = 2.0f * (float)x / (float)V.W - 1.0f;
+    const float aspect = (float)V.W / (float)V.H;
+    return scl3(lscl3(u, V.right), aspect);
+}
+__device__ __forceinline__ f3 ray_row(const ViewDev &V, uint32_t y) {
+    return lscl3(2.0f * (float)y / (float)V.H - 1.0f, V.up);
+}
+__device__ __forceinline__ void raygen(const ViewDev &V, uint32_t x, uint32_t y, f3 &o, f3 &d) {
     o = V.eye;
-    d = norm3(add3(add3(scl3(lscl3(u, V.right), aspect), lscl3(v, V.up)), V.front));
+    d = norm3(add3(add3(ld3(__ldg(V.ray_x + x)), ld3(__ldg(V.ray_y + y))), V.front));
 }
 
-// Conservative slab test of a traversal box (boxes carry BOX_MARGIN, so the
-// rounding of the FMA form never culls a box that holds a candidate face).
-__device__ __forceinline__ bool slab_fma(float lox, float hix, float loy, float hiy, float loz, float hiz, f3 inv,
-                                         f3 oi, float tmin, float tmax, float &tn) {
-    float t0x = __fmaf_rn(lox, inv.x, oi.x), t1x = __fmaf_rn(hix, inv.x, oi.x);
-    float t0y = __fmaf_rn(loy, inv.y, oi.y), t1y = __fmaf_rn(hiy, inv.y, oi.y);
-    float t0z = __fmaf_rn(loz, inv.z, oi.z), t1z = __fmaf_rn(hiz, inv.z, oi.z);
-    tn = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fmaxf(fminf(t0z, t1z), tmin));
-    float tf = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fminf(fmaxf(t0z, t1z), tmax));
-    return tn <= tf;
+// Start of a frame: clears the counters and fills every view's primary-ray
+// tables (W + H entries; the terms take three divisions and nine products per
+// ray when the closest hit and the shading work them out each for themselves;
+// with the integer divisions and the materials' R / pi gone too, the 1080p
+// frame in flight went from 1014 to 995 us).  blockIdx.y is the view.
+template <bool BATCH>
+__global__ void __launch_bounds__(128) k_frame_begin(const __grid_constant__ FrameArgs a) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0 && i < CNT_WORDS) a.counters[i] = 0;
+    const ViewDev &V = BATCH ? a.views[blockIdx.y] : a.v0;
+    if (i < V.W) {
+        const f3 c = ray_col(V, i);
+        V.ray_x[i] = make_float4(c.x, c.y, c.z, 0.0f);
+    } else if (i < V.W + V.H) {
+        const f3 c = ray_row(V, i - V.W);
+        V.ray_y[i - V.W] = make_float4(c.x, c.y, c.z, 0.0f);
+    }
 }
 
 // Pops the next pending child whose box starts at or before best_t (boxes
@@ -463,7 +477,8 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
             range.cur = min(base + (uint32_t)__popc(need), range.end);
             if (!has) {
                 const uint32_t idx = base + (uint32_t)__popc(need & lanemask_lt());
-                if (idx < range.end && (b == 0 ? bounce0_pixel<BATCH>(a, idx, p) : (p = qin[idx], true))) {
+                uint32_t x = 0, y = 0;
+                if (idx < range.end && (b == 0 ? bounce0_pixel<BATCH>(a, idx, p, x, y) : (p = qin[idx], true))) {
                     has = true;
                     traced++;
                     const ViewDev &V = view_of<BATCH>(a, p);
@@ -474,7 +489,7 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
                         nblk = V.sc.n_blk_rec;
                         root = V.sc.geo_root;
                     }
-                    if (b == 0) raygen(V, p - V.pix_off, o, d);
+                    if (b == 0) raygen(V, x, y, o, d);
                     else { o = ld3(a.ray_o[p]); d = ld3(a.ray_d[p]); }
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
                     oi = f3{-o.x * inv.x, -o.y * inv.y, -o.z * inv.z};
@@ -618,7 +633,8 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
         const float b1 = __int_as_float(hv.z), b2 = __int_as_float(hv.w);
         const float b0 = (1.0f - b1) - b2;
         f3 t0, t1, t2;
-        Frame fr;
+        Frame fr;                    // the tangent and bitangent where the direction needs them
+        const float4 *ft = nullptr;  // a voxel face's row of d_faces
         uint32_t slot;
         float u = 0.0f, v = 0.0f;  // the texture coordinate (read with an atlas only)
         if (MESH && (uint32_t)hv.x >= S.n_blk_rec) {
@@ -631,7 +647,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
             t0 = ld3(A);
             t1 = ld3(B);
             t2 = ld3(C);
-            fr = tri_frame(t0, t1, t2);
+            fr.n = tri_frame(t0, t1, t2).n;
             slot = __float_as_uint(C.w);
             face = (int)(0x80000000u | tr);
             rc = make_int4((int)__float_as_uint(A.w), (int)__float_as_uint(B.w), -1, 0);
@@ -645,10 +661,13 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
             face = hv.y & 7;
             half = (hv.y >> 3) & 1;
             const int wx = rec_wx(rc), wy = rec_wy(rc), wz = rec_wz(rc);
-            t0 = corner_pos(wx, wy, wz, face_corner(face, half, 0));
-            t1 = corner_pos(wx, wy, wz, face_corner(face, half, 1));
-            t2 = corner_pos(wx, wy, wz, face_corner(face, half, 2));
-            fr = c_frames[2 * face + half];
+            ft = d_faces + 3 * (2 * face + half);
+            const float4 q = __ldg(ft);
+            const uint32_t cb = __float_as_uint(q.w);
+            fr.n = ld3(q);
+            t0 = corner_pos(wx, wy, wz, cb & 7u);
+            t1 = corner_pos(wx, wy, wz, (cb >> 3) & 7u);
+            t2 = corner_pos(wx, wy, wz, cb >> 6);
             const uint32_t blk_id = ((uint32_t)rc.z >> 21) & 0xFFu;
             slot = 6u * blk_id + (uint32_t)face;
             if (S.atlas) {  // gen_mesh's corner uvs
@@ -678,11 +697,13 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
                    (1000.0f * __ldg(lin + x1.z)) * ndd};
             metal = __ldg(lin + x2.x);
         } else {
-            const vrg_material &m = S.mats[slot];
-            R = f3{__ldg(&m.reflectivity[0]), __ldg(&m.reflectivity[1]), __ldg(&m.reflectivity[2])};
-            alpha = __ldg(&m.alpha);
-            metal = __ldg(&m.metallic);
-            E = f3{__ldg(&m.emission[0]) * ndd, __ldg(&m.emission[1]) * ndd, __ldg(&m.emission[2]) * ndd};
+            // (reflectivity, alpha), (emission, metallic)
+            const float4 *m = reinterpret_cast<const float4 *>(S.mats + slot);
+            const float4 ra = __ldg(m), em = __ldg(m + 1);
+            R = ld3(ra);
+            alpha = ra.w;
+            E = f3{em.x * ndd, em.y * ndd, em.z * ndd};
+            metal = em.w;
         }
         const float r0 = mm_rand(mm_combine(seed, 0));
         if (r0 < metal) {
@@ -694,7 +715,8 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
             pdf = 1.0f;
         } else {
             new_o = add3(new_o, lscl3(EPS_TRACE * 1.5f, n));
-            R = f3{R.x / PI_F, R.y / PI_F, R.z / PI_F};
+            if (S.atlas) R = f3{R.x / PI_F, R.y / PI_F, R.z / PI_F};
+            else R = ld3(__ldg(S.lambert + slot));
             if (!need_dir) {
                 new_d = f3{0.0f, 0.0f, 0.0f};
                 goto done;
@@ -719,6 +741,13 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
                 sincos_turns(ux, &s, &c);
                 const float vv = sqrtf(fmaxf(0.0f, 1.0f - uy * uy));
                 const f3 hs = f3{vv * c, uy, vv * s};
+                if (!MESH || ft) {
+                    fr.t = ld3(__ldg(ft + 1));
+                    fr.b = ld3(__ldg(ft + 2));
+                } else {  // (worked out again here, not carried through the descent)
+                    const float4 *q = S.tri_rec + 3 * (size_t)((uint32_t)face & 0x7FFFFFFFu);
+                    fr = tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2)));
+                }
                 new_d = norm3(add3(add3(lscl3(hs.x, fr.t), lscl3(hs.y, fr.n)), lscl3(hs.z, fr.b)));
             }
             pdf = dot3(new_d, n) / PI_F;
@@ -814,7 +843,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
         }
         const uint32_t passes = split ? (n_route + 31u) / 32u : 1u;
         for (uint32_t pass = 0; pass < passes; pass++) {
-            uint32_t p = 0;
+            uint32_t p = 0, px = 0, py = 0;
             bool active;
             if (split) {
                 const uint32_t r = 32 * pass + lane;
@@ -822,7 +851,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 if (active) p = route[r];
             } else {
                 const uint32_t i = base + lane;
-                active = i < n_in && (b == 0 ? bounce0_pixel<BATCH>(a, i, p) : (p = qin[i], true));
+                active = i < n_in && (b == 0 ? bounce0_pixel<BATCH>(a, i, p, px, py) : (p = qin[i], true));
             }
             bool cont = false, anyj = false, qhit = false, want_train = false;
             const bool at_query = a.cache && b + 1 == a.nb_render;
@@ -838,7 +867,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 const uint32_t lp = p - V.pix_off;
                 f3 o, d;
                 if (b == 0) {
-                    raygen(V, lp, o, d);
+                    raygen(V, px, py, o, d);
                     if (CAPTURE) {
                         st3(a.c_origin, p, o);
                         st3(a.c_dir, p, d);
@@ -1232,7 +1261,7 @@ __global__ void __launch_bounds__(128) k_hit_eval(const __grid_constant__ FrameA
         const int fw = __float_as_int(ro.w);
         f3 n3;
         if (fw >= 0) {
-            n3 = c_frames[2 * fw].n;
+            n3 = ld3(__ldg(d_faces + 6 * fw));
         } else {
             const float4 *q = sc.tri_rec + 3 * (size_t)((uint32_t)fw & 0x7FFFFFFFu);
             n3 = tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2))).n;
@@ -1265,10 +1294,18 @@ __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameAr
 }  // namespace
 
 vrg_status upload_frames(cudaStream_t s) {
-    Frame fr[12];
+    float4 t[12 * 3];
     for (int f = 0; f < 6; f++)
-        for (int h = 0; h < 2; h++) fr[2 * f + h] = face_frame(f, h);
-    VRG_CUDA_TRY(cudaMemcpyToSymbolAsync(c_frames, fr, sizeof(fr), 0, cudaMemcpyHostToDevice, s));
+        for (int h = 0; h < 2; h++) {
+            const Frame fr = face_frame(f, h);
+            const uint32_t bits = face_corner(f, h, 0) | face_corner(f, h, 1) << 3 | face_corner(f, h, 2) << 6;
+            float4 *q = t + 3 * (2 * f + h);
+            q[0] = make_float4(fr.n.x, fr.n.y, fr.n.z, 0.0f);
+            memcpy(&q[0].w, &bits, 4);
+            q[1] = make_float4(fr.t.x, fr.t.y, fr.t.z, 0.0f);
+            q[2] = make_float4(fr.b.x, fr.b.y, fr.b.z, 0.0f);
+        }
+    VRG_CUDA_TRY(cudaMemcpyToSymbolAsync(d_faces, t, sizeof(t), 0, cudaMemcpyHostToDevice, s));
     return VRG_OK;
 }
 
@@ -1329,6 +1366,15 @@ static void bounce_grids(const FrameArgs &a, uint32_t max_rays, int &gt, int &gs
         gs = std::min(gs, cap);
         ga = std::min(ga, cap);
     }
+}
+
+// the frame's counters cleared and its ray tables filled
+vrg_status launch_frame_begin(cudaStream_t s, const FrameArgs &a, uint32_t max_entries) {
+    const dim3 g((std::max(max_entries, (uint32_t)CNT_WORDS) + 127) / 128, a.views ? a.n_views : 1);
+    if (a.views) k_frame_begin<true><<<g, 128, 0, s>>>(a);
+    else k_frame_begin<false><<<g, 128, 0, s>>>(a);
+    VRG_CUDA_TRY(cudaGetLastError());
+    return VRG_OK;
 }
 
 // closest hit of bounce b

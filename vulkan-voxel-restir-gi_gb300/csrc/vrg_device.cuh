@@ -361,6 +361,7 @@ struct DevScene {
     int light_root;                // >= 0 inner node 0, < 0 ~instance (one light instance), EMPTY_ROOT no light
     const InstDev *inst;
     const vrg_material *mats;
+    const float4 *lambert;         // per material: reflectivity / pi
     uint32_t n_inst;
     // texture atlas (NULL: constant slot colours): [slot][3 maps][h][w] RGBA8,
     // and the sRGB-to-linear table of the 256 byte values

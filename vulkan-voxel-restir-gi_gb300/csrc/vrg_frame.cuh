@@ -39,8 +39,27 @@ struct ViewDev {
     DevScene sc;
     f3 eye, front, right, up;
     uint32_t W, H, pix_off, pix_end;
-    uint32_t frame, temporal_seed, spatial_seed, pad;
+    uint32_t frame, temporal_seed, spatial_seed;
+    uint32_t w_magic;             // div_magic(W)
+    // the primary rays' direction terms of the frame's camera per column and
+    // per row (k_frame_begin): d = normalize((ray_x[x] + ray_y[y]) + front)
+    float4 *ray_x, *ray_y;
 };
+
+// n / d and n % d for any 32-bit n by one high product and a correction, with
+// m = floor(2^32 / d) from the host (the quotient is short by at most 1; cf.
+// Granlund and Montgomery, PLDI 1994): 5 instructions, an integer division
+// with its remainder about 25.
+inline uint32_t div_magic(uint32_t d) { return d <= 1 ? 0xFFFFFFFFu : (uint32_t)((1ull << 32) / d); }
+__host__ __device__ __forceinline__ void div_mod(uint32_t n, uint32_t d, uint32_t m, uint32_t &q, uint32_t &rem) {
+    q = (uint32_t)(((uint64_t)n * m) >> 32);
+    rem = n - q * d;
+    if (rem >= d) {
+        q++;
+        rem -= d;
+    }
+}
+
 constexpr int VIEW_SHIFT = 8;  // vtab entry per 256 pixels: the view of the group's first pixel
 
 struct FrameArgs {
@@ -52,6 +71,7 @@ struct FrameArgs {
                                   // built with mesh support run; voxel-only frames run without it)
     uint32_t P;                   // pixels of the frame (all views)
     uint32_t n0, tiles_x;         // bounce-0 slots and 8x4 tiles per row (bounce0_pixel)
+    uint32_t tile_magic;          // div_magic(tiles_x)
     uint32_t nb, nee_type;
     uint32_t mode, spatial_iters;
     float spatial_radius;
@@ -127,13 +147,19 @@ __device__ __forceinline__ const ViewDev &view_of(const FrameArgs &a, uint32_t p
 // start close together.  Slot i (< n0) is pixel p, or no pixel in the part of
 // an edge tile outside the view.  A batched frame keeps the pixel order.
 template <bool BATCH>
-__device__ __forceinline__ bool bounce0_pixel(const FrameArgs &a, uint32_t i, uint32_t &p) {
+__device__ __forceinline__ bool bounce0_pixel(const FrameArgs &a, uint32_t i, uint32_t &p, uint32_t &x, uint32_t &y) {
     if constexpr (BATCH) {
         p = i;
-        return i < a.P;
+        if (i >= a.P) return false;
+        const ViewDev &V = view_of<BATCH>(a, p);
+        div_mod(p - V.pix_off, V.W, V.w_magic, y, x);
+        return true;
     } else {
         const uint32_t t = i >> 5, k = i & 31u;
-        const uint32_t x = (t % a.tiles_x) * 8u + (k & 7u), y = (t / a.tiles_x) * 4u + (k >> 3);
+        uint32_t tx, ty;
+        div_mod(t, a.tiles_x, a.tile_magic, ty, tx);
+        x = tx * 8u + (k & 7u);
+        y = ty * 4u + (k >> 3);
         p = y * a.v0.W + x;
         return x < a.v0.W && y < a.v0.H;
     }

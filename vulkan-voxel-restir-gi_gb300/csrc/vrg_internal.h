@@ -118,7 +118,7 @@ struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::vector<vrg_material> mats;
-    DevBufPtr d_mats;
+    DevBufPtr d_mats;                    // the material table, then reflectivity / pi per slot (lambert_of)
     DevBufPtr d_atlas;                   // texture atlas (RGBA8) + sRGB table, or empty
     uint32_t atlas_w = 0, atlas_h = 0;
     const float *d_srgb = nullptr;
@@ -132,6 +132,10 @@ struct Context {
     // dropped, whatever the order in which the handles are destroyed
     std::atomic<int> refs{1};
 };
+// reflectivity / pi (raytrace.rs:502), float4 per material, behind a table of n materials
+inline const float4 *lambert_of(const Context *c) {
+    return c->d_mats ? (const float4 *)((const vrg_material *)c->d_mats->ptr + c->mats.size()) : nullptr;
+}
 void ctx_retain(Context *c);
 void ctx_release(Context *c);
 
@@ -215,6 +219,9 @@ struct Renderer {
     uint32_t n_views = 0;
     std::vector<uint32_t> vw, vh;         // view extents
     std::vector<uint64_t> voff;           // first pixel of each view
+    std::vector<uint64_t> vtoff;          // first entry of each view in FrameSet::ray_tab
+    uint64_t tab_entries = 0;             // its entries, all views
+    uint32_t tab_max = 0;                 // the most of one view
     DevBufPtr view_buf;                   // a ViewDev[n_views] table per array set + vtab
     ViewDev *d_views[3] = {};
     uint16_t *d_vtab = nullptr;
@@ -251,6 +258,7 @@ struct Renderer {
         uint8_t *nlive = nullptr;
         float4 *rec = nullptr;                 // [nb][2][P]
         float4 *xv = nullptr, *nv = nullptr, *xs = nullptr, *ns = nullptr;
+        float4 *ray_tab = nullptr;             // per view: W + H primary-ray terms (ViewDev::ray_x, ray_y)
     };
     static constexpr int SETS = 3;        // frames whose bounces may be in flight at once (at most)
     uint32_t n_sets = SETS;               // this renderer's sets (a batched renderer: 2)
