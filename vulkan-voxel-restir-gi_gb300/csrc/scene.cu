@@ -9,14 +9,16 @@
 //   * the closest-hit traversal layout: a world-space 4-wide BVH over the
 //     combined [top level | every object's BLAS] tree, in which each
 //     128-byte node holds its (up to) four grandchild-level children's boxes
-//     as SoA (translated to world space and widened by BOX_MARGIN, so culling
-//     is conservative) and child references (>= 0 node, < 0 ~record), with
+//     as SoA (translated to world space; the walks widen them by ray_margin, and
+//     scenes with meshes store them widened by BOX_MARGIN, so culling is
+//     conservative) and child references (>= 0 node, < 0 ~record), with
 //     top-level leaves linked straight to the object's BLAS root; and
 //     16-byte world-space records per surface block / light triangle;
 //   * the light any-hit layout: a 2-wide world-space BVH over lamp blocks.
 // Several scenes commit together with one SAH build for all their top-level
 // trees and one for all their lamp trees.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "vrg_internal.h"
@@ -40,10 +42,6 @@ struct InstBuild {
     int ioff[3];
     float m[12];               // the transform, row-major [R|t]
 };
-
-__device__ __forceinline__ int bl_root_ref(const InstBuild &I) {
-    return I.bl[0].left_node_idx != INVALID ? (int)I.wbase : ~(int)(I.refbase + I.leaf[0]);
-}
 
 // world-space box of an object-space node box: translated, or for another
 // transform the AABB of its 8 transformed corners (Aabb::transform, aabb.rs:75-92)
@@ -127,7 +125,7 @@ __device__ __forceinline__ void child_of(const vrg_bvh_node *tl, const InstBuild
 }
 
 __global__ void k_wide4(const vrg_bvh_node *tl, uint32_t n_tl, const InstBuild *inst, uint32_t n_inst,
-                        uint32_t n_total, float4 *wide4) {
+                        uint32_t n_total, float margin, float4 *wide4) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n_total) return;
     int k = -1;
@@ -162,10 +160,12 @@ __global__ void k_wide4(const vrg_bvh_node *tl, uint32_t n_tl, const InstBuild *
     for (int i = 0; i < 4; i++) {
         if (i < n) {
             float lo[3], hi[3];
-            world_box(out[i].node, out[i].k >= 0 ? &inst[out[i].k] : nullptr, out[i].off, lo, hi);
+            const InstBuild *I = out[i].k >= 0 ? &inst[out[i].k] : nullptr;
+            world_box(out[i].node, I, out[i].off, lo, hi);
+            const float w = I && !(I->flags & INST_MESH) ? 0.0f : margin;  // (a chunk's boxes hold no mesh)
             for (int a = 0; a < 3; a++) {
-                b[2 * a][i] = lo[a] - BOX_MARGIN;
-                b[2 * a + 1][i] = hi[a] + BOX_MARGIN;
+                b[2 * a][i] = lo[a] - w;
+                b[2 * a + 1][i] = hi[a] + w;
             }
             refs[i] = out[i].ref;
         } else {
@@ -452,7 +452,8 @@ __global__ void k_lamp_fill(const int4 *rec, const uint32_t *grp, uint32_t n, co
 // (the lamp-block tree): for every inner node, its children with each inner
 // child replaced by that child's two children; the layout of k_wide4
 // (lo/hi x, y, z SoA, refs: >= 0 node, < 0 ~record, EMPTY_ROOT unused)
-__global__ void k_wide4_single(const vrg_bvh_node *nodes, const uint32_t *leaf, uint32_t n_nodes, float4 *wide4) {
+__global__ void k_wide4_single(const vrg_bvh_node *nodes, const uint32_t *leaf, uint32_t n_nodes, float margin,
+                               float4 *wide4) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n_nodes) return;
     const vrg_bvh_node &nd = nodes[g];
@@ -475,8 +476,8 @@ __global__ void k_wide4_single(const vrg_bvh_node *nodes, const uint32_t *leaf, 
         if (i < n) {
             const vrg_bvh_node &c = nodes[out[i]];
             for (int a = 0; a < 3; a++) {
-                b[2 * a][i] = c.min[a] - BOX_MARGIN;
-                b[2 * a + 1][i] = c.max[a] + BOX_MARGIN;
+                b[2 * a][i] = c.min[a] - margin;
+                b[2 * a + 1][i] = c.max[a] + margin;
             }
             refs[i] = c.left_node_idx != INVALID ? (int)out[i] : ~(int)leaf[out[i]];
         } else {
@@ -492,30 +493,6 @@ __global__ void k_wide4_single(const vrg_bvh_node *nodes, const uint32_t *leaf, 
     w[6] = make_float4(__int_as_float(refs[0]), __int_as_float(refs[1]), __int_as_float(refs[2]),
                        __int_as_float(refs[3]));
     w[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-}
-
-// traversal layout of a single-level tree whose leaf prim p is record p
-__global__ void k_wide_single(const vrg_bvh_node *nodes, const uint32_t *leaf, uint32_t n_nodes, float4 *wide) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n_nodes) return;
-    const vrg_bvh_node &nd = nodes[g];
-    if (nd.left_node_idx == INVALID) return;
-    const uint32_t ch[2] = {nd.left_node_idx, nd.right_node_idx_or_prim_idx};
-    float box[2][6];
-    int ref[2];
-    for (int s = 0; s < 2; s++) {
-        const vrg_bvh_node &c = nodes[ch[s]];
-        ref[s] = c.left_node_idx != INVALID ? (int)ch[s] : ~(int)leaf[ch[s]];
-        for (int a = 0; a < 3; a++) {
-            box[s][a] = c.min[a] - BOX_MARGIN;
-            box[s][3 + a] = c.max[a] + BOX_MARGIN;
-        }
-    }
-    float4 *w = wide + 4 * (size_t)g;
-    w[0] = make_float4(box[0][0], box[0][3], box[0][1], box[0][4]);
-    w[1] = make_float4(box[0][2], box[0][5], box[1][0], box[1][3]);
-    w[2] = make_float4(box[1][1], box[1][4], box[1][2], box[1][5]);
-    w[3] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), 0.0f, 0.0f);
 }
 
 }  // namespace
@@ -619,6 +596,9 @@ struct CommitPrep {
     uint32_t lamp_depth = 0;
     DevScene dev{};                             // installed only when the whole commit succeeds
 };
+
+// the margin stored in a scene's traversal boxes (see ray_margin)
+float box_margin(const CommitPrep &cp) { return cp.tri_recs ? BOX_MARGIN : 0.0f; }
 
 vrg_status commit_prepare(Scene *sc, CommitPrep &cp) {
     cp.sc = sc;
@@ -884,7 +864,7 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
     const InstBuild *d_gb = (const InstBuild *)(B + cp.o_gb), *d_lb = (const InstBuild *)(B + cp.o_lb);
     if (cp.n_geo_wide) {
         k_wide4<<<(uint32_t)((cp.n_geo_wide + 255) / 256), 256, 0, s>>>(d_tl + cp.n_light_tl, cp.n_geo_tl, d_gb, ni,
-                                                                       (uint32_t)cp.n_geo_wide,
+                                                                       (uint32_t)cp.n_geo_wide, box_margin(cp),
                                                                        (float4 *)(B + cp.o_gw));
         VRG_CUDA_TRY(cudaGetLastError());
     }
@@ -923,6 +903,10 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
     D.mats = (const vrg_material *)sc->ctx->d_mats->ptr;
     D.lambert = lambert_of(sc->ctx);
     D.n_inst = ni;
+    D.extent = 0.0f;
+    if (cp.n_geo_tl)
+        for (int a = 0; a < 3; a++)
+            D.extent = std::max(D.extent, std::max(std::fabs(sc->h_geo_tl[0].min[a]), std::fabs(sc->h_geo_tl[0].max[a])));
     // geometry root: the TL root, or with one object its BLAS root / single record
     if (cp.n_geo_tl == 0) {
         D.geo_root = EMPTY_ROOT;
@@ -1021,7 +1005,7 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
         DevScene &D = cp.dev;
         if (cp.n_lamps > 1) {
             const uint32_t nn = 2 * cp.n_lamps - 1;
-            k_wide4_single<<<(nn + 255) / 256, 256, 0, s>>>(nodes + 2 * cp.lamp_off, leaf + 2 * cp.lamp_off, nn,
+            k_wide4_single<<<(nn + 255) / 256, 256, 0, s>>>(nodes + 2 * cp.lamp_off, leaf + 2 * cp.lamp_off, nn, box_margin(cp),
                                                             (float4 *)D.lamp_wide);
             VRG_CUDA_TRY(cudaGetLastError());
             D.lamp_root = 0;

@@ -292,6 +292,14 @@ __global__ void __launch_bounds__(128) k_frame_begin(const __grid_constant__ Fra
     }
 }
 
+// the slab test's offsets of the near and far planes, the boxes widened by m
+__device__ __forceinline__ void slab_offsets(f3 o, f3 inv, float m, f3 &oin, f3 &oif) {
+    const f3 oi = f3{-o.x * inv.x, -o.y * inv.y, -o.z * inv.z};
+    const f3 w = f3{m * fabsf(inv.x), m * fabsf(inv.y), m * fabsf(inv.z)};
+    oin = sub3(oi, w);
+    oif = add3(oi, w);
+}
+
 // Pops the next pending child whose box starts at or before best_t (boxes
 // are culled only when strictly beyond it); false when none is left.
 __device__ __forceinline__ bool pop_near(const int2 *stack, int &sp, float best_t, int &node) {
@@ -351,10 +359,10 @@ __device__ __forceinline__ float4 fma4(float4 v, float m, float c) {
 // inverse its near distance is +inf, so the slot is never entered and needs
 // no test of its ref.
 __device__ __forceinline__ void slab4(float4 NX, float4 FX, float4 NY, float4 FY, float4 NZ, float4 FZ, float4 RF,
-                                      f3 inv, f3 oi, float tmin, float tmax, float tk[4], int rk[4]) {
+                                      f3 inv, f3 oin, f3 oif, float tmin, float tmax, float tk[4], int rk[4]) {
     const int rf[4] = {__float_as_int(RF.x), __float_as_int(RF.y), __float_as_int(RF.z), __float_as_int(RF.w)};
-    const float4 ax = fma4(NX, inv.x, oi.x), ay = fma4(NY, inv.y, oi.y), az = fma4(NZ, inv.z, oi.z);
-    const float4 bx = fma4(FX, inv.x, oi.x), by = fma4(FY, inv.y, oi.y), bz = fma4(FZ, inv.z, oi.z);
+    const float4 ax = fma4(NX, inv.x, oin.x), ay = fma4(NY, inv.y, oin.y), az = fma4(NZ, inv.z, oin.z);
+    const float4 bx = fma4(FX, inv.x, oif.x), by = fma4(FY, inv.y, oif.y), bz = fma4(FZ, inv.z, oif.z);
     const float nx[4] = {ax.x, ax.y, ax.z, ax.w}, ny[4] = {ay.x, ay.y, ay.z, ay.w}, nz[4] = {az.x, az.y, az.z, az.w};
     const float fx[4] = {bx.x, bx.y, bx.z, bx.w}, fy[4] = {by.x, by.y, by.z, by.w}, fz[4] = {bz.x, bz.y, bz.z, bz.w};
 #pragma unroll
@@ -453,13 +461,14 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
     const int4 *recs = a.v0.sc.geo_rec;
     const float4 *tris = a.v0.sc.tri_rec;
     uint32_t nblk = a.v0.sc.n_blk_rec;
+    float extent = a.v0.sc.extent;
     int root = a.v0.sc.geo_root;
     if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
     __syncthreads();
     WarpRange range = range_first(n_in);
     bool has = false;
     uint32_t p = 0, steps = 0, traced = 0, n_nodes = 0, n_leaves = 0;
-    f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oi = f3{0, 0, 0};
+    f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oin = f3{0, 0, 0}, oif = f3{0, 0, 0};
     float best_t = 0.0f, hb1 = 0.0f, hb2 = 0.0f;
     uint64_t best_key = 0;
     int node = 0, sp = 0, hrec = -1;
@@ -487,12 +496,13 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
                         recs = V.sc.geo_rec;
                         tris = V.sc.tri_rec;
                         nblk = V.sc.n_blk_rec;
+                        extent = V.sc.extent;
                         root = V.sc.geo_root;
                     }
                     if (b == 0) raygen(V, x, y, o, d);
                     else { o = ld3(a.ray_o[p]); d = ld3(a.ray_d[p]); }
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
-                    oi = f3{-o.x * inv.x, -o.y * inv.y, -o.z * inv.z};
+                    slab_offsets(o, inv, ray_margin(extent, o), oin, oif);
                     px = signbit(inv.x) ? 1 : 0;
                     py = signbit(inv.y) ? 3 : 2;
                     pz = signbit(inv.z) ? 5 : 4;
@@ -521,7 +531,7 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
                 const float4 RF = __ldg(w + 6);
                 float tk[4];
                 int rk[4];
-                slab4(NX, FX, NY, FY, NZ, FZ, RF, inv, oi, EPS_TRACE, best_t, tk, rk);
+                slab4(NX, FX, NY, FY, NZ, FZ, RF, inv, oin, oif, EPS_TRACE, best_t, tk, rk);
                 // tk sorted ascending (misses at +inf)
                 if (tk[0] == INFINITY) {
                     done = !pop_near(stack, sp, best_t, node);
@@ -1091,10 +1101,11 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
     const uint32_t *table = a.v0.sc.lamp_table;
     const float4 *tris = a.v0.sc.tri_rec;
     int root = a.v0.sc.lamp_root;
+    float extent = a.v0.sc.extent;
     const float tmin = EPS_NEE, tmax = 1000.0f;
     bool has = false;
     uint32_t p = 0, idx = 0, steps = 0, n_nodes = 0, n_leaves = 0, n_hits = 0;
-    f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oi = f3{0, 0, 0};
+    f3 o = f3{0, 0, 0}, d = f3{0, 0, 0}, inv = f3{0, 0, 0}, oin = f3{0, 0, 0}, oif = f3{0, 0, 0};
     int node = EMPTY_ROOT, sp = 0, nh = 0, nl = 0;  // node < 0: the walk has ended
     int px = 0, py = 2, pz = 4;  // near-plane float4 per axis, picked by the ray's direction signs
     int stack[TRAV_STACK], lamps[LAMP_LIST];
@@ -1122,11 +1133,12 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                         table = V.sc.lamp_table;
                         tris = V.sc.tri_rec;
                         root = V.sc.lamp_root;
+                        extent = V.sc.extent;
                     }
                     o = ld3(a.ajob[b & 1][2 * (size_t)idx]);
                     d = ld3(a.ajob[b & 1][2 * (size_t)idx + 1]);
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
-                    oi = f3{-o.x * inv.x, -o.y * inv.y, -o.z * inv.z};
+                    slab_offsets(o, inv, ray_margin(extent, o), oin, oif);
                     px = signbit(inv.x) ? 1 : 0;
                     py = signbit(inv.y) ? 3 : 2;
                     pz = signbit(inv.z) ? 5 : 4;
@@ -1156,8 +1168,8 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                 const float4 RF = __ldg(w + 6);
                 const int rf[4] = {__float_as_int(RF.x), __float_as_int(RF.y), __float_as_int(RF.z),
                                    __float_as_int(RF.w)};
-                const float4 ax = fma4(NX, inv.x, oi.x), ay = fma4(NY, inv.y, oi.y), az = fma4(NZ, inv.z, oi.z);
-                const float4 bx = fma4(FX, inv.x, oi.x), by = fma4(FY, inv.y, oi.y), bz = fma4(FZ, inv.z, oi.z);
+                const float4 ax = fma4(NX, inv.x, oin.x), ay = fma4(NY, inv.y, oin.y), az = fma4(NZ, inv.z, oin.z);
+                const float4 bx = fma4(FX, inv.x, oif.x), by = fma4(FY, inv.y, oif.y), bz = fma4(FZ, inv.z, oif.z);
                 const float nx[4] = {ax.x, ax.y, ax.z, ax.w}, ny[4] = {ay.x, ay.y, ay.z, ay.w};
                 const float nz[4] = {az.x, az.y, az.z, az.w}, fx[4] = {bx.x, bx.y, bx.z, bx.w};
                 const float fy[4] = {by.x, by.y, by.z, by.w}, fz[4] = {bz.x, bz.y, bz.z, bz.w};
