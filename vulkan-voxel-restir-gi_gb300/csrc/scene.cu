@@ -291,10 +291,19 @@ __global__ void k_light_pairs(const vrg_bvh_node *tl, uint32_t n_tl, const InstB
         if (g == 0) par[J.wbase] = INVALID;  // the only light instance
     }
     float4 *q = pair + LIGHT_PAIR * (size_t)g;
-    q[0] = make_float4(lo[0].x, lo[1].x, lo[0].y, lo[1].y);
-    q[1] = make_float4(lo[0].z, lo[1].z, hi[0].x, hi[1].x);
-    q[2] = make_float4(hi[0].y, hi[1].y, hi[0].z, hi[1].z);
-    q[3] = make_float4(power[0], power[1], __int_as_float(ref[0]), __int_as_float(ref[1]));
+    f3 sum[2];
+    float ee[2];
+    for (int k = 0; k < 2; k++) {
+        sum[k] = add3(lo[k], hi[k]);
+        const f3 e = sub3(hi[k], lo[k]);
+        ee[k] = dot3(e, e);
+    }
+    q[0] = make_float4(sum[0].x, sum[1].x, sum[0].y, sum[1].y);
+    q[1] = make_float4(sum[0].z, sum[1].z, ee[0], ee[1]);
+    q[2] = make_float4(power[0], power[1], __int_as_float(ref[0]), __int_as_float(ref[1]));
+    q[3] = make_float4(lo[0].x, lo[1].x, hi[0].x, hi[1].x);
+    q[4] = make_float4(lo[0].y, lo[1].y, hi[0].y, hi[1].y);
+    q[5] = make_float4(lo[0].z, lo[1].z, hi[0].z, hi[1].z);
 }
 
 // world-space light-triangle records of every instance, one thread per light

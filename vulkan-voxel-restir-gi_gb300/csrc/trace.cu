@@ -32,101 +32,96 @@ __device__ float4 d_faces[12 * 3];
 namespace {
 
 // The shading point's part of nodeImportance, the same for every node of a
-// walk, worked out once per walk (the descent and the reverse walk are
-// bound by instruction issue; this took the 1080p frame from 1.114 to 1.086
-// ms).  Voxel-face normals are one of +-x, +-y, +-z: then dot(c - p, n) is
-// exactly +-(c_a - p_a) (the other two products are +-0), so the 8 corners
-// reduce to the box's min and max along the normal axis, 4 corners each.
+// walk, worked out once per walk.  Voxel-face normals are one of +-x, +-y,
+// +-z: then dot(c - p, n) is exactly +-(c_a - p_a) (the other two products are
+// +-0), so the 8 corners reduce to the box's min and max along the normal
+// axis, 4 corners each.
 struct ImpPt {
     f3 point, normal;
-    int ax;     // the normal's axis (| 4 when it is -1 there) when it is +-1 on one axis and 0 on
-                // the others, else -1
-    float pa;   // point[ax]
+    int ax;         // the normal's axis when it is +-1 on one axis and 0 on the others, else -1
+    float sg, sp;   // its sign there; -sg * point[ax]
 };
 __device__ __forceinline__ ImpPt imp_point(f3 point, f3 normal) {
     ImpPt P;
     P.point = point;
     P.normal = normal;
     P.ax = -1;
-    P.pa = 0.0f;
+    P.sg = P.sp = 0.0f;
     const bool nx = normal.x != 0.0f, ny = normal.y != 0.0f, nz = normal.z != 0.0f;
     if ((int)nx + (int)ny + (int)nz == 1) {
         const int ax = nx ? 0 : (ny ? 1 : 2);
         const float na = cmp3(normal, ax);
         if (na == 1.0f || na == -1.0f) {
-            P.ax = ax | (na < 0.0f ? 4 : 0);
-            P.pa = cmp3(point, ax);
+            P.ax = ax;
+            P.sg = na;
+            P.sp = -na * cmp3(point, ax);
         }
     }
     return P;
 }
 
-// Packed binary32 arithmetic, one rounding per component: fused
-// multiply-adds only.  (A packed product followed by a packed sum is
-// contracted into one by the assembler, with .rn and without -fmad, so sums
-// of products stay scalar.)
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-// (x*x + y*y) + z*z per component
-__device__ __forceinline__ float2 sq3(float2 x, float2 y, float2 z) {
-    return make_float2(dot3(f3{x.x, y.x, z.x}, f3{x.x, y.x, z.x}), dot3(f3{x.y, y.y, z.y}, f3{x.y, y.y, z.y}));
-}
-
 // nodeImportance (raytrace.rs:181-208: uint visibility, EPS 1e-3;
 // nee_pdf.rs:125-152: float visibility, EPS 1e-4) of both children of light
-// node g.  The 8 corners are the axis-aligned box that v000 and v111 span (as
-// in the reference, not the transformed box).  The centre's 0.5 * (v000 +
-// v111) is exact, so the fused subtraction of the point rounds as the
-// separate one does.
+// node g: power / max(|e|^2, |c|^2) * the visible share of the 8 corners of
+// the axis-aligned box that v000 and v111 span (as in the reference, not the
+// transformed box), c the vector from the point to the box's centre.
+// Packed operations (two per instruction) are fused multiply-adds only, where
+// one rounding is what the shader does: the centre's 0.5 * (v000 + v111) is
+// exact, and v * sign - sign * p rounds as v - p.  (The assembler contracts a
+// packed product followed by a packed sum, with .rn and without -fmad, so the
+// exact |c|^2 stays scalar.)
 struct LightPair {
-    float2 power, dist, vis;  // power, squared distance and visible share of (left, right)
-    int left, right;          // refs
-    __device__ __forceinline__ float imp_l() const { return power.x / dist.x * vis.x; }
-    __device__ __forceinline__ float imp_r() const { return power.y / dist.y * vis.y; }
+    float2 power, ee, cx, cy, cz, vis;  // of (left, right)
+    int left, right;                    // refs
+    __device__ __forceinline__ float imp_l() const {
+        return power.x / fmaxf(ee.x, (cx.x * cx.x + cy.x * cy.x) + cz.x * cz.x) * vis.x;
+    }
+    __device__ __forceinline__ float imp_r() const {
+        return power.y / fmaxf(ee.y, (cx.y * cx.y + cy.y * cy.y) + cz.y * cz.y) * vis.y;
+    }
+    // both within 2^-20: fused sums and an approximate reciprocal
+    __device__ __forceinline__ float2 imp_near() const {
+        const float2 cc = __ffma2_rn(cx, cx, __ffma2_rn(cy, cy, __fmul2_rn(cz, cz)));
+        float a, b;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(fmaxf(ee.x, cc.x)));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(fmaxf(ee.y, cc.y)));
+        return make_float2(power.x * vis.x * a, power.y * vis.y * b);
+    }
 };
 template <bool NEE>
 __device__ __forceinline__ LightPair light_pair(const DevScene &sc, const ImpPt &P, uint32_t g) {
     const float4 *q = sc.light_pair + LIGHT_PAIR * (size_t)g;
-    const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
-    const float2 lx = make_float2(a.x, a.y), ly = make_float2(a.z, a.w), lz = make_float2(b.x, b.y);
-    const float2 hx = make_float2(b.z, b.w), hy = make_float2(c.x, c.y), hz = make_float2(c.z, c.w);
-    const f3 point = P.point, normal = P.normal;
+    const float4 a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
     const float eps = NEE ? EPS_NEE : EPS_TRACE;
     const float2 half = make_float2(0.5f, 0.5f);
-    const float2 ee = sq3(sub2(hx, lx), sub2(hy, ly), sub2(hz, lz));
-    const float2 cc = sq3(__ffma2_rn(half, __fadd2_rn(lx, hx), make_float2(-point.x, -point.x)),
-                          __ffma2_rn(half, __fadd2_rn(ly, hy), make_float2(-point.y, -point.y)),
-                          __ffma2_rn(half, __fadd2_rn(lz, hz), make_float2(-point.z, -point.z)));
-    const float dl = fmaxf(ee.x, cc.x), dr = fmaxf(ee.y, cc.y);
-    float vl, vr;  // the visible share of the corners
-    if (P.ax >= 0) {
-        // voxel-face normal: the corners' two distances along its axis, 4
-        // corners each; (v - pa) * sign rounds as v - pa
-        const int ax = P.ax & 3;
-        const float sg = (P.ax & 4) ? -1.0f : 1.0f;
-        const float2 lo = ax == 0 ? lx : (ax == 1 ? ly : lz), hi = ax == 0 ? hx : (ax == 1 ? hy : hz);
-        const float2 s2 = make_float2(sg, sg), o2 = make_float2(-sg * P.pa, -sg * P.pa);
-        const float2 u = __ffma2_rn(lo, s2, o2), v = __ffma2_rn(hi, s2, o2);
-        vl = (u.x >= eps ? 0.5f : 0.0f) + (v.x >= eps ? 0.5f : 0.0f);
-        vr = (u.y >= eps ? 0.5f : 0.0f) + (v.y >= eps ? 0.5f : 0.0f);
-    } else {
-        float n[2] = {0.0f, 0.0f};
-#pragma unroll
-        for (int s = 0; s < 2; s++) {
-            const float x[2] = {s ? lx.y : lx.x, s ? hx.y : hx.x}, y[2] = {s ? ly.y : ly.x, s ? hy.y : hy.x},
-                        z[2] = {s ? lz.y : lz.x, s ? hz.y : hz.x};
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                n[s] += dot3(sub3(f3{x[(k >> 2) & 1], y[(k >> 1) & 1], z[k & 1]}, point), normal) >= eps ? 0.125f : 0.0f;
-        }
-        vl = n[0];
-        vr = n[1];
-    }
+    const f3 point = P.point;
     LightPair R;
+    R.cx = __ffma2_rn(half, make_float2(a.x, a.y), make_float2(-point.x, -point.x));
+    R.cy = __ffma2_rn(half, make_float2(a.z, a.w), make_float2(-point.y, -point.y));
+    R.cz = __ffma2_rn(half, make_float2(b.x, b.y), make_float2(-point.z, -point.z));
+    R.ee = make_float2(b.z, b.w);
     R.power = make_float2(d.x, d.y);
-    R.dist = make_float2(dl, dr);
-    R.vis = make_float2(vl, vr);
     R.left = __float_as_int(d.z);
     R.right = __float_as_int(d.w);
+    if (P.ax >= 0) {
+        const float4 w = __ldg(q + 3 + P.ax);
+        const float2 s2 = make_float2(P.sg, P.sg), p2 = make_float2(P.sp, P.sp);
+        const float2 u = __ffma2_rn(make_float2(w.x, w.y), s2, p2), v = __ffma2_rn(make_float2(w.z, w.w), s2, p2);
+        R.vis.x = (u.x >= eps ? 0.5f : 0.0f) + (v.x >= eps ? 0.5f : 0.0f);
+        R.vis.y = (u.y >= eps ? 0.5f : 0.0f) + (v.y >= eps ? 0.5f : 0.0f);
+    } else {
+        const float4 x = __ldg(q + 3), y = __ldg(q + 4), z = __ldg(q + 5);
+        float n[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float2 kx = (k & 4) ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
+            const float2 ky = (k & 2) ? make_float2(y.z, y.w) : make_float2(y.x, y.y);
+            const float2 kz = (k & 1) ? make_float2(z.z, z.w) : make_float2(z.x, z.y);
+            n[0] += dot3(sub3(f3{kx.x, ky.x, kz.x}, point), P.normal) >= eps ? 0.125f : 0.0f;
+            n[1] += dot3(sub3(f3{kx.y, ky.y, kz.y}, point), P.normal) >= eps ? 0.125f : 0.0f;
+        }
+        R.vis = make_float2(n[0], n[1]);
+    }
     return R;
 }
 
@@ -168,21 +163,18 @@ __device__ Descent light_descent(const DevScene &sc, f3 point, f3 normal, uint32
                 continue;
             }
         }
-        // left iff rnd < lI / (lI + rI), in the shader's rounded divisions.
-        // Quotients within 2 ulp (__fdividef) decide it when the sides of
-        // rnd * (lI + rI) < lI are more than 2^-16 apart, far beyond their
-        // error (below 2^-20 for sums in this range); else the exact ones do.
-        // Only the chosen importance's sign is used, and a child chosen with
-        // certainty has one far above the underflow.  (Three divisions fewer per
-        // level: the shading of bounce 0 at 1080p 137 -> 130 us, the frame in
-        // flight 1022 -> 1014 us.)
+        // left iff rnd < lI / (lI + rI), in the shader's rounded arithmetic.
+        // Values within 2^-20 decide it when the sides of rnd * (lI + rI) < lI
+        // are more than 2^-16 of the sum apart (and the sum far from over- and
+        // underflow); else the exact ones do.  Only the sign of the chosen
+        // importance is used, and a child chosen so has over 2^-16 of the sum.
         const LightPair c = light_pair<false>(sc, P, (uint32_t)ref);
         const float rnd = mm_rand(seed);
-        float lI = __fdividef(c.power.x, c.dist.x) * c.vis.x, rI = __fdividef(c.power.y, c.dist.y) * c.vis.y;
-        const float tot = lI + rI, at = rnd * tot;
-        bool left = at < lI * (1.0f - 1.0f / 65536.0f);
-        const bool sure = (left || at > lI * (1.0f + 1.0f / 65536.0f)) && at > 0.0f && tot > 1e-20f && tot < 1e20f;
-        if (!sure) {
+        const float2 near = c.imp_near();
+        float lI = near.x, rI = near.y;
+        const float tot = lI + rI, diff = __fmaf_rn(rnd, tot, -lI);
+        bool left = diff < 0.0f;
+        if (!(fabsf(diff) > tot * (1.0f / 65536.0f) && tot > 1e-20f && tot < 1e20f)) {
             lI = c.imp_l();
             rI = c.imp_r();
             left = rnd < lI / (lI + rI);  // the shader's right ratio is never read

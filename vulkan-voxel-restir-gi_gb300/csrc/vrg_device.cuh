@@ -276,19 +276,20 @@ struct InstDev {
 
 // The light tree as its two walks read it, over the combined index space
 // [top level | every instance's BLAS] (world space; node j of instance k is
-// InstDev::light_base + j).  Per inner node, 64 bytes, its two children side
-// by side (L, R):
-//   0 (min.x L R, min.y L R)  1 (min.z L R, max.x L R)  2 (max.y L R, max.z L R)
-//   3 (power L R, ref L R)
-// min and max are nodeImportance's v000 and v111 (the instance transform
-// applied to the node's min and max).  A ref >= 0 is an inner node; a leaf is
-// ~instance in the top level, ~(BLAS node) below.  A top-level leaf's own
+// InstDev::light_base + j).  Per inner node, 96 bytes, its two children side
+// by side (L, R), with v000 and v111 nodeImportance's corners (the instance
+// transform applied to the node's min and max) and e = v111 - v000:
+//   0 (v000.x + v111.x L R, the same of y L R)  1 (the same of z L R, |e|^2 L R)
+//   2 (power L R, ref L R)  3..5 per axis (v000 L R, v111 L R)
+// A walk reads 0..2 and the axis of its normal: four 16-byte loads for both
+// children's importance, against ten 8-byte loads of two 40-byte nodes, and
+// packed arithmetic (f32x2) for the pair.  A ref >= 0 is an inner node; a leaf
+// is ~instance in the top level, ~(BLAS node) below.  A top-level leaf's own
 // slot holds its instance's BLAS root as L.  light_par: parent << 1 | (is the
 // right child), INVALID at the top; a BLAS root's parent is its top-level
-// leaf's.  Both children's importance then takes four 16-byte loads of one
-// 64-byte line instead of ten 8-byte loads of two 40-byte nodes, and packed
-// arithmetic (f32x2) for the pair; the way up follows light_par alone.
-constexpr int LIGHT_PAIR = 4;  // float4 per node
+// leaf's; the way up follows light_par alone.  (The shading of bounce 0 at
+// 1080p: 159 us with the 40-byte nodes, 110 now.)
+constexpr int LIGHT_PAIR = 6;  // float4 per node
 
 // The instance transform applied to a point: a translation exactly (p + t),
 // any other row-major 3x4 [R|t] as ((r0*x + r1*y) + r2*z) + t per row — the
