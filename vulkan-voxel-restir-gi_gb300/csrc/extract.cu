@@ -347,7 +347,7 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
         const ChunkSummary &cs = batch[c]->sum;
         if (cs.n_light) {
             tree_node_off[2 * c + 1] = (uint32_t)node_cursor;
-            trees.push_back(SahTree{cs.n_light, (uint32_t)tot_geo + light_off[c], (uint32_t)node_cursor, 0});
+            trees.push_back(SahTree{cs.n_light, (uint32_t)tot_geo + light_off[c], (uint32_t)node_cursor, SAH_POWER});
             node_cursor += 2 * (uint64_t)cs.n_light - 1;
         }
     }

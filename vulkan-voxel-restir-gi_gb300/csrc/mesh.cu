@@ -127,7 +127,7 @@ vrg_status mesh_upload(Context *ctx, const vrg_vertex3d *v, uint64_t nverts, Obj
     VRG_CUDA_TRY(cudaMemcpyAsync(B + o_cen, cen.data(), (size_t)np * 16, cudaMemcpyHostToDevice, s));
     VRG_CUDA_TRY(cudaMemcpyAsync(B + o_id, ids.data(), (size_t)np * 4, cudaMemcpyHostToDevice, s));
     std::vector<SahTree> trees{SahTree{n, 0, 0, 0}};
-    if (nl) trees.push_back(SahTree{nl, n, n_geo_nodes, 0});
+    if (nl) trees.push_back(SahTree{nl, n, n_geo_nodes, SAH_POWER});
     SahInputs in{(const float4 *)(B + o_lo), (const float4 *)(B + o_hi), (const float4 *)(B + o_cen),
                  (const uint32_t *)(B + o_id)};
     vrg_bvh_node *nodes = (vrg_bvh_node *)(B + o_nodes);

@@ -513,7 +513,7 @@ vrg_status standalone_sah(Context *ctx, bool tri, uint32_t count, const uint32_t
     uint64_t total_prims = 0, total_nodes = 0;
     std::vector<SahTree> trees(count);
     for (uint32_t t = 0; t < count; t++) {
-        trees[t] = SahTree{n[t], prim_offset[t], node_offset[t], 0};
+        trees[t] = SahTree{n[t], prim_offset[t], node_offset[t], SAH_POWER};
         total_prims = std::max<uint64_t>(total_prims, (uint64_t)prim_offset[t] + n[t]);
         if (n[t]) total_nodes = std::max<uint64_t>(total_nodes, (uint64_t)node_offset[t] + 2 * (uint64_t)n[t] - 1);
     }
@@ -798,7 +798,7 @@ vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint3
         for (auto &cp : cps) {
             tin.insert(tin.end(), cp.tl_in.begin(), cp.tl_in.end());
             tid.insert(tid.end(), cp.tl_ids.begin(), cp.tl_ids.end());
-            if (cp.n_light_inst) trees.push_back(SahTree{cp.n_light_inst, cp.tl_prim_off, cp.tl_node_off, 0});
+            if (cp.n_light_inst) trees.push_back(SahTree{cp.n_light_inst, cp.tl_prim_off, cp.tl_node_off, SAH_POWER});
             if (cp.n_geo_inst)
                 trees.push_back(SahTree{cp.n_geo_inst, cp.tl_prim_off + cp.n_light_inst,
                                         cp.tl_node_off + cp.n_light_tl, 0});

@@ -55,8 +55,9 @@ struct SahTree {
     uint32_t n;          // prims
     uint32_t prim_off;   // into the prim arrays
     uint32_t node_off;   // into the node array (2n-1 nodes)
-    uint32_t pad;
+    uint32_t flags;      // SAH_POWER: leaf powers (SahInputs::cen.w) may differ from 0
 };
+constexpr uint32_t SAH_POWER = 1u;
 struct SahInputs {
     const float4 *lo;    // prim AABB min (xyz)
     const float4 *hi;    // prim AABB max (xyz)
