@@ -35,11 +35,12 @@ DevBuf::~DevBuf() {
     if (ptr) cudaFreeAsync(ptr, stream);
 }
 
-vrg_status dev_alloc(cudaStream_t s, size_t bytes, DevBufPtr &out) {
+static vrg_status dev_alloc_from(cudaMemPool_t pool, cudaStream_t s, size_t bytes, DevBufPtr &out) {
     auto b = std::make_shared<DevBuf>();
     b->stream = s;
     b->bytes = bytes;
-    cudaError_t e = cudaMallocAsync(&b->ptr, bytes ? bytes : 16, s);
+    const size_t n = bytes ? bytes : 16;
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&b->ptr, n, pool, s) : cudaMallocAsync(&b->ptr, n, s);
     if (e != cudaSuccess) {
         cudaGetLastError();  // a failed allocation is reported here, not by the next launch check
         b->ptr = nullptr;
@@ -48,6 +49,10 @@ vrg_status dev_alloc(cudaStream_t s, size_t bytes, DevBufPtr &out) {
     }
     out = b;
     return VRG_OK;
+}
+vrg_status dev_alloc(cudaStream_t s, size_t bytes, DevBufPtr &out) { return dev_alloc_from(nullptr, s, bytes, out); }
+vrg_status dev_alloc(Context *ctx, size_t bytes, DevBufPtr &out) {
+    return dev_alloc_from(ctx->pool, ctx->stream, bytes, out);
 }
 
 static void release_object(Object *o) {
@@ -71,6 +76,8 @@ void ctx_release(Context *c) {
     c->d_mats.reset();
     c->d_atlas.reset();
     cudaStreamSynchronize(c->stream);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
     cudaStreamDestroy(c->stream);
     delete static_cast<vrg_context *>(c);
 }
@@ -128,8 +135,23 @@ VRG_API vrg_status vrg_context_create(const vrg_context_desc *desc, vrg_context 
         return VRG_ERR_CUDA;
     }
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
+    {  // (without a pool of its own the context allocates from the device's)
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = POOL_KEEP;
+        if (cudaMemPoolCreate(&c->pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            c->pool = nullptr;
+        } else {
+            cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+    }
     vrg_status st = upload_frames(c->stream);
     if (st != VRG_OK) {
+        if (c->pool) cudaMemPoolDestroy(c->pool);
         cudaStreamDestroy(c->stream);
         delete c;
         return st;
@@ -258,11 +280,17 @@ VRG_API vrg_status vrg_upload_chunk(vrg_context *ctx, const uint8_t *blocks, con
         return VRG_ERR_STATE;
     }
     const uint32_t air = ctx->n_types;
-    for (uint32_t i = 0; i < VRG_CHUNK_BLOCKS; i++)
-        if (blocks[i] > air) {
-            set_error("block id %u at %u exceeds air id %u", blocks[i], i, air);
-            return VRG_ERR_INVALID_ARGUMENT;
-        }
+    auto highest = [](const uint8_t *b, uint32_t n) {  // (a plain maximum, so that it vectorizes)
+        uint8_t m = 0;
+        for (uint32_t i = 0; i < n; i++) m = b[i] > m ? b[i] : m;
+        return (uint32_t)m;
+    };
+    if (highest(blocks, VRG_CHUNK_BLOCKS) > air) {
+        uint32_t i = 0;
+        while (blocks[i] <= air) i++;
+        set_error("block id %u at %u exceeds air id %u", blocks[i], i, air);
+        return VRG_ERR_INVALID_ARGUMENT;
+    }
     vrg_object *o = new vrg_object();
     o->ctx = ctx;
     ctx_retain(ctx);
@@ -273,25 +301,20 @@ VRG_API vrg_status vrg_upload_chunk(vrg_context *ctx, const uint8_t *blocks, con
         if (!nb) continue;
         o->slab_present |= 1u << f;
         uint8_t *s = o->slabs.data() + f * 1024;
-        for (int a = 0; a < 32; a++)
-            for (int b = 0; b < 32; b++) {
-                uint32_t idx;
-                switch (f) {  // the neighbour's boundary plane facing this chunk
-                case 0: idx = 31 * 1024 + a * 32 + b; break;  // left: x=31, (y,z)
-                case 1: idx = 0 * 1024 + a * 32 + b; break;   // right: x=0
-                case 2: idx = a * 1024 + 31 * 32 + b; break;  // down: y=31, (x,z)
-                case 3: idx = a * 1024 + 0 * 32 + b; break;   // up: y=0
-                case 4: idx = a * 1024 + b * 32 + 31; break;  // back: z=31, (x,y)
-                default: idx = a * 1024 + b * 32 + 0; break;  // front: z=0
-                }
-                uint8_t v = nb[idx];
-                if (v > air) {
-                    delete o;
-                    set_error("neighbour %d block id %u exceeds air id %u", f, v, air);
-                    return VRG_ERR_INVALID_ARGUMENT;
-                }
-                s[a * 32 + b] = v;
-            }
+        // the neighbour's boundary plane facing this chunk
+        if (f < 2) {  // left: x=31, right: x=0, (y,z)
+            memcpy(s, nb + (f == 0 ? 31 * 1024 : 0), 1024);
+        } else if (f < 4) {  // down: y=31, up: y=0, (x,z)
+            for (int a = 0; a < 32; a++) memcpy(s + a * 32, nb + a * 1024 + (f == 2 ? 31 * 32 : 0), 32);
+        } else {  // back: z=31, front: z=0, (x,y)
+            for (int a = 0; a < 1024; a++) s[a] = nb[a * 32 + (f == 4 ? 31 : 0)];
+        }
+        const uint32_t v = highest(s, 1024);
+        if (v > air) {
+            delete o;
+            set_error("neighbour %d block id %u exceeds air id %u", f, v, air);
+            return VRG_ERR_INVALID_ARGUMENT;
+        }
     }
     o->refs = 2;  // caller + pending list
     {

@@ -21,29 +21,31 @@ namespace {
 
 constexpr int CHUNK_BYTES = VRG_CHUNK_BLOCKS + 6 * 1024;  // blocks + 6 neighbour planes
 
+// Masks of a chunk's rows: a row is the 32 blocks z = 0..31 of (x, y), one
+// thread's share, and its masks are 32-bit words with bit z.
 struct ExtractArgs {
     const uint8_t *in;           // [n_chunks][CHUNK_BYTES]
-    uint8_t *masks;              // [n_chunks][32768]
-    uint32_t *counts;            // [n_chunks][4]: faces, light faces, surface blocks, pad
+    uint32_t *rows;              // [n_chunks][6][1024]: exposed faces f of row x * 32 + y
+    uint32_t *counts;            // [n_chunks][4]: faces, light faces, surface blocks, lamp blocks
     const vrg_material *mats;
     uint32_t air;
 };
 
-__device__ __forceinline__ bool translucent(const vrg_material *mats, uint32_t air, uint32_t b) {
-    if (b == air) return true;
-    return (mats[6u * b].flags & VRG_MAT_TRANSLUCENT) != 0u;
-}
-
-// neighbour block id across face f of block (x,y,z) (chunk.rs:170-205)
-__device__ __forceinline__ uint32_t neighbour(const uint8_t *blk, const uint8_t *slabs, int x, int y, int z, int f) {
-    switch (f) {
-    case 0: return x == 0 ? slabs[0 * 1024 + y * 32 + z] : blk[(x - 1) * 1024 + y * 32 + z];
-    case 1: return x == 31 ? slabs[1 * 1024 + y * 32 + z] : blk[(x + 1) * 1024 + y * 32 + z];
-    case 2: return y == 0 ? slabs[2 * 1024 + x * 32 + z] : blk[x * 1024 + (y - 1) * 32 + z];
-    case 3: return y == 31 ? slabs[3 * 1024 + x * 32 + z] : blk[x * 1024 + (y + 1) * 32 + z];
-    case 4: return z == 0 ? slabs[4 * 1024 + x * 32 + y] : blk[x * 1024 + y * 32 + z - 1];
-    default: return z == 31 ? slabs[5 * 1024 + x * 32 + y] : blk[x * 1024 + y * 32 + z + 1];
+// which of a row's 32 blocks (16-byte aligned) are translucent (air is), and
+// which are air; tbits: the translucent block ids
+__device__ __forceinline__ uint32_t row_translucent(const uint8_t *row, const uint32_t *tbits, uint32_t air,
+                                                    uint32_t *is_air) {
+    const uint4 a = *reinterpret_cast<const uint4 *>(row), b = *reinterpret_cast<const uint4 *>(row + 16);
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t t = 0, e = 0;
+#pragma unroll
+    for (int z = 0; z < 32; z++) {
+        const uint32_t id = (w[z >> 2] >> (8 * (z & 3))) & 255u;
+        t |= ((tbits[id >> 5] >> (id & 31u)) & 1u) << z;
+        e |= (id == air ? 1u : 0u) << z;
     }
+    if (is_air) *is_air = e;
+    return t;
 }
 
 __device__ __forceinline__ uint32_t block_reduce_add(uint32_t v, uint32_t *sh) {
@@ -88,43 +90,72 @@ __device__ __forceinline__ uint32_t block_exscan(uint32_t v, uint32_t *sh) {
     return r;
 }
 
+// The exposed faces (chunk.rs:170-205) of a chunk, a thread per row: a face is
+// exposed when the block across it is translucent, so a row's faces are word
+// operations on its own and its four neighbour rows' translucency masks, and
+// shifts of its own along z.  (Block by block, with six byte loads each, the
+// kernel took 54 us for one chunk, the latency of its loads; now 13.)
 __global__ void __launch_bounds__(1024) k_extract_masks(ExtractArgs a) {
-    __shared__ uint32_t sh[33];
+    __shared__ uint32_t sh[33], s_tbits[8], s_rows[1024];
+    __shared__ uint8_t s_lum[256];  // per block id: its luminous faces
     const uint8_t *in = a.in + (size_t)blockIdx.x * CHUNK_BYTES;
     const uint8_t *slabs = in + VRG_CHUNK_BLOCKS;
-    uint8_t *masks = a.masks + (size_t)blockIdx.x * VRG_CHUNK_BLOCKS;
+    uint32_t *rows = a.rows + (size_t)blockIdx.x * 6 * 1024;
     const int t = threadIdx.x, x = t >> 5, y = t & 31;
-    uint32_t faces = 0, lfaces = 0, surf = 0;
-    for (int z = 0; z < 32; z++) {
-        uint32_t bi = (uint32_t)(t * 32 + z);
-        uint32_t b = in[bi];
-        uint32_t m = 0;
-        if (b != a.air) {
-            for (int f = 0; f < 6; f++) {
-                if (translucent(a.mats, a.air, neighbour(in, slabs, x, y, z, f))) {
-                    m |= 1u << f;
-                    if (a.mats[6u * b + (uint32_t)f].luminance > 0.0f) lfaces++;
-                }
-            }
-        }
-        faces += __popc(m);
-        surf += m ? 1u : 0u;
-        masks[bi] = (uint8_t)m;
+    if (t < 256) {
+        const bool known = (uint32_t)t < a.air;
+        const uint32_t m = __ballot_sync(0xffffffffu, (uint32_t)t == a.air ||
+                                                          (known && (a.mats[6u * t].flags & VRG_MAT_TRANSLUCENT)));
+        if ((t & 31) == 0) s_tbits[t >> 5] = m;
+        uint32_t l = 0;
+        if (known)
+            for (uint32_t f = 0; f < 6; f++) l |= (a.mats[6u * t + f].luminance > 0.0f ? 1u : 0u) << f;
+        s_lum[t] = (uint8_t)l;
     }
-    uint32_t F = block_reduce_add(faces, sh);
-    uint32_t Lf = block_reduce_add(lfaces, sh);
-    uint32_t S = block_reduce_add(surf, sh);
+    __syncthreads();
+    uint32_t air = 0;
+    const uint32_t own = row_translucent(in + t * 32, s_tbits, a.air, &air);
+    s_rows[t] = own;
+    __syncthreads();
+    const uint32_t back = slabs[4 * 1024 + t], front = slabs[5 * 1024 + t];
+    uint32_t m[6];
+    m[0] = x == 0 ? row_translucent(slabs + y * 32, s_tbits, a.air, nullptr) : s_rows[t - 32];
+    m[1] = x == 31 ? row_translucent(slabs + 1024 + y * 32, s_tbits, a.air, nullptr) : s_rows[t + 32];
+    m[2] = y == 0 ? row_translucent(slabs + 2 * 1024 + x * 32, s_tbits, a.air, nullptr) : s_rows[t - 1];
+    m[3] = y == 31 ? row_translucent(slabs + 3 * 1024 + x * 32, s_tbits, a.air, nullptr) : s_rows[t + 1];
+    m[4] = (own << 1) | ((s_tbits[back >> 5] >> (back & 31u)) & 1u);
+    m[5] = (own >> 1) | (((s_tbits[front >> 5] >> (front & 31u)) & 1u) << 31);
+    uint32_t any = 0, faces = 0, lfaces = 0, lamps = 0;
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+        m[f] &= ~air;
+        rows[f * 1024 + t] = m[f];
+        any |= m[f];
+        faces += __popc(m[f]);
+    }
+    for (uint32_t s = any; s; s &= s - 1u) {
+        const int z = __ffs(s) - 1;
+        uint32_t l = s_lum[in[t * 32 + z]];
+#pragma unroll
+        for (int f = 0; f < 6; f++) l &= ~((~m[f] >> z & 1u) << f);
+        lfaces += __popc(l);
+        lamps += l ? 1u : 0u;
+    }
+    const uint32_t F = block_reduce_add(faces, sh);
+    const uint32_t Lf = block_reduce_add(lfaces, sh);
+    const uint32_t S = block_reduce_add(__popc(any), sh);
+    const uint32_t Lb = block_reduce_add(lamps, sh);
     if (t == 0) {
         a.counts[4 * blockIdx.x + 0] = F;
         a.counts[4 * blockIdx.x + 1] = Lf;
         a.counts[4 * blockIdx.x + 2] = S;
-        a.counts[4 * blockIdx.x + 3] = 0;
+        a.counts[4 * blockIdx.x + 3] = Lb;
     }
 }
 
 struct WriteArgs {
     const uint8_t *in;
-    const uint8_t *masks;
+    const uint32_t *rows;
     const vrg_material *mats;
     uint32_t air;
     const uint32_t *geo_off;     // [n_chunks] prim offset of the chunk's geometry prims
@@ -143,30 +174,33 @@ __global__ void __launch_bounds__(1024) k_extract_write(WriteArgs a) {
     __shared__ uint32_t sh[33];
     const uint32_t c = blockIdx.x;
     const uint8_t *in = a.in + (size_t)c * CHUNK_BYTES;
-    const uint8_t *masks = a.masks + (size_t)c * VRG_CHUNK_BLOCKS;
     const int t = threadIdx.x;
-    uint32_t faces = 0, lfaces = 0, surf = 0;
-    for (int z = 0; z < 32; z++) {
-        uint32_t bi = (uint32_t)(t * 32 + z);
-        uint32_t m = masks[bi];
-        if (!m) continue;
-        uint32_t b = in[bi];
-        faces += __popc(m);
-        surf++;
-        for (int f = 0; f < 6; f++)
-            if ((m >> f) & 1u)
-                if (a.mats[6u * b + (uint32_t)f].luminance > 0.0f) lfaces++;
+    uint32_t row[6], any = 0, faces = 0, lfaces = 0;
+    for (int f = 0; f < 6; f++) {
+        row[f] = a.rows[((size_t)c * 6 + f) * 1024 + t];
+        any |= row[f];
+        faces += __popc(row[f]);
+    }
+    auto mask_at = [&](int z) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int f = 0; f < 6; f++) m |= ((row[f] >> z) & 1u) << f;
+        return m;
+    };
+    for (uint32_t s = any; s; s &= s - 1u) {
+        const int z = __ffs(s) - 1;
+        const uint32_t b = in[t * 32 + z];
+        for (uint32_t m = mask_at(z); m; m &= m - 1u)
+            if (a.mats[6u * b + (uint32_t)__ffs(m) - 1u].luminance > 0.0f) lfaces++;
     }
     uint32_t face_base = block_exscan(faces, sh);
     uint32_t lface_base = block_exscan(lfaces, sh);
-    uint32_t surf_base = block_exscan(surf, sh);
+    uint32_t surf_base = block_exscan(__popc(any), sh);
     const int x = t >> 5, y = t & 31;
     const uint32_t goff = a.geo_off[c], loff = a.light_off[c], gl = a.loc_off[c], ll = a.lloc_off[c];
-    for (int z = 0; z < 32; z++) {
-        uint32_t bi = (uint32_t)(t * 32 + z);
-        uint32_t m = masks[bi];
-        if (!m) continue;
-        uint32_t b = in[bi];
+    for (uint32_t s = any; s; s &= s - 1u) {
+        const int z = __ffs(s) - 1;
+        const uint32_t bi = (uint32_t)(t * 32 + z), m = mask_at(z), b = in[bi];
         uint32_t first_tri = 2u * face_base;
         // geometry prim: block AABB, centroid (min+max)/2 (build.rs:391-400)
         {
@@ -216,13 +250,39 @@ __global__ void __launch_bounds__(1024) k_extract_write(WriteArgs a) {
     }
 }
 
-// per light node: leaf payload (the triangle of the leaf's prim)
-__global__ void k_light_leaf_payload(const uint32_t *leaf_prim, const uint32_t *light_tri, uint32_t *payload,
-                                     uint32_t n_nodes) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_nodes) return;
-    uint32_t p = leaf_prim[i];
-    payload[i] = (p == INVALID) ? INVALID : light_tri[p];
+// A chunk's trees in the flush's arrays: nodes (INVALID: none) and first prims
+// of its geometry and light trees, light nodes, and its light_tri offset.
+struct ChunkTrees {
+    uint32_t node_off[2], prim_off[2], n_light_nodes, light_off, payload_off, pad;
+};
+// What the host keeps of a tree's root (build_bl_bvh return convention,
+// build.rs:359-371): of a leaf root, its prim's own bounds and power.
+struct RootSummary {
+    float lo[3], hi[3], power;
+};
+
+// per light node: the triangle of the leaf's prim; blockIdx.y is the chunk,
+// whose first two threads also sum up its roots
+__global__ void __launch_bounds__(256) k_chunk_finish(const ChunkTrees *trees, const vrg_bvh_node *nodes,
+                                                      const uint32_t *leaf_prim, const uint32_t *light_tri,
+                                                      SahInputs in, uint32_t *payload, RootSummary *roots) {
+    const ChunkTrees C = trees[blockIdx.y];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < C.n_light_nodes) {
+        const uint32_t p = leaf_prim[C.node_off[1] + i];
+        payload[C.payload_off + i] = (p == INVALID) ? INVALID : light_tri[C.light_off + p];
+    }
+    if (i < 2 && C.node_off[i] != INVALID) {
+        const vrg_bvh_node n = nodes[C.node_off[i]];
+        RootSummary r;
+        if (n.left_node_idx == INVALID) {
+            const float4 l = in.lo[C.prim_off[i]], h = in.hi[C.prim_off[i]];
+            r = RootSummary{{l.x, l.y, l.z}, {h.x, h.y, h.z}, in.cen[C.prim_off[i]].w};
+        } else {
+            r = RootSummary{{n.min[0], n.min[1], n.min[2]}, {n.max[0], n.max[1], n.max[2]}, n.power};
+        }
+        roots[2 * blockIdx.y + i] = r;
+    }
 }
 
 }  // namespace
@@ -235,26 +295,49 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
         set_error("too many chunks in one flush (%u)", nc);
         return VRG_ERR_UNSUPPORTED;
     }
-    // stage blocks + neighbour planes
-    size_t in_bytes = (size_t)nc * CHUNK_BYTES;
-    uint8_t *h_in = nullptr;
-    VRG_CUDA_TRY(cudaMallocHost(&h_in, in_bytes + 16 * (size_t)nc));
-    std::unique_ptr<uint8_t, void (*)(uint8_t *)> h_guard(h_in, [](uint8_t *x) { cudaFreeHost(x); });
+    // stage blocks + neighbour planes; the same page-locked buffer takes the
+    // counts, the trees' places and the roots (all copies in and out of one
+    // flush, ended by its last synchronization)
+    const size_t in_bytes = (size_t)nc * CHUNK_BYTES, cnt_bytes = 16 * (size_t)nc;
+    const size_t plan_bytes = nc * (16 + sizeof(ChunkTrees)), out_bytes = 2 * nc * sizeof(RootSummary) + 16;
+    const size_t stage_bytes = in_bytes + cnt_bytes + plan_bytes + out_bytes;
+    if (ctx->h_stage_bytes < stage_bytes) {
+        if (ctx->h_stage) {
+            cudaStreamSynchronize(s);
+            cudaFreeHost(ctx->h_stage);
+        }
+        ctx->h_stage = nullptr;
+        ctx->h_stage_bytes = 0;
+        VRG_CUDA_TRY(cudaMallocHost(&ctx->h_stage, stage_bytes));
+        ctx->h_stage_bytes = stage_bytes;
+    }
+    // (given back after a flush of many chunks, also when it fails)
+    struct StageGuard {
+        Context *c;
+        ~StageGuard() {
+            if (c->h_stage_bytes <= Context::STAGE_KEEP) return;
+            cudaStreamSynchronize(c->stream);
+            cudaFreeHost(c->h_stage);
+            c->h_stage = nullptr;
+            c->h_stage_bytes = 0;
+        }
+    } guard{ctx};
+    uint8_t *h_in = ctx->h_stage;
     for (uint32_t c = 0; c < nc; c++) {
         memcpy(h_in + (size_t)c * CHUNK_BYTES, batch[c]->blocks.data(), VRG_CHUNK_BLOCKS);
         memcpy(h_in + (size_t)c * CHUNK_BYTES + VRG_CHUNK_BLOCKS, batch[c]->slabs.data(), 6 * 1024);
     }
     DevBufPtr tmp;
-    VRG_TRY(dev_alloc(s, in_bytes + (size_t)nc * VRG_CHUNK_BLOCKS + 16 * (size_t)nc, tmp));
+    VRG_TRY(dev_alloc(ctx, in_bytes + (size_t)nc * 6 * 1024 * 4 + cnt_bytes, tmp));
     uint8_t *d_in = (uint8_t *)tmp->ptr;
-    uint8_t *d_masks = d_in + in_bytes;
-    uint32_t *d_counts = (uint32_t *)(d_masks + (size_t)nc * VRG_CHUNK_BLOCKS);
+    uint32_t *d_rows = (uint32_t *)(d_in + in_bytes);
+    uint32_t *d_counts = d_rows + (size_t)nc * 6 * 1024;
     VRG_CUDA_TRY(cudaMemcpyAsync(d_in, h_in, in_bytes, cudaMemcpyHostToDevice, s));
-    ExtractArgs ea{d_in, d_masks, d_counts, (const vrg_material *)ctx->d_mats->ptr, ctx->n_types};
+    ExtractArgs ea{d_in, d_rows, d_counts, (const vrg_material *)ctx->d_mats->ptr, ctx->n_types};
     k_extract_masks<<<nc, 1024, 0, s>>>(ea);
     VRG_CUDA_TRY(cudaGetLastError());
     uint32_t *h_counts = (uint32_t *)(h_in + in_bytes);
-    VRG_CUDA_TRY(cudaMemcpyAsync(h_counts, d_counts, 16 * (size_t)nc, cudaMemcpyDeviceToHost, s));
+    VRG_CUDA_TRY(cudaMemcpyAsync(h_counts, d_counts, cnt_bytes, cudaMemcpyDeviceToHost, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
 
     // layout of the batch: persistent arrays per object + builder inputs (temp)
@@ -268,6 +351,7 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
         cs.n_tris = 2 * F;
         cs.n_light = 2 * Lf;
         cs.n_geo = S;
+        cs.n_lamps = h_counts[4 * c + 3];
         geo_off[c] = (uint32_t)tot_geo;
         light_off[c] = (uint32_t)tot_light;
         tot_geo += S;
@@ -291,7 +375,7 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     uint64_t o_payload = o; o += al(tot_light_nodes * 4);
     uint64_t persist_bytes = o;
     DevBufPtr batch_buf;
-    VRG_TRY(dev_alloc(s, std::max<uint64_t>(persist_bytes, 256), batch_buf));
+    VRG_TRY(dev_alloc(ctx, std::max<uint64_t>(persist_bytes, 256), batch_buf));
     uint8_t *B = (uint8_t *)batch_buf->ptr;
     DevBufPtr bin;
     uint64_t ob = 0;
@@ -299,22 +383,50 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     uint64_t o_hi = ob; ob += al(n_prims * 16);
     uint64_t o_cen = ob; ob += al(n_prims * 16);
     uint64_t o_id = ob; ob += al(n_prims * 4);
-    uint64_t o_offs = ob; ob += al(4 * (uint64_t)nc * 4);
-    VRG_TRY(dev_alloc(s, std::max<uint64_t>(ob, 256), bin));
+    uint64_t o_plan = ob; ob += al(plan_bytes);
+    uint64_t o_out = ob; ob += al(out_bytes);
+    VRG_TRY(dev_alloc(ctx, std::max<uint64_t>(ob, 256), bin));
     uint8_t *I = (uint8_t *)bin->ptr;
-    // prim index space: geometry prims first, then light prims
-    std::vector<uint32_t> offs(4 * (size_t)nc);
+    // Prim index space: geometry prims first, then light prims.  One batched
+    // SAH build: geometry trees (build_tl_bvh semantics over block AABBs) and
+    // light trees (build_bl_bvh over light triangles).
+    uint32_t *offs = (uint32_t *)(h_in + in_bytes + cnt_bytes);
+    ChunkTrees *ct = (ChunkTrees *)(offs + 4 * (size_t)nc);
+    std::vector<SahTree> trees;
+    uint64_t node_cursor = 0;
+    uint32_t max_light_nodes = 0;
+    for (int k = 0; k < 2; k++)
+        for (uint32_t c = 0; c < nc; c++) {
+            const ChunkSummary &cs = batch[c]->sum;
+            const uint32_t n = k ? cs.n_light : cs.n_geo, first = k ? (uint32_t)tot_geo + light_off[c] : geo_off[c];
+            ct[c].node_off[k] = n ? (uint32_t)node_cursor : INVALID;
+            ct[c].prim_off[k] = first;
+            if (k) {
+                ct[c].n_light_nodes = n ? 2 * n - 1 : 0;
+                ct[c].light_off = light_off[c];
+                ct[c].payload_off = (uint32_t)(node_cursor - tot_geo_nodes);
+                ct[c].pad = 0;
+                max_light_nodes = std::max(max_light_nodes, ct[c].n_light_nodes);
+            }
+            if (!n) continue;
+            trees.push_back(SahTree{n, first, (uint32_t)node_cursor, k ? SAH_POWER : 0u});
+            node_cursor += 2 * (uint64_t)n - 1;
+        }
     for (uint32_t c = 0; c < nc; c++) {
         offs[c] = geo_off[c];
         offs[nc + c] = (uint32_t)tot_geo + light_off[c];
         offs[2 * nc + c] = geo_off[c];
         offs[3 * nc + c] = light_off[c];
     }
-    uint32_t *d_offs = (uint32_t *)(I + o_offs);
-    VRG_CUDA_TRY(cudaMemcpyAsync(d_offs, offs.data(), offs.size() * 4, cudaMemcpyHostToDevice, s));
+    uint32_t *d_offs = (uint32_t *)(I + o_plan);
+    const ChunkTrees *d_ct = (const ChunkTrees *)(d_offs + 4 * (size_t)nc);
+    RootSummary *d_roots = (RootSummary *)(I + o_out);
+    uint32_t *d_levels = (uint32_t *)(d_roots + 2 * (size_t)nc);
+    VRG_CUDA_TRY(cudaMemcpyAsync(d_offs, offs, plan_bytes, cudaMemcpyHostToDevice, s));
+    VRG_CUDA_TRY(cudaMemsetAsync(d_levels, 0, 4, s));
     WriteArgs wa;
     wa.in = d_in;
-    wa.masks = d_masks;
+    wa.rows = d_rows;
     wa.mats = (const vrg_material *)ctx->d_mats->ptr;
     wa.air = ctx->n_types;
     wa.geo_off = d_offs;
@@ -330,58 +442,19 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     k_extract_write<<<nc, 1024, 0, s>>>(wa);
     VRG_CUDA_TRY(cudaGetLastError());
 
-    // one batched SAH build: geometry trees (build_tl_bvh semantics over block
-    // AABBs) and light trees (build_bl_bvh over light triangles)
-    std::vector<SahTree> trees;
-    std::vector<uint32_t> tree_node_off(2 * (size_t)nc, INVALID);
-    uint64_t node_cursor = 0;
-    for (uint32_t c = 0; c < nc; c++) {
-        const ChunkSummary &cs = batch[c]->sum;
-        if (cs.n_geo) {
-            tree_node_off[2 * c] = (uint32_t)node_cursor;
-            trees.push_back(SahTree{cs.n_geo, geo_off[c], (uint32_t)node_cursor, 0});
-            node_cursor += 2 * (uint64_t)cs.n_geo - 1;
-        }
-    }
-    for (uint32_t c = 0; c < nc; c++) {
-        const ChunkSummary &cs = batch[c]->sum;
-        if (cs.n_light) {
-            tree_node_off[2 * c + 1] = (uint32_t)node_cursor;
-            trees.push_back(SahTree{cs.n_light, (uint32_t)tot_geo + light_off[c], (uint32_t)node_cursor, SAH_POWER});
-            node_cursor += 2 * (uint64_t)cs.n_light - 1;
-        }
-    }
     SahInputs sin{wa.lo, wa.hi, wa.cen, wa.id};
     SahOutputs sout{(vrg_bvh_node *)(B + o_nodes), (uint32_t *)(B + o_perm), (uint32_t *)(B + o_leaf)};
     uint32_t levels = 0;
-    VRG_TRY(sah_build(s, trees, (uint32_t)n_prims, (uint32_t)n_nodes, sin, sout, &levels));
-    // leaf payloads of the light trees
-    for (uint32_t c = 0; c < nc; c++) {
-        const ChunkSummary &cs = batch[c]->sum;
-        if (!cs.n_light) continue;
-        uint32_t nn = 2 * cs.n_light - 1;
-        uint32_t off = tree_node_off[2 * c + 1];
-        uint32_t payload_off = off - (uint32_t)tot_geo_nodes;
-        k_light_leaf_payload<<<(nn + 255) / 256, 256, 0, s>>>(sout.leaf_prim + off, wa.light_tri + light_off[c],
-                                                             (uint32_t *)(B + o_payload) + payload_off, nn);
-    }
+    VRG_TRY(sah_build(ctx, trees, (uint32_t)n_prims, (uint32_t)n_nodes, sin, sout, &levels, d_levels));
+    k_chunk_finish<<<dim3((std::max(2u, max_light_nodes) + 255) / 256, nc), 256, 0, s>>>(
+        d_ct, sout.nodes, sout.leaf_prim, wa.light_tri, sin, (uint32_t *)(B + o_payload), d_roots);
     VRG_CUDA_TRY(cudaGetLastError());
-    // root summaries (build_bl_bvh return convention, build.rs:359-371)
-    std::vector<vrg_bvh_node> roots(2 * (size_t)nc);
-    std::vector<float4> first_lo(2 * (size_t)nc), first_hi(2 * (size_t)nc), first_cen(2 * (size_t)nc);
-    for (uint32_t c = 0; c < nc; c++) {
-        for (int k = 0; k < 2; k++) {
-            uint32_t off = tree_node_off[2 * c + k];
-            if (off == INVALID) continue;
-            VRG_CUDA_TRY(cudaMemcpyAsync(&roots[2 * c + k], sout.nodes + off, sizeof(vrg_bvh_node),
-                                         cudaMemcpyDeviceToHost, s));
-            uint32_t p0 = k == 0 ? geo_off[c] : (uint32_t)tot_geo + light_off[c];
-            VRG_CUDA_TRY(cudaMemcpyAsync(&first_lo[2 * c + k], wa.lo + p0, 16, cudaMemcpyDeviceToHost, s));
-            VRG_CUDA_TRY(cudaMemcpyAsync(&first_hi[2 * c + k], wa.hi + p0, 16, cudaMemcpyDeviceToHost, s));
-            VRG_CUDA_TRY(cudaMemcpyAsync(&first_cen[2 * c + k], wa.cen + p0, 16, cudaMemcpyDeviceToHost, s));
-        }
-    }
+    const RootSummary *roots = (const RootSummary *)(h_in + in_bytes + cnt_bytes + plan_bytes);
+    VRG_CUDA_TRY(cudaMemcpyAsync((void *)roots, d_roots, out_bytes, cudaMemcpyDeviceToHost, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    uint32_t lv_dev;
+    memcpy(&lv_dev, roots + 2 * (size_t)nc, 4);
+    levels = std::max(levels, lv_dev);
     for (uint32_t c = 0; c < nc; c++) {
         Object *ob = batch[c];
         ChunkSummary &cs = ob->sum;
@@ -389,35 +462,22 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
         ob->geo_local = (const int2 *)(B + o_geo_local) + geo_off[c];
         ob->light_tri = (const uint32_t *)(B + o_light_tri) + light_off[c];
         if (cs.n_geo) {
-            uint32_t off = tree_node_off[2 * c];
+            const uint32_t off = ct[c].node_off[0];
             ob->geo_nodes = sout.nodes + off;
             ob->geo_leaf = sout.leaf_prim + off;
             ob->geo_perm = sout.perm + geo_off[c];
-            const vrg_bvh_node &r = roots[2 * c];
-            if (r.left_node_idx == INVALID) {
-                const float4 &l = first_lo[2 * c], &h = first_hi[2 * c];
-                cs.geo_lo[0] = l.x; cs.geo_lo[1] = l.y; cs.geo_lo[2] = l.z;
-                cs.geo_hi[0] = h.x; cs.geo_hi[1] = h.y; cs.geo_hi[2] = h.z;
-            } else {
-                for (int k = 0; k < 3; k++) { cs.geo_lo[k] = r.min[k]; cs.geo_hi[k] = r.max[k]; }
-            }
+            memcpy(cs.geo_lo, roots[2 * c].lo, 12);
+            memcpy(cs.geo_hi, roots[2 * c].hi, 12);
         }
         if (cs.n_light) {
-            uint32_t off = tree_node_off[2 * c + 1];
+            const uint32_t off = ct[c].node_off[1];
             ob->light_nodes = sout.nodes + off;
             ob->light_leaf = sout.leaf_prim + off;
             ob->light_perm = sout.perm + tot_geo + light_off[c];
             ob->light_leaf_tri = (const uint32_t *)(B + o_payload) + (off - tot_geo_nodes);
-            const vrg_bvh_node &r = roots[2 * c + 1];
-            if (r.left_node_idx == INVALID) {
-                const float4 &l = first_lo[2 * c + 1], &h = first_hi[2 * c + 1];
-                cs.light_lo[0] = l.x; cs.light_lo[1] = l.y; cs.light_lo[2] = l.z;
-                cs.light_hi[0] = h.x; cs.light_hi[1] = h.y; cs.light_hi[2] = h.z;
-                cs.light_power = first_cen[2 * c + 1].w;
-            } else {
-                for (int k = 0; k < 3; k++) { cs.light_lo[k] = r.min[k]; cs.light_hi[k] = r.max[k]; }
-                cs.light_power = r.power;
-            }
+            memcpy(cs.light_lo, roots[2 * c + 1].lo, 12);
+            memcpy(cs.light_hi, roots[2 * c + 1].hi, 12);
+            cs.light_power = roots[2 * c + 1].power;
         }
         ob->levels = levels;
         ob->flushed = true;

@@ -117,7 +117,7 @@ vrg_status mesh_upload(Context *ctx, const vrg_vertex3d *v, uint64_t nverts, Obj
     const uint64_t o_id = off; off += al((uint64_t)np * 4);
     cudaStream_t s = ctx->stream;
     DevBufPtr buf;
-    VRG_TRY(dev_alloc(s, off, buf));
+    VRG_TRY(dev_alloc(ctx, off, buf));
     uint8_t *B = (uint8_t *)buf->ptr;
     VRG_CUDA_TRY(cudaMemcpyAsync(B + o_tri, tri.data(), (size_t)n * 48, cudaMemcpyHostToDevice, s));
     VRG_CUDA_TRY(cudaMemcpyAsync(B + o_uv, uv.data(), (size_t)n * 24, cudaMemcpyHostToDevice, s));
@@ -134,7 +134,7 @@ vrg_status mesh_upload(Context *ctx, const vrg_vertex3d *v, uint64_t nverts, Obj
     uint32_t *leaf = (uint32_t *)(B + o_leaf);
     SahOutputs out{nodes, (uint32_t *)(B + o_perm), leaf};
     uint32_t levels = 0;
-    VRG_TRY(sah_build(s, trees, np, n_nodes, in, out, &levels));
+    VRG_TRY(sah_build(ctx, trees, np, n_nodes, in, out, &levels));
     // roots (build_bl_bvh's returned AABB and power, build.rs:359-371: a leaf
     // root holds its prim's unpadded AABB and power) and the light leaf payload
     // (node -> triangle index)
@@ -159,6 +159,7 @@ vrg_status mesh_upload(Context *ctx, const vrg_vertex3d *v, uint64_t nverts, Obj
     cs.n_tris = n;
     cs.n_light = nl;
     cs.n_geo = n;
+    cs.n_lamps = nl;
     for (int a = 0; a < 3; a++) {
         cs.geo_lo[a] = root[0].min[a];
         cs.geo_hi[a] = root[0].max[a];

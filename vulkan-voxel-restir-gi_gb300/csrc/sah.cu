@@ -709,8 +709,9 @@ static vrg_status tree_smem_init() {
     return VRG_OK;
 }
 
-vrg_status sah_build(cudaStream_t s, const std::vector<SahTree> &trees, uint32_t total_prims,
-                     uint32_t total_nodes, const SahInputs &in, const SahOutputs &out, uint32_t *levels) {
+vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t total_prims, uint32_t total_nodes,
+                     const SahInputs &in, const SahOutputs &out, uint32_t *levels, uint32_t *levels_dev) {
+    cudaStream_t s = ctx->stream;
     if (trees.empty() || total_prims == 0) {
         if (levels) *levels = 0;
         return VRG_OK;
@@ -733,7 +734,7 @@ vrg_status sah_build(cudaStream_t s, const std::vector<SahTree> &trees, uint32_t
     const size_t q_cap = n_large ? std::max<size_t>(n_large, (size_t)total_prims / 3 + 1) : 0;
     const size_t bytes = nt * sizeof(SahTree) + 2 * q_cap * sizeof(Item) + 64 + (size_t)total_nodes * 4;
     DevBufPtr scratch;
-    VRG_TRY(dev_alloc(s, bytes, scratch));
+    VRG_TRY(dev_alloc(ctx, bytes, scratch));
     uint8_t *p = (uint8_t *)scratch->ptr;
     SahTree *d_trees = (SahTree *)p; p += nt * sizeof(SahTree);
     Item *q0 = (Item *)p; p += q_cap * sizeof(Item);
@@ -741,12 +742,13 @@ vrg_status sah_build(cudaStream_t s, const std::vector<SahTree> &trees, uint32_t
     uint32_t *cnt = (uint32_t *)p; p += 64;
     uint32_t *arrive = (uint32_t *)p;
     VRG_CUDA_TRY(cudaMemcpyAsync(d_trees, by_size.data(), nt * sizeof(SahTree), cudaMemcpyHostToDevice, s));
-    VRG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 64, s));
+    if (!levels_dev) VRG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 64, s));
+    uint32_t *lv_dev = levels_dev ? levels_dev : cnt + 8;
     for (uint32_t a = n_large; a < nt && by_size[a].n;) {
         uint32_t b = a;
         const uint32_t n = by_size[a].n;
         while (b < nt && by_size[b].n && (nt - n_large <= TREE_ONE_WAVE || 2 * by_size[b].n > n)) b++;
-        k_sah_tree<<<b - a, TREE_THREADS, tree_smem(n), s>>>(d_trees + a, in, out, arrive, cnt + 8);
+        k_sah_tree<<<b - a, TREE_THREADS, tree_smem(n), s>>>(d_trees + a, in, out, arrive, lv_dev);
         VRG_CUDA_TRY(cudaGetLastError());
         a = b;
     }
@@ -786,7 +788,9 @@ vrg_status sah_build(cudaStream_t s, const std::vector<SahTree> &trees, uint32_t
         k_power_up<<<dim3(std::min(1024u, (max_nodes + 255) / 256), n_large), 256, 0, s>>>(d_trees, out.nodes, arrive);
         VRG_CUDA_TRY(cudaGetLastError());
     }
-    if (levels) {
+    if (levels && levels_dev) {
+        *levels = lv;
+    } else if (levels) {
         VRG_CUDA_TRY(cudaMemcpyAsync(&h_cnt, cnt + 8, 4, cudaMemcpyDeviceToHost, s));
         VRG_CUDA_TRY(cudaStreamSynchronize(s));
         *levels = std::max(lv, h_cnt);

@@ -532,7 +532,7 @@ vrg_status standalone_sah(Context *ctx, bool tri, uint32_t count, const uint32_t
     uint64_t o_nodes = o; o += al(total_nodes * sizeof(vrg_bvh_node));
     uint64_t o_leaf = o; o += al(total_nodes * 4);
     DevBufPtr b;
-    VRG_TRY(dev_alloc(s, o, b));
+    VRG_TRY(dev_alloc(ctx, o, b));
     uint8_t *B = (uint8_t *)b->ptr;
     if (tri) {
         VRG_CUDA_TRY(cudaMemcpyAsync(B + o_raw, prims, total_prims * 36, cudaMemcpyHostToDevice, s));
@@ -563,7 +563,7 @@ vrg_status standalone_sah(Context *ctx, bool tri, uint32_t count, const uint32_t
                  (const uint32_t *)(B + o_id)};
     SahOutputs out{(vrg_bvh_node *)(B + o_nodes), (uint32_t *)(B + o_perm), (uint32_t *)(B + o_leaf)};
     uint32_t levels = 0;
-    VRG_TRY(sah_build(s, trees, (uint32_t)total_prims, (uint32_t)total_nodes, in, out, &levels));
+    VRG_TRY(sah_build(ctx, trees, (uint32_t)total_prims, (uint32_t)total_nodes, in, out, &levels));
     if (nodes_out)
         VRG_CUDA_TRY(cudaMemcpyAsync(nodes_out, out.nodes, total_nodes * sizeof(vrg_bvh_node), cudaMemcpyDeviceToHost, s));
     if (order_out) VRG_CUDA_TRY(cudaMemcpyAsync(order_out, out.perm, total_prims * 4, cudaMemcpyDeviceToHost, s));
@@ -602,7 +602,6 @@ struct CommitPrep {
     uint64_t lamp_off = 0;                      // in the shared lamp build
     uint32_t n_lamps = 0;
     DevBufPtr lamp_buf;
-    uint32_t lamp_depth = 0;
     DevScene dev{};                             // installed only when the whole commit succeeds
 };
 
@@ -738,6 +737,7 @@ vrg_status commit_prepare(Scene *sc, CommitPrep &cp) {
         l.refbase = l.rbase;
         light_nodes += cs.n_light ? 2 * (uint64_t)cs.n_light - 1 : 0;
         cp.light_recs += cs.n_light;
+        cp.n_lamps += cs.n_lamps;
         cp.max_levels = std::max(cp.max_levels, o->levels);
     }
     cp.n_light_nodes_all = light_nodes;
@@ -758,14 +758,15 @@ vrg_status commit_prepare(Scene *sc, CommitPrep &cp) {
     cp.o_inst = o; o += al((uint64_t)ni * sizeof(InstDev));
     cp.o_gb = o; o += al((uint64_t)ni * sizeof(InstBuild));
     cp.o_lb = o; o += al((uint64_t)ni * sizeof(InstBuild));
-    VRG_TRY(dev_alloc(sc->ctx->stream, std::max<uint64_t>(o, 256), cp.buf));
+    VRG_TRY(dev_alloc(sc->ctx, std::max<uint64_t>(o, 256), cp.buf));
     cp.B = (uint8_t *)cp.buf->ptr;
     return VRG_OK;
 }
 
 // all scenes' top-level trees in one SAH build; fills h_light_tl / h_geo_tl
 // and each scene's device copy of its nodes ([light TL | geometry TL])
-vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint32_t *tl_levels) {
+vrg_status commit_top_levels(Context *ctx, std::vector<CommitPrep> &cps, uint32_t *tl_levels) {
+    cudaStream_t s = ctx->stream;
     uint32_t n_prims = 0, n_nodes = 0;
     for (auto &cp : cps) {
         cp.tl_prim_off = n_prims;
@@ -774,7 +775,7 @@ vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint3
         n_nodes += cp.n_light_tl + cp.n_geo_tl;
     }
     *tl_levels = 0;
-    std::vector<vrg_bvh_node> h_nodes(n_nodes);
+    std::vector<vrg_bvh_node> h_nodes(n_nodes + 1, vrg_bvh_node{});  // (the last: the trees' levels)
     if (n_prims) {
         auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
         uint64_t o = 0;
@@ -785,10 +786,10 @@ vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint3
         uint64_t o_cen = o; o += al((uint64_t)n_prims * 16);
         uint64_t o_id = o; o += al((uint64_t)n_prims * 4);
         uint64_t o_perm = o; o += al((uint64_t)n_prims * 4);
-        uint64_t o_nodes = o; o += al((uint64_t)n_nodes * sizeof(vrg_bvh_node));
+        uint64_t o_nodes = o; o += al((uint64_t)n_nodes * sizeof(vrg_bvh_node) + 4);  // and the trees' levels
         uint64_t o_leaf = o; o += al((uint64_t)n_nodes * 4);
         DevBufPtr sb;
-        VRG_TRY(dev_alloc(s, o, sb));
+        VRG_TRY(dev_alloc(ctx, o, sb));
         uint8_t *S = (uint8_t *)sb->ptr;
         std::vector<float> tin;
         std::vector<uint32_t> tid;
@@ -813,14 +814,16 @@ vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint3
                      (const uint32_t *)(S + o_id)};
         vrg_bvh_node *nodes = (vrg_bvh_node *)(S + o_nodes);
         SahOutputs out{nodes, (uint32_t *)(S + o_perm), (uint32_t *)(S + o_leaf)};
-        VRG_TRY(sah_build(s, trees, n_prims, n_nodes, in, out, tl_levels));
+        uint32_t *d_lv = (uint32_t *)(nodes + n_nodes);
+        VRG_CUDA_TRY(cudaMemsetAsync(d_lv, 0, 4, s));
+        VRG_TRY(sah_build(ctx, trees, n_prims, n_nodes, in, out, tl_levels, d_lv));
         for (auto &cp : cps) {
             vrg_bvh_node *d_tl = (vrg_bvh_node *)(cp.B + cp.o_tln);
             VRG_CUDA_TRY(cudaMemcpyAsync(d_tl, nodes + cp.tl_node_off,
                                          (size_t)(cp.n_light_tl + cp.n_geo_tl) * sizeof(vrg_bvh_node),
                                          cudaMemcpyDeviceToDevice, s));
         }
-        VRG_CUDA_TRY(cudaMemcpyAsync(h_nodes.data(), nodes, (size_t)n_nodes * sizeof(vrg_bvh_node),
+        VRG_CUDA_TRY(cudaMemcpyAsync(h_nodes.data(), nodes, (size_t)n_nodes * sizeof(vrg_bvh_node) + 4,
                                      cudaMemcpyDeviceToHost, s));
     }
     // a scene without lights gets the dummy node (BvhNode::default, bvh/mod.rs:27-38; scene.rs:276-277)
@@ -833,6 +836,7 @@ vrg_status commit_top_levels(cudaStream_t s, std::vector<CommitPrep> &cps, uint3
         VRG_CUDA_TRY(cudaMemcpyAsync(cp.B + cp.o_tln, &dummy, sizeof(dummy), cudaMemcpyHostToDevice, s));
     }
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    *tl_levels = std::max(*tl_levels, h_nodes[n_nodes].left_node_idx);
     for (auto &cp : cps) {
         const vrg_bvh_node *h = h_nodes.data() + cp.tl_node_off;
         cp.sc->h_light_tl.assign(h, h + cp.n_light_tl);
@@ -937,7 +941,10 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
 }
 
 // all scenes' lamp-block trees in one SAH build
-vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
+// (their number of lamps is known from the objects, so nothing is read back but
+// the tree levels, which arrive at the commit's end: *levels)
+vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, uint32_t *levels, uint32_t *levels_copy) {
+    cudaStream_t s = ctx->stream;
     uint64_t L = 0;
     for (auto &cp : cps) {
         cp.lamp_off = L;
@@ -953,7 +960,7 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     uint64_t o = 0;
     uint64_t o_flag = o; o += al(L * 4);
-    uint64_t o_tot = o; o += al((uint64_t)nc * 4);
+    uint64_t o_tot = o; o += al((uint64_t)nc * 4 + 4);  // lamps per scene, then the trees' levels
     uint64_t o_lo = o; o += al(L * 16);
     uint64_t o_hi = o; o += al(L * 16);
     uint64_t o_cen = o; o += al(L * 16);
@@ -962,10 +969,10 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
     uint64_t o_nodes = o; o += al(2 * L * sizeof(vrg_bvh_node));
     uint64_t o_leaf = o; o += al(2 * L * 4);
     DevBufPtr sb;
-    VRG_TRY(dev_alloc(s, o, sb));
+    VRG_TRY(dev_alloc(ctx, o, sb));
     uint8_t *S = (uint8_t *)sb->ptr;
     uint32_t *tot = (uint32_t *)(S + o_tot);
-    VRG_CUDA_TRY(cudaMemsetAsync(tot, 0, (size_t)nc * 4, s));
+    VRG_CUDA_TRY(cudaMemsetAsync(tot, 0, (size_t)nc * 4 + 4, s));
     for (uint32_t c = 0; c < nc; c++) {
         CommitPrep &cp = cps[c];
         const uint64_t n = cp.light_recs;
@@ -974,7 +981,7 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
         const uint64_t q_rec = q; q += al(n * 16);
         const uint64_t q_tab = q; q += al(n * 12 * 4);
         const uint64_t q_wide = q; q += al(2 * n * 128);
-        VRG_TRY(dev_alloc(s, q, cp.lamp_buf));
+        VRG_TRY(dev_alloc(ctx, q, cp.lamp_buf));
         uint8_t *Q = (uint8_t *)cp.lamp_buf->ptr;
         int4 *lamp = (int4 *)(Q + q_rec);
         uint32_t *table = (uint32_t *)(Q + q_tab);
@@ -994,21 +1001,16 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
         D.lamp_rec = lamp;
         D.lamp_table = table;
     }
-    std::vector<uint32_t> n_lamps(nc);
-    VRG_CUDA_TRY(cudaMemcpyAsync(n_lamps.data(), tot, (size_t)nc * 4, cudaMemcpyDeviceToHost, s));
-    VRG_CUDA_TRY(cudaStreamSynchronize(s));
     std::vector<SahTree> trees;
-    for (uint32_t c = 0; c < nc; c++) {
-        cps[c].n_lamps = n_lamps[c];
-        if (n_lamps[c]) trees.push_back(SahTree{n_lamps[c], (uint32_t)cps[c].lamp_off, 2 * (uint32_t)cps[c].lamp_off, 0});
-    }
+    for (auto &cp : cps)
+        if (cp.n_lamps) trees.push_back(SahTree{cp.n_lamps, (uint32_t)cp.lamp_off, 2 * (uint32_t)cp.lamp_off, 0});
     SahInputs in{(const float4 *)(S + o_lo), (const float4 *)(S + o_hi), (const float4 *)(S + o_cen),
                  (const uint32_t *)(S + o_id)};
     vrg_bvh_node *nodes = (vrg_bvh_node *)(S + o_nodes);
     uint32_t *leaf = (uint32_t *)(S + o_leaf);
     SahOutputs out{nodes, (uint32_t *)(S + o_perm), leaf};
-    uint32_t levels = 0;
-    VRG_TRY(sah_build(s, trees, (uint32_t)L, (uint32_t)(2 * L), in, out, &levels));
+    VRG_TRY(sah_build(ctx, trees, (uint32_t)L, (uint32_t)(2 * L), in, out, levels, tot + nc));
+    VRG_CUDA_TRY(cudaMemcpyAsync(levels_copy, tot + nc, 4, cudaMemcpyDeviceToHost, s));
     for (auto &cp : cps) {
         if (!cp.n_lamps) continue;
         DevScene &D = cp.dev;
@@ -1021,7 +1023,6 @@ vrg_status commit_lamps(cudaStream_t s, std::vector<CommitPrep> &cps) {
         } else {
             D.lamp_root = ~0;
         }
-        cp.lamp_depth = 3 * ((levels + 2 + 1) / 2) + 1;  // up to 3 pushes per 4-wide level
     }
     return VRG_OK;
 }
@@ -1061,19 +1062,22 @@ vrg_status scene_commit_many(Scene *const *scs, uint32_t n) {
     }
     if (cps.empty()) return VRG_OK;
     uint32_t tl_levels = 0;
-    VRG_TRY(commit_top_levels(s, cps, &tl_levels));
+    VRG_TRY(commit_top_levels(ctx, cps, &tl_levels));
     for (auto &cp : cps) VRG_TRY(commit_layouts(s, cp, (const vrg_bvh_node *)(cp.B + cp.o_tln)));
-    VRG_TRY(commit_lamps(s, cps));
+    uint32_t lamp_levels = 0, lamp_levels_dev = 0;
+    VRG_TRY(commit_lamps(ctx, cps, &lamp_levels, &lamp_levels_dev));
+    VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    lamp_levels = std::max(lamp_levels, lamp_levels_dev);
     for (auto &cp : cps) {
-        // the 4-wide walk pushes up to 3 refs per 4-wide level (half the binary depth)
-        const uint32_t bound = std::max(3 * ((tl_levels + cp.max_levels + 4 + 1) / 2) + 1, cp.lamp_depth);
+        // the 4-wide walks push up to 3 refs per 4-wide level (half the binary depth)
+        const uint32_t lamp_depth = cp.n_lamps ? 3 * ((lamp_levels + 2 + 1) / 2) + 1 : 0;
+        const uint32_t bound = std::max(3 * ((tl_levels + cp.max_levels + 4 + 1) / 2) + 1, lamp_depth);
         if (bound >= (uint32_t)TRAV_STACK) {
             set_error("BVH depth bound %u exceeds the traversal stack (%d)", bound, TRAV_STACK);
             return VRG_ERR_UNSUPPORTED;
         }
         cp.sc->depth_bound = bound;
     }
-    VRG_CUDA_TRY(cudaStreamSynchronize(s));
     for (auto &cp : cps) {
         Scene *sc = cp.sc;
         sc->dev = cp.dev;

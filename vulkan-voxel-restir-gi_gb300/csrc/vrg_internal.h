@@ -49,6 +49,14 @@ struct DevBuf {
 };
 using DevBufPtr = std::shared_ptr<DevBuf>;
 vrg_status dev_alloc(cudaStream_t s, size_t bytes, DevBufPtr &out);
+// From the context's own pool, on its stream: for what a scene build or a
+// host-array call allocates and frees again.  The default pool gives memory
+// back at every synchronization, which the next allocation maps anew (40 us
+// each, about ten per edited chunk); this pool keeps up to POOL_KEEP bytes
+// until the context goes.
+struct Context;
+constexpr uint64_t POOL_KEEP = 64ull << 20;
+vrg_status dev_alloc(Context *ctx, size_t bytes, DevBufPtr &out);
 
 // ---- SAH builder ------------------------------------------------------
 struct SahTree {
@@ -69,10 +77,12 @@ struct SahOutputs {
     uint32_t *perm;       // local prim order per tree (prim_off-relative)
     uint32_t *leaf_prim;  // per node: local prim index of a leaf, INVALID for internal nodes
 };
-// Builds every tree; trees with n == 0 are skipped.  *levels receives the
-// number of level passes (an upper bound on depth - 2).
-vrg_status sah_build(cudaStream_t s, const std::vector<SahTree> &trees, uint32_t total_prims,
-                     uint32_t total_nodes, const SahInputs &in, const SahOutputs &out, uint32_t *levels);
+// Builds every tree on the context's stream; trees with n == 0 are skipped.
+// *levels receives the number of level passes (an upper bound on depth - 2).
+// With levels_dev (a zeroed device word) the call does not synchronize for it:
+// the bound is then the larger of *levels and that word after the build.
+vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t total_prims,
+                     uint32_t total_nodes, const SahInputs &in, const SahOutputs &out, uint32_t *levels, uint32_t *levels_dev = nullptr);
 
 // ---- chunk extraction ---------------------------------------------------
 struct ChunkSummary {      // per chunk, copied to the host after a flush
@@ -80,7 +90,7 @@ struct ChunkSummary {      // per chunk, copied to the host after a flush
     float light_lo[3], light_hi[3];
     float light_power;
     float geo_lo[3], geo_hi[3];
-    uint32_t pad;
+    uint32_t n_lamps;      // blocks with a luminous exposed face; of a mesh, its light triangles
 };
 
 struct Context;
@@ -127,6 +137,11 @@ struct Context {
     std::mutex mu;                       // guards pending + stream use from upload threads
     std::vector<Object *> pending;
     int num_sms = 0;
+    cudaMemPool_t pool = nullptr;        // dev_alloc(Context *)
+    // page-locked staging of a flush (guarded by mu), kept up to STAGE_KEEP bytes
+    static constexpr size_t STAGE_KEEP = 16u << 20;
+    uint8_t *h_stage = nullptr;
+    size_t h_stage_bytes = 0;
     // references: the handle, and every object, scene, renderer and cache made
     // from it (as the reference's Arc-shared queues and allocators): the
     // context, its stream and its buffers are freed when the last one is
