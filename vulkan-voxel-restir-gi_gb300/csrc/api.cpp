@@ -751,19 +751,32 @@ VRG_API vrg_status vrg_renderer_create_batched(vrg_context *ctx, uint32_t n_view
     const size_t view_tab = ((size_t)n_views * sizeof(ViewDev) + 255) & ~(size_t)255;
     const size_t tab_off = view_tab * r->n_sets;
     DevBufPtr vb;
-    st = dev_alloc(ctx->stream, tab_off + n_groups * 2, vb);
+    r->vtile.assign(n_views + 1, 0);
+    for (uint32_t v = 0; v < n_views; v++)
+        r->vtile[v + 1] = r->vtile[v] + ((widths[v] + 7) / 8) * ((heights[v] + 3) / 4);
+    const size_t n_tgroups = ((size_t)r->vtile[n_views] + (1u << TILE_SHIFT) - 1) >> TILE_SHIFT;
+    const size_t ttab_off = tab_off + ((n_groups * 2 + 255) & ~(size_t)255);
+    st = dev_alloc(ctx->stream, ttab_off + n_tgroups * 2, vb);
     if (st != VRG_OK) return fail(st);
     r->view_buf = vb;
     for (uint32_t k = 0; k < r->n_sets; k++) r->d_views[k] = (ViewDev *)((uint8_t *)vb->ptr + k * view_tab);
     r->d_vtab = (uint16_t *)((uint8_t *)vb->ptr + tab_off);
-    std::vector<uint16_t> vtab(n_groups);
+    r->d_ttab = (uint16_t *)((uint8_t *)vb->ptr + ttab_off);
+    std::vector<uint16_t> ttab(n_tgroups);
     uint32_t v = 0;
+    for (size_t g = 0; g < n_tgroups; g++) {
+        while (v + 1 < n_views && (g << TILE_SHIFT) >= r->vtile[v + 1]) v++;
+        ttab[g] = (uint16_t)v;
+    }
+    std::vector<uint16_t> vtab(n_groups);
+    v = 0;
     for (size_t g = 0; g < n_groups; g++) {
         const uint64_t p = (uint64_t)g << VIEW_SHIFT;
         while (v + 1 < n_views && p >= off[v + 1]) v++;
         vtab[g] = (uint16_t)v;
     }
     if (cudaMemcpyAsync(r->d_vtab, vtab.data(), n_groups * 2, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
+        cudaMemcpyAsync(r->d_ttab, ttab.data(), n_tgroups * 2, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
         cudaHostAlloc((void **)&r->h_views, 2 * (size_t)n_views * sizeof(ViewDev), cudaHostAllocDefault) !=
             cudaSuccess) {
@@ -1012,6 +1025,15 @@ static void apply_tuning(const vrg_renderer *r, FrameArgs &a) {
 // renderers have one)
 static uint32_t frame_set(const vrg_renderer *r) { return r->frame % r->n_sets; }
 
+// 8x4-pixel tiles of a view
+static uint32_t view_tiles(uint32_t w, uint32_t h) { return ((w + 7) / 8) * ((h + 3) / 4); }
+static void set_tiles(ViewDev &d, uint32_t first) {
+    d.tiles_x = (d.W + 7) / 8;
+    d.tile_magic = div_magic(d.tiles_x);
+    d.tile_off = first;
+    d.tile_end = first + view_tiles(d.W, d.H);
+}
+
 static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool want_radiance, FrameArgs &a) {
     if (pr->num_bounces == 0 || pr->spatial_iterations > 64 || pr->nee_type > 2 || pr->mode > 1) {
         set_error("invalid render parameters");
@@ -1096,9 +1118,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     const uint32_t ring = r->frame % slots;
     memset(&a, 0, sizeof(a));
     a.P = (uint32_t)P;
-    a.tiles_x = (r->W + 7) / 8;
-    a.tile_magic = div_magic(a.tiles_x);
-    a.n0 = r->n_views ? (uint32_t)P : a.tiles_x * ((r->H + 3) / 4) * 32u;
+    a.n0 = (r->n_views ? r->vtile[r->n_views] : view_tiles(r->W, r->H)) * 32u;
     a.nb = nb_total;
     a.nb_render = pr->num_bounces;
     a.cache = cache ? 1u : 0u;
@@ -1496,6 +1516,7 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
     a.v0.pix_end = (uint32_t)P;
     a.v0.frame = r->frame;
     a.v0.w_magic = div_magic(r->W);
+    set_tiles(a.v0, 0);
     a.v0.ray_x = r->fs[frame_set(r)].ray_tab;
     a.v0.ray_y = a.v0.ray_x + r->W;
     a.v0.temporal_seed = pr->temporal_seed;
@@ -1608,6 +1629,7 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
         d.pix_end = (uint32_t)(r->voff[v] + (uint64_t)r->vw[v] * r->vh[v]);
         d.frame = r->frame;
         d.w_magic = div_magic(d.W);
+        set_tiles(d, r->vtile[v]);
         d.ray_x = r->fs[frame_set(r)].ray_tab + r->vtoff[v];
         d.ray_y = d.ray_x + d.W;
         d.temporal_seed = w.temporal_seed;
@@ -1626,6 +1648,7 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
     r->stage ^= 1u;
     a.views = r->d_views[set];
     a.vtab = r->d_vtab;
+    a.ttab = r->d_ttab;
     a.n_views = n_views;
     if (graph) {
         // the FrameArgs bytes name the recording: buffers, ring slot and parameters

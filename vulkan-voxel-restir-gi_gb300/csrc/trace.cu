@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
             if (!has) {
                 const uint32_t idx = base + (uint32_t)__popc(need & lanemask_lt());
                 uint32_t x = 0, y = 0;
-                if (idx < range.end && (b == 0 ? bounce0_pixel<BATCH>(a, idx, p, x, y) : (p = qin[idx], true))) {
+                if (idx < range.end &&
+                    (b == 0 ? bounce0_pixel(view_of_tile<BATCH>(a, idx >> 5), idx, p, x, y) : (p = qin[idx], true))) {
                     has = true;
                     traced++;
                     const ViewDev &V = view_of<BATCH>(a, p);
@@ -861,7 +862,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 if (active) p = route[r];
             } else {
                 const uint32_t i = base + lane;
-                active = i < n_in && (b == 0 ? bounce0_pixel<BATCH>(a, i, p, px, py) : (p = qin[i], true));
+                active = i < n_in && (b == 0 ? bounce0_pixel(view_of_tile<BATCH>(a, i >> 5), i, p, px, py) : (p = qin[i], true));
             }
             bool cont = false, anyj = false, qhit = false, want_train = false;
             const bool at_query = a.cache && b + 1 == a.nb_render;

@@ -44,6 +44,8 @@ struct ViewDev {
     // the primary rays' direction terms of the frame's camera per column and
     // per row (k_frame_begin): d = normalize((ray_x[x] + ray_y[y]) + front)
     float4 *ray_x, *ray_y;
+    // its 8x4-pixel tiles: [tile_off, tile_end) of the frame's tiles, tiles_x per row
+    uint32_t tile_off, tile_end, tiles_x, tile_magic;  // tile_magic: div_magic(tiles_x)
 };
 
 // n / d and n % d for any 32-bit n by one high product and a correction, with
@@ -60,6 +62,7 @@ __host__ __device__ __forceinline__ void div_mod(uint32_t n, uint32_t d, uint32_
     }
 }
 
+constexpr int TILE_SHIFT = 3;  // ttab entry per 8 tiles: the view of the group's first tile
 constexpr int VIEW_SHIFT = 8;  // vtab entry per 256 pixels: the view of the group's first pixel
 
 struct FrameArgs {
@@ -70,8 +73,8 @@ struct FrameArgs {
     uint32_t mesh;                // a scene of the frame holds mesh triangles (the bounce kernels
                                   // built with mesh support run; voxel-only frames run without it)
     uint32_t P;                   // pixels of the frame (all views)
-    uint32_t n0, tiles_x;         // bounce-0 slots and 8x4 tiles per row (bounce0_pixel)
-    uint32_t tile_magic;          // div_magic(tiles_x)
+    uint32_t n0;                  // bounce-0 slots: 32 per 8x4-pixel tile (bounce0_pixel)
+    const uint16_t *ttab;         // batched frame: view of tile group t >> TILE_SHIFT
     uint32_t nb, nee_type;
     uint32_t mode, spatial_iters;
     float spatial_radius;
@@ -142,27 +145,31 @@ __device__ __forceinline__ const ViewDev &view_of(const FrameArgs &a, uint32_t p
     }
 }
 
-// Bounce 0 of a single view takes its pixels in 8x4 tiles, so that a warp's
-// primary rays, and through the queue order the secondary rays they spawn,
-// start close together.  Slot i (< n0) is pixel p, or no pixel in the part of
-// an edge tile outside the view.  A batched frame keeps the pixel order.
+// The view that owns tile t of the frame.
 template <bool BATCH>
-__device__ __forceinline__ bool bounce0_pixel(const FrameArgs &a, uint32_t i, uint32_t &p, uint32_t &x, uint32_t &y) {
+__device__ __forceinline__ const ViewDev &view_of_tile(const FrameArgs &a, uint32_t t) {
     if constexpr (BATCH) {
-        p = i;
-        if (i >= a.P) return false;
-        const ViewDev &V = view_of<BATCH>(a, p);
-        div_mod(p - V.pix_off, V.W, V.w_magic, y, x);
-        return true;
+        uint32_t v = a.ttab[t >> TILE_SHIFT];
+        while (t >= a.views[v].tile_end) v++;
+        return a.views[v];
     } else {
-        const uint32_t t = i >> 5, k = i & 31u;
-        uint32_t tx, ty;
-        div_mod(t, a.tiles_x, a.tile_magic, ty, tx);
-        x = tx * 8u + (k & 7u);
-        y = ty * 4u + (k >> 3);
-        p = y * a.v0.W + x;
-        return x < a.v0.W && y < a.v0.H;
+        (void)t;
+        return a.v0;
     }
+}
+
+// Bounce 0 takes a view's pixels in 8x4 tiles, so that a warp's primary rays,
+// and through the queue order the secondary rays they spawn, start close
+// together.  Slot i (< n0) of view V is pixel p = (x, y), or no pixel in the
+// part of an edge tile outside the view.
+__device__ __forceinline__ bool bounce0_pixel(const ViewDev &V, uint32_t i, uint32_t &p, uint32_t &x, uint32_t &y) {
+    const uint32_t t = (i >> 5) - V.tile_off, k = i & 31u;
+    uint32_t tx, ty;
+    div_mod(t, V.tiles_x, V.tile_magic, ty, tx);
+    x = tx * 8u + (k & 7u);
+    y = ty * 4u + (k >> 3);
+    p = V.pix_off + y * V.W + x;
+    return x < V.W && y < V.H;
 }
 
 }  // namespace vrg

@@ -240,7 +240,8 @@ struct Renderer {
     uint32_t tab_max = 0;                 // the most of one view
     DevBufPtr view_buf;                   // a ViewDev[n_views] table per array set + vtab
     ViewDev *d_views[3] = {};
-    uint16_t *d_vtab = nullptr;
+    uint16_t *d_vtab = nullptr, *d_ttab = nullptr;
+    std::vector<uint32_t> vtile;          // first 8x4-pixel tile of each view, then their number
     ViewDev *h_views = nullptr;           // pinned staging, 2 x n_views
     cudaEvent_t ev_stage[2] = {};         // after the copy out of each staging half
     uint32_t stage = 0;
