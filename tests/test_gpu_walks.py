@@ -1,7 +1,8 @@
 """The persistent walks' work distribution and the light-hit collection at the
 sizes where they can go wrong, bit for bit (0 ulp) against the oracle and
 against the same frame without capture:
-- queues shorter than a warp, ending inside a warp's static share of 32, and
+- queues shorter than a warp, a few entries short of one per resident warp and
+  exactly one per warp, ending inside a warp's static share of 32, and
   long enough that every warp takes further chunks (a grid of one CTA per SM);
 - worlds with so many lamps that a ray sets aside more of them than its list
   holds, and crosses several (the sums of several hits)."""
@@ -17,6 +18,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("W,H,grid,refill,emissive", [
     (1, 1, 0, 0, 0.01),
     (33, 1, 0, 32, 0.05),
+    (81, 60, 0, 8, 0.05),
+    (76, 64, 0, 16, 0.05),
     (96, 61, 0, 1, 0.3),
     (301, 173, 1, 8, 0.01),
     (301, 173, 1, 32, 0.3),

@@ -389,12 +389,23 @@ struct WarpRange {
 };
 constexpr uint32_t CHUNK_MAX = 256;
 
+// Entries of a warp's static share: 32, or one where the queue holds fewer
+// entries than there are resident warps: a warp's divergent lanes follow one
+// another, and such a queue's kernel lasts as long as its slowest warp (64x64
+// pixels: closest hits 22 -> 18 us, the frame 132 -> 128).  Longer queues keep
+// whole warps: spread at 8 entries per warp and more, a 957x541 frame in flight
+// took 288 us, not 270.
+__device__ __forceinline__ uint32_t first_share(uint32_t n_in, uint32_t all) {
+    return n_in >= all ? 32u : 1u;
+}
+
 __device__ __forceinline__ WarpRange range_first(uint32_t n_in) {
     const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), all = gridDim.x * (blockDim.x >> 5);
+    const uint32_t share = first_share(n_in, all);
     WarpRange r;
-    r.cur = min(32u * w, n_in);
-    r.end = min(32u * w + 32u, n_in);
-    r.last = 32u * all;
+    r.cur = min(share * w, n_in);
+    r.end = min(share * w + share, n_in);
+    r.last = share * all;
     r.more = r.last < n_in;
     return r;
 }
@@ -405,7 +416,7 @@ __device__ __forceinline__ void range_next(WarpRange &r, uint32_t n_in, uint32_t
     const uint32_t size = min(((n_in - r.last) / (128u * all) + 1u) * 32u, CHUNK_MAX);
     uint32_t base = 0;
     if ((threadIdx.x & 31u) == 0) base = atomicAdd(fetch, size);
-    base = 32u * all + __shfl_sync(0xffffffffu, base, 0);
+    base = first_share(n_in, all) * all + __shfl_sync(0xffffffffu, base, 0);
     r.cur = min(base, n_in);
     r.last = r.end = min(base + size, n_in);
     r.more = r.end < n_in;
@@ -819,7 +830,7 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                          : n_in >= 2u * SHADE_BATCH * 32u * warps ? SHADE_BATCH
                          : n_in >= 2u * 64u * warps               ? 2u
                                                                   : 1u;
-    const uint32_t span = 32u * per;
+    const uint32_t span = split ? 32u * per : first_share(n_in, warps);
     uint32_t *route = s_route[threadIdx.x >> 5];
     for (uint32_t base = wid * span; base < n_in; base += warps * span) {
         uint32_t n_route = 0;
@@ -862,7 +873,8 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 if (active) p = route[r];
             } else {
                 const uint32_t i = base + lane;
-                active = i < n_in && (b == 0 ? bounce0_pixel(view_of_tile<BATCH>(a, i >> 5), i, p, px, py) : (p = qin[i], true));
+                active = (uint32_t)lane < span && i < n_in &&
+                         (b == 0 ? bounce0_pixel(view_of_tile<BATCH>(a, i >> 5), i, p, px, py) : (p = qin[i], true));
             }
             bool cont = false, anyj = false, qhit = false, want_train = false;
             const bool at_query = a.cache && b + 1 == a.nb_render;
