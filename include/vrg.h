@@ -167,7 +167,8 @@ typedef struct vrg_frame_output {
 } vrg_frame_output;
 
 typedef struct vrg_frame_stats {
-    float ms_total;            /* device time of the whole frame (CUDA events) */
+    float ms_total;            /* device time of the whole frame (CUDA events); the stages'
+                                  times below are of the device's global timer */
     float ms_bounce[8];        /* per bounce: closest hit + shading (the light-pdf walk of
                                   bounce b runs on its own stream beside bounce b+1) */
     float ms_resolve;          /* outgoing radiance + temporal (+ cache inference/training) */
@@ -176,8 +177,8 @@ typedef struct vrg_frame_stats {
     uint64_t rays_any;         /* light any-hit queries issued */
     uint32_t error_flags;      /* device-side error word (stack overflow etc.) */
     uint32_t reserved;
-    float ms_trace[8];         /* per bounce: k_trace alone */
-    float ms_shade[8];         /* per bounce: k_shade alone */
+    float ms_trace[8];         /* per bounce: k_trace, from the end of the stage before */
+    float ms_shade[8];         /* per bounce: k_shade, from the end of k_trace */
     float ms_anyhit[8];        /* per bounce: the light-pdf walk (k_anyhit, k_hit_eval,
                                   k_hit_sum) on its stream */
     uint64_t nodes_visited;    /* closest-hit traversal: 4-wide inner nodes fetched (128 B each) */

@@ -14,7 +14,7 @@
 namespace vrg {
 
 vrg_status upload_frames(cudaStream_t s);
-vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, cudaEvent_t ev_trace, uint32_t max_rays);
+vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
 vrg_status launch_frame_begin(cudaStream_t s, const FrameArgs &a, uint32_t max_entries);
 vrg_status launch_light_pdf(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
 vrg_status launch_resolve(cudaStream_t s, const FrameArgs &a);
@@ -672,16 +672,13 @@ static vrg_status renderer_events(vrg_renderer *r) {
         VRG_CUDA_TRY(cudaEventCreateWithFlags(&r->ev_done[k], cudaEventDisableTiming));
         VRG_CUDA_TRY(cudaEventRecord(r->ev_done[k], r->ctx->stream));  // after the buffers' clear
     }
-    for (auto &row : r->ev_lp)
-        for (auto &e : row) VRG_CUDA_TRY(cudaEventCreate(&e));
     VRG_CUDA_TRY(cudaEventCreateWithFlags(&r->ev_fork, cudaEventDisableTiming));
     VRG_CUDA_TRY(cudaEventCreateWithFlags(&r->ev_join, cudaEventDisableTiming));
     VRG_CUDA_TRY(cudaEventCreateWithFlags(&r->ev_start, cudaEventDisableTiming));
     VRG_CUDA_TRY(cudaEventCreateWithFlags(&r->ev_updated, cudaEventDisableTiming));
     for (auto &e : r->ev) VRG_CUDA_TRY(cudaEventCreate(&e));
-    for (auto &row : r->ev_k)
-        for (auto &e : row) VRG_CUDA_TRY(cudaEventCreate(&e));
     for (auto &e : r->ev_fence) VRG_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    VRG_CUDA_TRY(cudaMallocHost(&r->h_counters, CNT_WORDS * 4));
     // the kernels' occupancy grids, queried once here (never inside a stream capture)
     int occ[3], sms = 1;
     bounce_occupancy(false, occ, &sms);
@@ -808,9 +805,6 @@ VRG_API vrg_status vrg_renderer_destroy(vrg_renderer *r) {
     drop_graphs(r);
     for (auto &e : r->ev)
         if (e) cudaEventDestroy(e);
-    for (auto &row : r->ev_k)
-        for (auto &e : row)
-            if (e) cudaEventDestroy(e);
     for (auto &e : r->ev_stage)
         if (e) cudaEventDestroy(e);
     for (int k = 0; k < Renderer::SETS; k++) {
@@ -826,9 +820,6 @@ VRG_API vrg_status vrg_renderer_destroy(vrg_renderer *r) {
         if (r->ev_bounced[k]) cudaEventDestroy(r->ev_bounced[k]);
         if (r->ev_done[k]) cudaEventDestroy(r->ev_done[k]);
     }
-    for (auto &row : r->ev_lp)
-        for (auto &e : row)
-            if (e) cudaEventDestroy(e);
     for (auto &e : r->ev_fence)
         if (e) cudaEventDestroy(e);
     if (r->ev_fork) cudaEventDestroy(r->ev_fork);
@@ -840,7 +831,7 @@ VRG_API vrg_status vrg_renderer_destroy(vrg_renderer *r) {
             cudaStreamSynchronize(q);
             cudaStreamDestroy(q);
         }
-    if (r->h_pinned) cudaFreeHost(r->h_pinned);
+    if (r->h_counters) cudaFreeHost(r->h_counters);
     if (r->h_views) cudaFreeHost(r->h_views);
     r->res_buf.reset();
     Context *c = r->ctx;
@@ -1198,10 +1189,9 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     return VRG_OK;
 }
 
-// The frame's launch sequence on the context stream.  timed: CUDA events
-// around every stage (r->ev: frame start, after each bounce, after resolve,
-// after spatial; r->ev_k: after k_trace / k_shade of each bounce); a graph
-// recording passes false.
+// The frame's launch sequence on the context stream, with an event before and
+// after it when it is timed (a.timed: its kernels write the stages' own times;
+// not in a graph recording).
 //
 // A cache frame forks once the training paths' query vertices are shaded,
 // while that bounce's light-pdf walk still runs: the training paths' extra
@@ -1235,13 +1225,12 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
 // so a scene's device data is final before any frame reads it; a resize
 // clears the arrays on the library stream and re-records ev_done.
 // Other frames run their bounces on the library stream itself.
-static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, bool pipelined = false,
-                               bool in_graph = false) {
+static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool pipelined, bool in_graph = false) {
     cudaStream_t s = r->ctx->stream;
     const uint32_t k = frame_set(r);
     const bool fork = a.cache && !a.capture;
     const uint32_t nb_main = fork ? a.nb_render : a.nb;
-    const bool own = pipelined && !a.capture && !timed && !in_graph;
+    const bool own = pipelined && !a.capture && !in_graph;
     cudaStream_t bs = own ? r->bs[k] : s;  // stream of the bounces
     cudaStream_t lp = r->lps[k];
     if (own) VRG_CUDA_TRY(cudaStreamWaitEvent(bs, r->ev_done[k], 0));
@@ -1264,8 +1253,8 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
         VRG_CUDA_TRY(cudaEventRecord(r->ev_updated, r->aux));
         updated = true;
     }
+    if (a.timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[0], s));
     VRG_TRY(launch_frame_begin(bs, a, r->tab_max));
-    if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[0], s));
     // Bounce b's light-pdf walk runs on the light-pdf stream beside bounce
     // b + 1's closest hit and shading.  Ordering: the walk of b waits for the
     // shading of b; the shading of b + 2 (which refills the job buffers of
@@ -1274,9 +1263,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
     auto walk = [&](uint32_t b) -> vrg_status {
         VRG_CUDA_TRY(cudaEventRecord(r->ev_shaded[k][b], bs));
         VRG_CUDA_TRY(cudaStreamWaitEvent(lp, r->ev_shaded[k][b], 0));
-        if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev_lp[0][b], lp));
         VRG_TRY(launch_light_pdf(lp, a, b, 0));
-        if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev_lp[1][b], lp));
         VRG_CUDA_TRY(cudaEventRecord(r->ev_lpdone[k][b], lp));
         last_lp = (int)b;
         return VRG_OK;
@@ -1316,8 +1303,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
         for (uint32_t b = nb_main; b < a.nb; b++) {
             if (b >= nb_main + 2 && (int)b - 2 <= last_tw)
                 VRG_CUDA_TRY(cudaStreamWaitEvent(st, r->ev_lpdone[k][b - 2], 0));
-            VRG_TRY(launch_trace_shade(st, at, b, timed ? r->ev_k[0][b] : nullptr, a.train_cap));
-            if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev_k[1][b], st));
+            VRG_TRY(launch_trace_shade(st, at, b, a.train_cap));
             if (b + 1 < a.nb) {
                 VRG_CUDA_TRY(cudaEventRecord(r->ev_shaded[k][b], st));
                 VRG_CUDA_TRY(cudaStreamWaitEvent(r->aux_lp, r->ev_shaded[k][b], 0));
@@ -1325,7 +1311,6 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
                 VRG_CUDA_TRY(cudaEventRecord(r->ev_lpdone[k][b], r->aux_lp));
                 last_tw = (int)b;
             }
-            if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[b + 1], st));
         }
         if (last_tw >= 0) VRG_CUDA_TRY(cudaStreamWaitEvent(st, r->ev_lpdone[k][last_tw], 0));
         // the targets' recurrence starts at the query vertex, whose record the
@@ -1351,15 +1336,11 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
             aT.qsel = 1;
             aT.queue[b & 1] = Q.t_queue[0];  // its continuing rays: the first training bounce's queue
             aT.queue[(b + 1) & 1] = Q.t_queue[1];
-            VRG_TRY(launch_trace_shade(bs, aT, b, nullptr, a.P));
+            VRG_TRY(launch_trace_shade(bs, aT, b, a.P));
             if (b + 1 < a.nb) VRG_TRY(walk(b));
             VRG_TRY(branch(bs, true));
         }
-        VRG_TRY(launch_trace_shade(bs, a, b, timed ? r->ev_k[0][b] : nullptr, 0));
-        if (timed) {  // (timed frames run their bounces on the library stream)
-            VRG_CUDA_TRY(cudaEventRecord(r->ev_k[1][b], s));
-            VRG_CUDA_TRY(cudaEventRecord(r->ev[b + 1], s));
-        }
+        VRG_TRY(launch_trace_shade(bs, a, b, 0));
         if (b + 1 < a.nb && !(early && b + 1 == nb_main)) VRG_TRY(walk(b));
     }
     // a cache frame's training branch and cache queries start before the last
@@ -1390,7 +1371,6 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
         VRG_TRY(nrc_train(r->cache, s, a.train_cap, a.counters + CNT_TRAIN, a.train_list, a.q_pos, a.q_dir,
                           nullptr, a.target, true, a.counters + CNT_ERROR));
     }
-    if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[a.nb + 1], s));
     // the TMA-staged spatial pass when the tuning asks for it and the ring
     // slot has its tensor map
     const CUtensorMap *res_map = nullptr;
@@ -1403,50 +1383,48 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool timed, 
     // the set is free for the frame n_sets ahead (recorded after the graph
     // launch when the frame is recorded in a graph)
     if (!in_graph) VRG_CUDA_TRY(cudaEventRecord(r->ev_done[k], s));
-    if (timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[a.nb + 2], s));
+    if (a.timed) VRG_CUDA_TRY(cudaEventRecord(r->ev[1], s));
     return VRG_OK;
 }
 
-// Stats of the frame just launched (synchronizes).  per_kernel: the frame was
-// launched with timed == true; otherwise ev[0]/ev[1] bracket a graph launch.
+// Stats of the frame just launched (synchronizes); ev[0]/ev[1] bracket it.
+// per_kernel: the frame was not a graph launch; its stage times are reported.
 static vrg_status frame_stats(vrg_renderer *r, const FrameArgs &a, bool per_kernel, vrg_frame_stats *stats) {
+    const uint32_t *cnt = r->h_counters;
+    VRG_CUDA_TRY(cudaMemcpyAsync(r->h_counters, a.counters, CNT_WORDS * 4, cudaMemcpyDeviceToHost, r->ctx->stream));
     VRG_CUDA_TRY(cudaStreamSynchronize(r->ctx->stream));
     memset(stats, 0, sizeof(*stats));
     float ms = 0.0f;
+    cudaEventElapsedTime(&ms, r->ev[0], r->ev[1]);
+    stats->ms_total = ms;
     if (per_kernel) {
-        cudaEventElapsedTime(&ms, r->ev[0], r->ev[a.nb + 2]);
-        stats->ms_total = ms;
-        // main-stream bounces: closest hit + shading; their light-pdf walks
-        // run beside the next bounce and are timed on their own stream
+        // a stage's time in ms from the frame's start (a stage that did not run: `before`)
+        uint64_t t0;
+        memcpy(&t0, cnt + CNT_STAMP + 2 * ST_BEGIN, 8);
+        auto at = [&](int stage, double before) {
+            uint64_t t;
+            memcpy(&t, cnt + CNT_STAMP + 2 * stage, 8);
+            return t > t0 ? std::max(before, (double)(t - t0) * 1e-6) : before;
+        };
+        // main-stream bounces: closest hit + shading, each from the end of the
+        // stage before it; their light-pdf walks run beside the next bounce
         const uint32_t nb_main = (a.cache && !a.capture) ? a.nb_render : a.nb;
-        for (uint32_t b = 0; b < a.nb && b < 8; b++) {
-            cudaEventElapsedTime(&ms, r->ev[b], r->ev[b + 1]);
-            stats->ms_bounce[b] = ms;
-            cudaEventElapsedTime(&ms, r->ev[b], r->ev_k[0][b]);
-            stats->ms_trace[b] = ms;
-            cudaEventElapsedTime(&ms, r->ev_k[0][b], r->ev_k[1][b]);
-            stats->ms_shade[b] = ms;
-            if (b < nb_main) {
-                if (b + 1 < a.nb) {
-                    cudaEventElapsedTime(&ms, r->ev_lp[0][b], r->ev_lp[1][b]);
-                    stats->ms_anyhit[b] = ms;
-                }
-            } else {
-                cudaEventElapsedTime(&ms, r->ev_k[1][b], r->ev[b + 1]);
-                stats->ms_anyhit[b] = ms;
-            }
+        double end = 0.0, main_end = 0.0;
+        for (uint32_t b = 0; b < a.nb; b++) {
+            const double traced = at(ST_TRACED + b, end), shaded = at(ST_SHADED + b, traced);
+            stats->ms_bounce[b] = (float)(shaded - end);
+            stats->ms_trace[b] = (float)(traced - end);
+            stats->ms_shade[b] = (float)(shaded - traced);
+            const double walk = at(ST_WALK + b, 0.0);
+            stats->ms_anyhit[b] = (float)(at(ST_WALKED + b, walk) - walk);
+            end = shaded;
+            if (b + 1 == nb_main) main_end = end;
         }
         // a forked cache frame's resolve stage starts at the fork (it runs beside the training branch)
-        cudaEventElapsedTime(&ms, r->ev[(a.cache && !a.capture) ? a.nb_render : a.nb], r->ev[a.nb + 1]);
-        stats->ms_resolve = ms;
-        cudaEventElapsedTime(&ms, r->ev[a.nb + 1], r->ev[a.nb + 2]);
-        stats->ms_spatial = ms;
-    } else {
-        cudaEventElapsedTime(&ms, r->ev[0], r->ev[1]);
-        stats->ms_total = ms;
+        const double spatial = at(ST_SPATIAL, main_end);
+        stats->ms_resolve = (float)(spatial - main_end);
+        stats->ms_spatial = std::max(0.0f, ms - (float)spatial);
     }
-    uint32_t cnt[CNT_WORDS];
-    VRG_CUDA_TRY(cudaMemcpy(cnt, a.counters, sizeof(cnt), cudaMemcpyDeviceToHost));
     uint64_t rays, any, nn, nlv;
     memcpy(&rays, cnt + CNT_RAYS, 8);
     memcpy(&any, cnt + CNT_ANY, 8);
@@ -1531,7 +1509,8 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
         }
     }
     // without stats the frame is not timed and may start beside the previous one
-    VRG_TRY(frame_launch(r, a, stats != nullptr, stats == nullptr));
+    a.timed = stats ? 1u : 0u;
+    VRG_TRY(frame_launch(r, a, stats == nullptr));
     if (out && out->host) {
         const size_t Po = (size_t)r->out_w * r->out_h;
         if (out->bgra8 && a.pack)
@@ -1660,7 +1639,7 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
             if (r->graphs.size() >= 8) drop_graphs(r);
             cudaGraph_t g = nullptr;
             VRG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            vrg_status st = frame_launch(r, a, false, false, true);
+            vrg_status st = frame_launch(r, a, false, true);
             cudaError_t ce = cudaStreamEndCapture(s, &g);
             if (st != VRG_OK) {
                 if (g) cudaGraphDestroy(g);
@@ -1680,7 +1659,8 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
         VRG_CUDA_TRY(cudaEventRecord(r->ev_done[set], s));
     } else {
         // without stats the frame is not timed and may run beside the previous one
-        VRG_TRY(frame_launch(r, a, stats != nullptr, stats == nullptr));
+        a.timed = stats ? 1u : 0u;
+        VRG_TRY(frame_launch(r, a, stats == nullptr));
     }
     bool host_out = false;
     if (outs) {

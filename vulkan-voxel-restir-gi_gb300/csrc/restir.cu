@@ -288,6 +288,7 @@ template <bool CAPTURE, bool BATCH>
 __global__ void __launch_bounds__(256, 5) k_spatial(const __grid_constant__ FrameArgs a) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.P) return;
+    stamp_start(a, ST_SPATIAL);
     spatial_pixel<CAPTURE, BATCH>(a, p, ResGlobal{a.res, a.P});
 }
 
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(256, 5) k_spatial_tma(const __grid_constant__ 
     const uint32_t W = a.v0.W, H = a.v0.H;
     const uint32_t x0 = blockIdx.x * ST_W, y0 = blockIdx.y * ST_H;
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(&bar), d = (uint32_t)__cvta_generic_to_shared(tile);
+    if (blockIdx.y == 0) stamp_start(a, ST_SPATIAL);
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(b) : "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");

@@ -273,7 +273,8 @@ __device__ __forceinline__ void raygen(const ViewDev &V, uint32_t x, uint32_t y,
 template <bool BATCH>
 __global__ void __launch_bounds__(128) k_frame_begin(const __grid_constant__ FrameArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.y == 0 && i < CNT_WORDS) a.counters[i] = 0;
+    if (blockIdx.y == 0 && i < CNT_WORDS && i / 2 != CNT_STAMP / 2 + ST_BEGIN) a.counters[i] = 0;
+    if (blockIdx.y == 0) stamp_start(a, ST_BEGIN);
     const ViewDev &V = BATCH ? a.views[blockIdx.y] : a.v0;
     if (i < V.W) {
         const f3 c = ray_col(V, i);
@@ -424,22 +425,23 @@ __device__ __forceinline__ void range_next(WarpRange &r, uint32_t n_in, uint32_t
 
 // Adds each warp's totals to N u64 counters, one atomic per CTA and counter:
 // the CTA's last warp to finish publishes the sums (s_sum: N + 1 words of
-// shared memory, zeroed before the walk).
+// shared memory, zeroed before the walk); true for the lane that did.
 template <int N>
-__device__ __forceinline__ void publish_totals(uint32_t *s_sum, uint32_t *counters, const int (&at)[N],
+__device__ __forceinline__ bool publish_totals(uint32_t *s_sum, uint32_t *counters, const int (&at)[N],
                                                const uint32_t (&v)[N]) {
-    if ((threadIdx.x & 31u) != 0) return;
+    if ((threadIdx.x & 31u) != 0) return false;
 #pragma unroll
     for (int k = 0; k < N; k++)
         if (v[k]) atomicAdd(s_sum + k, v[k]);
     __threadfence_block();
-    if (atomicAdd(s_sum + N, 1u) != (blockDim.x >> 5) - 1u) return;
+    if (atomicAdd(s_sum + N, 1u) != (blockDim.x >> 5) - 1u) return false;
     __threadfence_block();
 #pragma unroll
     for (int k = 0; k < N; k++) {
         const uint32_t t = atomicAdd(s_sum + k, 0u);
         if (t) atomicAdd(reinterpret_cast<unsigned long long *>(counters + at[k]), (unsigned long long)t);
     }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -609,7 +611,8 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
         n_nodes += __shfl_xor_sync(FULL, n_nodes, off);
         n_leaves += __shfl_xor_sync(FULL, n_leaves, off);
     }
-    publish_totals<3>(s_sum, a.counters, {CNT_RAYS, CNT_NODES, CNT_LEAVES}, {traced, n_nodes, n_leaves});
+    if (publish_totals<3>(s_sum, a.counters, {CNT_RAYS, CNT_NODES, CNT_LEAVES}, {traced, n_nodes, n_leaves}))
+        stamp_end(a, ST_TRACED + b);
 }
 
 // Shading of one path vertex (raytrace.rs:405-577): the hit's material
@@ -1045,6 +1048,9 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 a.ajob[b & 1][2 * (size_t)j + 1] = make_float4(new_d.x, new_d.y, new_d.z, pdf);
             }
         }
+        // (the end of the CTA's first warp; behind the loop the same stamp made
+        // every shading 1% slower, written or not)
+        if (threadIdx.x == 0 && n_in - base <= warps * span) stamp_end(a, ST_SHADED + b);
         __syncwarp();
     }
 }
@@ -1123,6 +1129,7 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
     int px = 0, py = 2, pz = 4;  // near-plane float4 per axis, picked by the ray's direction signs
     int stack[TRAV_STACK], lamps[LAMP_LIST];
     HitList hits;
+    stamp_start(a, ST_WALK + b);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n_in)
         atomicAdd(reinterpret_cast<unsigned long long *>(a.counters + CNT_ANY), (unsigned long long)n_in);
     if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
@@ -1314,6 +1321,7 @@ __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameAr
         finish_job(a, b, p, a.ajob[b & 1][2 * (size_t)idx + 1].w, nee);
         if (CAPTURE) a.c_nee[(size_t)b * a.P + p] = nee;
     }
+    if (threadIdx.x == 0) stamp_end(a, ST_WALKED + b);
 }
 
 }  // namespace
@@ -1446,14 +1454,12 @@ vrg_status launch_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t
 }
 
 // closest hit and shading of bounce b
-vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, cudaEvent_t ev_trace,
-                              uint32_t max_rays) {
+vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays) {
     if (a.views && a.capture) {
         set_error("capture is not available for batched frames");
         return VRG_ERR_UNSUPPORTED;
     }
     VRG_TRY(launch_trace(s, a, b, max_rays));
-    if (ev_trace) VRG_CUDA_TRY(cudaEventRecord(ev_trace, s));
     return launch_shade(s, a, b, max_rays);
 }
 

@@ -295,9 +295,7 @@ struct Renderer {
     float *c_origin = nullptr, *c_dir = nullptr, *c_normal = nullptr, *c_emis = nullptr, *c_refl = nullptr;
     float *c_mis = nullptr, *c_pdf = nullptr, *c_nee = nullptr, *c_L = nullptr, *c_q = nullptr;
     uint32_t *c_hit = nullptr;
-    // host staging
-    uint8_t *h_pinned = nullptr;
-    size_t h_pinned_bytes = 0;
+    uint32_t *h_counters = nullptr;       // pinned: a frame's counters and stage times, copied out behind it
     cudaStream_t aux = nullptr;           // second stream: a cache frame's training paths and step
     cudaStream_t aux_lp = nullptr;        // the training bounces' light-pdf walks, beside the next bounce
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_start = nullptr, ev_updated = nullptr;
@@ -312,9 +310,7 @@ struct Renderer {
     // copies out; vrg_renderer_wait_frame waits on them
     static constexpr uint32_t FENCES = 8;
     cudaEvent_t ev_fence[FENCES] = {};
-    cudaEvent_t ev_lp[2][8] = {};         // timing: light-pdf passes of bounce b begin / end
-    cudaEvent_t ev[16] = {};
-    cudaEvent_t ev_k[2][8] = {};          // after k_trace / after k_shade, per bounce
+    cudaEvent_t ev[2] = {};               // timing: a frame's begin / end
     Nrc *cache = nullptr;                 // attached radiance cache (not owned)
     DevBufPtr cache_buf;                  // per-pixel cache queries / predictions / targets
     uint32_t cache_cap = 0;               // training paths cache_buf was sized for
