@@ -13,7 +13,7 @@
 
 namespace vrg {
 
-vrg_status upload_frames(cudaStream_t s);
+vrg_status upload_frames(cudaStream_t s, const float4 **table);
 vrg_status launch_trace_shade(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
 vrg_status launch_frame_begin(cudaStream_t s, const FrameArgs &a, uint32_t max_entries);
 vrg_status launch_light_pdf(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
@@ -149,7 +149,7 @@ VRG_API vrg_status vrg_context_create(const vrg_context_desc *desc, vrg_context 
             cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
         }
     }
-    vrg_status st = upload_frames(c->stream);
+    vrg_status st = upload_frames(c->stream, &c->faces);
     if (st != VRG_OK) {
         if (c->pool) cudaMemPoolDestroy(c->pool);
         cudaStreamDestroy(c->stream);
@@ -563,7 +563,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
     size_t o = 0;
     // the arrays of a frame's bounces, one set per frame in flight
     struct SetOff {
-        size_t ro, rd, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, nv, xs, ns, rt;
+        size_t ro, rd, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, xs, rt;
     } so[Renderer::SETS];
     const int sets = (int)r->n_sets;
     for (int k = 0; k < sets; k++) {
@@ -584,9 +584,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
         q.nl = o; o += al(P);
         q.rec = o; o += al(P * 32 * nb);
         q.xv = o; o += al(P * 16);
-        q.nv = o; o += al(P * 16);
         q.xs = o; o += al(P * 16);
-        q.ns = o; o += al(P * 16);
         q.rt = o; o += al(r->tab_entries * 16);
     }
     size_t o_pl = o; o += al(P * 16);
@@ -617,9 +615,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
         F.nlive = B + q.nl;
         F.rec = (float4 *)(B + q.rec);
         F.xv = (float4 *)(B + q.xv);
-        F.nv = (float4 *)(B + q.nv);
         F.xs = (float4 *)(B + q.xs);
-        F.ns = (float4 *)(B + q.ns);
         F.ray_tab = (float4 *)(B + q.rt);
     }
     r->plain = (float4 *)(B + o_pl);
@@ -1157,9 +1153,8 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.nlive = F.nlive;
     a.rec = F.rec;
     a.xv = F.xv;
-    a.nv = F.nv;
     a.xs = F.xs;
-    a.ns = F.ns;
+    a.faces = r->ctx->faces;
     a.plain = r->plain;
     a.res = r->res + (size_t)ring * 5 * P;
     a.spatial = r->spatial;

@@ -981,12 +981,9 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 const float w = pdf / q;
                 a.rec[rb + p] = make_float4(E.x, E.y, E.z, w);
                 a.rec[rb + P + p] = make_float4(R.x, R.y, R.z, q);
-                if (b == 0) {
-                    a.xv[p] = make_float4(new_o.x, new_o.y, new_o.z, 0.0f);
-                    a.nv[p] = make_float4(n.x, n.y, n.z, 0.0f);
-                } else if (b == 1) {
-                    a.xs[p] = make_float4(new_o.x, new_o.y, new_o.z, 0.0f);
-                    a.ns[p] = make_float4(n.x, n.y, n.z, 0.0f);
+                if (b < 2) {
+                    const int nw = hv.x < 0 ? NORMAL_NONE : face < 0 ? face : 2 * face + half;
+                    (b == 0 ? a.xv : a.xs)[p] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(nw));
                 }
                 cont = !zero3(new_d) && (b + 1 < nb) && (!at_query || is_train);
                 if (cont) {
@@ -1326,7 +1323,7 @@ __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameAr
 
 }  // namespace
 
-vrg_status upload_frames(cudaStream_t s) {
+vrg_status upload_frames(cudaStream_t s, const float4 **table) {
     float4 t[12 * 3];
     for (int f = 0; f < 6; f++)
         for (int h = 0; h < 2; h++) {
@@ -1339,6 +1336,7 @@ vrg_status upload_frames(cudaStream_t s) {
             q[2] = make_float4(fr.b.x, fr.b.y, fr.b.z, 0.0f);
         }
     VRG_CUDA_TRY(cudaMemcpyToSymbolAsync(d_faces, t, sizeof(t), 0, cudaMemcpyHostToDevice, s));
+    VRG_CUDA_TRY(cudaGetSymbolAddress((void **)table, d_faces));
     return VRG_OK;
 }
 

@@ -25,6 +25,10 @@ constexpr int CNT_AHITS = 60;    // u64 at words 60-61: light hits collected by 
 constexpr int CNT_INFER = 48;    // radiance-cache queries of the frame
 constexpr int CNT_TRAIN = 49;    // radiance-cache training paths of the frame
 constexpr int MAX_BOUNCES = 8;
+// A vertex's normal in one word: 2 * face + half of a voxel face, bit 31 | its
+// record of a mesh triangle, or NORMAL_NONE (a miss).  (The two halves' normals
+// differ in the sign of zeros.)
+constexpr int NORMAL_NONE = 12;
 
 // The frame's stage times, written by its kernels: u64 nanoseconds of the
 // device's global timer from word CNT_STAMP on (0: the stage did not run).
@@ -128,7 +132,8 @@ struct FrameArgs {
     uint32_t *counters;
     uint8_t *nlive;
     float4 *rec;                  // [nb][2][P]: (E.xyz, w), (R.xyz, q)
-    float4 *xv, *nv, *xs, *ns;
+    float4 *xv, *xs;              // the first two vertices: position, normal word
+    const float4 *faces;          // face frames: normal, tangent, bitangent of 2 * face + half
     float4 *plain;                // L[0]
     float4 *res;                  // temporal ring slot [5][P]
     float4 *spatial;              // [5][P] (written when capture)

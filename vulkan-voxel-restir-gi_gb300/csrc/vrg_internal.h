@@ -128,6 +128,7 @@ struct Object {
 struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;
+    const float4 *faces = nullptr;       // the face frames' table on the device (upload_frames)
     std::vector<vrg_material> mats;
     DevBufPtr d_mats;                    // the material table, then reflectivity / pi per slot (lambert_of)
     DevBufPtr d_atlas;                   // texture atlas (RGBA8) + sRGB table, or empty
@@ -274,7 +275,7 @@ struct Renderer {
         uint2 *jmeta = nullptr;
         uint8_t *nlive = nullptr;
         float4 *rec = nullptr;                 // [nb][2][P]
-        float4 *xv = nullptr, *nv = nullptr, *xs = nullptr, *ns = nullptr;
+        float4 *xv = nullptr, *xs = nullptr;
         float4 *ray_tab = nullptr;             // per view: W + H primary-ray terms (ViewDev::ray_x, ray_y)
     };
     static constexpr int SETS = 3;        // frames whose bounces may be in flight at once (at most)
