@@ -172,7 +172,8 @@ typedef struct vrg_frame_stats {
     float ms_bounce[8];        /* per bounce: closest hit + shading (the light-pdf walk of
                                   bounce b runs on its own stream beside bounce b+1) */
     float ms_resolve;          /* outgoing radiance + temporal (+ cache inference/training) */
-    float ms_spatial;          /* spatial + finalize + pack */
+    float ms_spatial;          /* spatial + finalize + pack (a frame without reservoirs: the
+                                  outgoing radiance too) */
     uint64_t rays_closest;     /* closest-hit queries issued */
     uint64_t rays_any;         /* light any-hit queries issued */
     uint32_t error_flags;      /* device-side error word (stack overflow etc.) */

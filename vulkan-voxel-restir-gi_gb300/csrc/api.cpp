@@ -1110,7 +1110,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.nb_render = pr->num_bounces;
     a.cache = cache ? 1u : 0u;
     a.train_cap = cache ? nrc_batch(r->cache) : 0u;
-    a.restir = (pr->flags & VRG_RENDER_PLAIN_ONLY) ? 0u : 1u;
+    a.restir = a.nb >= 2 && !(pr->flags & VRG_RENDER_PLAIN_ONLY) ? 1u : 0u;
     {
         const Renderer::CacheSet &Q = r->cs[frame_set(r)];
         a.q_pos = Q.q_pos;

@@ -134,7 +134,7 @@ struct FrameArgs {
     float4 *rec;                  // [nb][2][P]: (E.xyz, w), (R.xyz, q)
     float4 *xv, *xs;              // the first two vertices: position, normal word
     const float4 *faces;          // face frames: normal, tangent, bitangent of 2 * face + half
-    float4 *plain;                // L[0]
+    float4 *plain;                // L[0], for the views that show it (debug_view 0)
     float4 *res;                  // temporal ring slot [5][P]
     float4 *spatial;              // [5][P] (written when capture)
     float4 *final_t;              // [P] (written when capture)
@@ -143,7 +143,7 @@ struct FrameArgs {
     double *accum;
     // radiance cache (VRG_RENDER_CACHE): paths end into the cache after
     // nb_render bounces; 1/16 of them (up to train_cap) trace to nb and train it
-    uint32_t nb_render, cache, train_cap, restir;  // restir: run the ReSTIR stages
+    uint32_t nb_render, cache, train_cap, restir;  // restir: reservoirs (two bounces or more)
     float4 *q_pos, *q_dir, *pred, *target;
     uint32_t *infer_list, *train_list;
     uint8_t *qflag;
