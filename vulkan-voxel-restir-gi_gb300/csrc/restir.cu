@@ -31,17 +31,6 @@ struct Res {
     float w_sum;
 };
 
-__device__ __forceinline__ Res load_res(const float4 *base, uint32_t P, uint32_t p) {
-    float4 a = base[p], b = base[P + p], c = base[2 * (size_t)P + p], d = base[3 * (size_t)P + p],
-           e = base[4 * (size_t)P + p];
-    Res r;
-    r.x_v = ld3(a); r.ucw = a.w;
-    r.n_v = ld3(b); r.w_sum = b.w;
-    r.x_s = ld3(c); r.m = __float_as_uint(c.w);
-    r.n_s = ld3(d); r.p_omega = d.w;
-    r.l = ld3(e); r.seed = __float_as_uint(e.w);
-    return r;
-}
 __device__ __forceinline__ void store_res(float4 *base, uint32_t P, uint32_t p, const Res &r) {
     base[p] = make_float4(r.x_v.x, r.x_v.y, r.x_v.z, r.ucw);
     base[P + p] = make_float4(r.n_v.x, r.n_v.y, r.n_v.z, r.w_sum);
@@ -164,45 +153,53 @@ __global__ void __launch_bounds__(256, 5) k_resolve(const __grid_constant__ Fram
         return;
     }
     if (a.debug_view == 0) a.plain[p] = make_float4(L.x, L.y, L.z, 0.0f);
-    // initial sample (interactive_rendering.rs:1359-1414)
-    Res S;
-    const float4 *tris = view_of<BATCH>(a, p).sc.tri_rec;
-    const float4 xv = a.xv[p];
-    S.x_v = ld3(xv);
-    S.n_v = vertex_normal<MESH>(a.faces, tris, xv.w);
-    if (nl >= 2) {
-        const float4 xs = a.xs[p];
-        S.x_s = ld3(xs);
-        S.n_s = vertex_normal<MESH>(a.faces, tris, xs.w);
-    } else {  // bounce 1 never traced: origin passes through, normal 0
-        S.x_s = S.x_v;
-        S.n_s = f3{0.0f, 0.0f, 0.0f};
-    }
-    S.l = L1;
-    S.p_omega = q0;
-    S.seed = 0;
-    // temporal resampling (restir_temporal_resampling.rs:256-301)
+    // The pixel's reservoir takes the frame's initial sample
+    // (interactive_rendering.rs:1359-1414) or keeps its own
+    // (restir_temporal_resampling.rs:256-301).  The choice reads the
+    // reservoir's w_sum, m and radiance only; a sample that is not taken is
+    // not read further, and one that is kept is not written again but for its
+    // first three planes, whose .w change.
     const ViewDev &V = view_of<BATCH>(a, p);
     const uint32_t ps = mm_combine(V.temporal_seed, p - V.pix_off);
-    Res R = load_res(a.res, P, p);
+    float4 r0 = a.res[p], r1 = a.res[(size_t)P + p], r2 = a.res[2 * (size_t)P + p];
+    const float4 r4 = a.res[4 * (size_t)P + p];
+    float w_sum = r1.w;
+    uint32_t m = __float_as_uint(r2.w);
     if (mm_rand(mm_combine(ps, 0)) < 0.4f) {
-        R.w_sum = 0.0f;
-        R.m = 0;
+        w_sum = 0.0f;
+        m = 0;
     }
-    if (a.mode == VRG_MODE_CONFIG && a.m_cap && R.m > a.m_cap) {  // M-cap (no reference counterpart)
-        R.w_sum = R.w_sum * ((float)a.m_cap / (float)R.m);
-        R.m = a.m_cap;
+    if (a.mode == VRG_MODE_CONFIG && a.m_cap && m > a.m_cap) {  // M-cap (no reference counterpart)
+        w_sum = w_sum * ((float)a.m_cap / (float)m);
+        m = a.m_cap;
     }
-    const float w = luminance3(S.l) / S.p_omega;
-    R.w_sum += w;
-    R.m += 1;
-    if (float_construct(mm_finalize(mm_combine(ps, 1))) < w / R.w_sum) {
-        R.x_v = S.x_v; R.n_v = S.n_v; R.x_s = S.x_s; R.n_s = S.n_s; R.l = S.l;
-        R.p_omega = S.p_omega; R.seed = S.seed;
+    const float w = luminance3(L1) / q0;
+    w_sum += w;
+    m += 1;
+    f3 l = ld3(r4);
+    if (float_construct(mm_finalize(mm_combine(ps, 1))) < w / w_sum) {
+        l = L1;
+        const float4 *tris = view_of<BATCH>(a, p).sc.tri_rec;
+        r0 = a.xv[p];
+        const f3 n_v = vertex_normal<MESH>(a.faces, tris, r0.w);
+        r1 = make_float4(n_v.x, n_v.y, n_v.z, 0.0f);
+        f3 n_s = f3{0.0f, 0.0f, 0.0f};
+        if (nl >= 2) {
+            r2 = a.xs[p];
+            n_s = vertex_normal<MESH>(a.faces, tris, r2.w);
+        } else {  // bounce 1 never traced: origin passes through, normal 0
+            r2 = r0;
+        }
+        a.res[3 * (size_t)P + p] = make_float4(n_s.x, n_s.y, n_s.z, q0);
+        a.res[4 * (size_t)P + p] = make_float4(l.x, l.y, l.z, __uint_as_float(0u));
     }
-    const float ph = luminance3(R.l);
-    R.ucw = (ph > 0.0f) ? R.w_sum / ((float)R.m * ph) : 0.0f;
-    store_res(a.res, P, p, R);
+    const float ph = luminance3(l);
+    r0.w = (ph > 0.0f) ? w_sum / ((float)m * ph) : 0.0f;
+    r1.w = w_sum;
+    r2.w = __uint_as_float(m);
+    a.res[p] = r0;
+    a.res[(size_t)P + p] = r1;
+    a.res[2 * (size_t)P + p] = r2;
 }
 
 // Where the spatial pass reads reservoirs: straight from the ring slot, or
