@@ -87,8 +87,11 @@ __device__ __forceinline__ void finish_pixel(const FrameArgs &a, uint32_t p, f3 
 // The outgoing radiance is the frame: this pass finishes the pixel, and there
 // is no spatial pass (1080p, 8 bounces, accumulated: 1813 us with the radiance
 // written here and finished there, 1784 in one).
+// Bound by memory: 8 CTAs per SM at 32 registers, though the reservoirs' variant
+// then spills 32 bytes (1080p in flight 840 us at 5 CTAs and 44 registers, 834 at
+// 6, 831 at 8).
 template <bool CAPTURE, bool BATCH, bool MESH, bool PLAIN>
-__global__ void __launch_bounds__(256, 5) k_resolve(const __grid_constant__ FrameArgs a) {
+__global__ void __launch_bounds__(256, 8) k_resolve(const __grid_constant__ FrameArgs a) {
     const uint32_t P = a.P;
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
