@@ -563,13 +563,12 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
     size_t o = 0;
     // the arrays of a frame's bounces, one set per frame in flight
     struct SetOff {
-        size_t ro, rd, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, xs, rt;
+        size_t ray, q0, q1, cnt, aq0, aq1, aj0, aj1, hit, hb, hv, jm, nl, rec, xv, xs, rt;
     } so[Renderer::SETS];
     const int sets = (int)r->n_sets;
     for (int k = 0; k < sets; k++) {
         SetOff &q = so[k];
-        q.ro = o; o += al(P * 16);
-        q.rd = o; o += al(P * 16);
+        q.ray = o; o += al(P * 32);
         q.q0 = o; o += al(P * 4);
         q.q1 = o; o += al(P * 4);
         q.cnt = o; o += al(CNT_WORDS * 4);
@@ -599,8 +598,7 @@ static vrg_status renderer_alloc(vrg_renderer *r) {
     for (int k = 0; k < Renderer::SETS; k++) {
         const SetOff &q = so[k < sets ? k : 0];
         Renderer::FrameSet &F = r->fs[k];
-        F.ray_o = (float4 *)(B + q.ro);
-        F.ray_d = (float4 *)(B + q.rd);
+        F.ray = (float4 *)(B + q.ray);
         F.queue[0] = (uint32_t *)(B + q.q0);
         F.queue[1] = (uint32_t *)(B + q.q1);
         F.counters = (uint32_t *)(B + q.cnt);
@@ -1136,8 +1134,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.accumulate = pr->accumulate;
     a.pack = (pr->flags & VRG_RENDER_NO_PACK) ? 0u : 1u;
     const Renderer::FrameSet &F = r->fs[frame_set(r)];
-    a.ray_o = F.ray_o;
-    a.ray_d = F.ray_d;
+    a.ray = F.ray;
     a.queue[0] = F.queue[0];
     a.queue[1] = F.queue[1];
     a.aqueue[0] = F.aqueue[0];

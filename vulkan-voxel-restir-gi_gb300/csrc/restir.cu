@@ -132,15 +132,15 @@ __global__ void __launch_bounds__(256, 8) k_resolve(const __grid_constant__ Fram
             const float4 pr = a.pred[p];
             L = f3{pr.x, pr.y, pr.z};
         } else {
-            const float4 e = a.rec[(size_t)qb * 2 * P + p];
+            const float4 e = a.rec[2 * ((size_t)qb * P + p)];
             L = f3{e.x, e.y, e.z};
         }
         if (qb == 1) L1 = L;
         top = qb - 1;
     }
     for (int b = top; b >= 0; b--) {
-        const size_t rb = (size_t)b * 2 * P;
-        const float4 e = a.rec[rb + p], r = a.rec[rb + P + p];
+        float4 e, r;
+        ld2(a.rec + 2 * ((size_t)b * P + p), e, r);
         // L = E + R * L * (bsdf_pdf / q) * valid, valid = 1 for traced rays
         L = f3{e.x + (r.x * L.x) * e.w, e.y + (r.y * L.y) * e.w, e.z + (r.z * L.z) * e.w};
         if (b == 1) L1 = L;
@@ -298,7 +298,8 @@ __device__ __forceinline__ void spatial_pixel(const FrameArgs &a, uint32_t p, co
     // finalize (restir_finalize.rs:121-141)
     const f3 dir = norm3(sub3(Rs.x_s, ld3(a.xv[p])));
     const float bp = dot3(dir, Rs.n_v) / PI_F;
-    const float4 e0 = a.rec[p], r0 = a.rec[P + p];
+    float4 e0, r0;
+    ld2(a.rec + 2 * (size_t)p, e0, r0);
     fin = f3{e0.x + ((r0.x * Rs.l.x) * Rs.ucw) * bp, e0.y + ((r0.y * Rs.l.y) * Rs.ucw) * bp,
              e0.z + ((r0.z * Rs.l.z) * Rs.ucw) * bp};
     ucw_view = Rs.ucw;
@@ -406,8 +407,8 @@ __global__ void __launch_bounds__(256) k_train_targets(const __grid_constant__ F
     const int nl = a.nlive[p], qb = (int)a.nb_render - 1;
     f3 L = f3{0.0f, 0.0f, 0.0f};
     for (int b = nl - 1; b >= qb; b--) {
-        const size_t rb = (size_t)b * 2 * P;
-        const float4 e = a.rec[rb + p], r = a.rec[rb + P + p];
+        float4 e, r;
+        ld2(a.rec + 2 * ((size_t)b * P + p), e, r);
         L = f3{e.x + (r.x * L.x) * e.w, e.y + (r.y * L.y) * e.w, e.z + (r.z * L.z) * e.w};
     }
     a.target[p] = make_float4(L.x, L.y, L.z, 0.0f);

@@ -506,7 +506,12 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ FrameA
                         root = V.sc.geo_root;
                     }
                     if (b == 0) raygen(V, x, y, o, d);
-                    else { o = ld3(a.ray_o[p]); d = ld3(a.ray_d[p]); }
+                    else {
+                        float4 ro, rd;
+                        ld2(a.ray + 2 * (size_t)p, ro, rd);
+                        o = ld3(ro);
+                        d = ld3(rd);
+                    }
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
                     slab_offsets(o, inv, ray_margin(extent, o), oin, oif);
                     px = signbit(inv.x) ? 1 : 0;
@@ -899,8 +904,10 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                         st3(a.c_dir, p, d);
                     }
                 } else {
-                    o = ld3(a.ray_o[p]);
-                    d = ld3(a.ray_d[p]);
+                    float4 ro, rd;
+                    ld2(a.ray + 2 * (size_t)p, ro, rd);
+                    o = ld3(ro);
+                    d = ld3(rd);
                 }
                 const uint32_t seed = mm_combine(V.frame * nb + b, lp);  // interactive_rendering.rs:1189
                 const int4 hv = a.hits[p];
@@ -974,13 +981,11 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 const float mis = stash_mis;
                 const int4 hv = stash_hit, rc = stash_rc;
                 const int half = stash_half;
-                const size_t rb = (size_t)b * 2 * P;
                 // the record without a light hit; a light-pdf job whose ray crosses
                 // lights gets its q and w from k_hit_eval / k_hit_sum
                 const float q = 0.0f * mis + (1.0f - mis) * inv2pi;
                 const float w = pdf / q;
-                a.rec[rb + p] = make_float4(E.x, E.y, E.z, w);
-                a.rec[rb + P + p] = make_float4(R.x, R.y, R.z, q);
+                st2(a.rec + 2 * ((size_t)b * P + p), make_float4(E.x, E.y, E.z, w), make_float4(R.x, R.y, R.z, q));
                 if (b < 2) {
                     const int nw = hv.x < 0 ? NORMAL_NONE : face < 0 ? face : 2 * face + half;
                     (b == 0 ? a.xv : a.xs)[p] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(nw));
@@ -988,8 +993,8 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                 cont = !zero3(new_d) && (b + 1 < nb) && (!at_query || is_train);
                 if (cont) {
                     // .w of the ray carries the face and the bsdf pdf to k_anyhit
-                    a.ray_o[p] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(face));
-                    a.ray_d[p] = make_float4(new_d.x, new_d.y, new_d.z, pdf);
+                    st2(a.ray + 2 * (size_t)p, make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(face)),
+                        make_float4(new_d.x, new_d.y, new_d.z, pdf));
                 } else {
                     a.nlive[p] = (uint8_t)(b + 1);
                 }
@@ -1041,8 +1046,8 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
             if (anyj) {
                 const uint32_t j = ab + __popc(am & lanemask_lt());
                 a.aqueue[b & 1][j] = p;
-                a.ajob[b & 1][2 * (size_t)j] = make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(face));
-                a.ajob[b & 1][2 * (size_t)j + 1] = make_float4(new_d.x, new_d.y, new_d.z, pdf);
+                st2(a.ajob[b & 1] + 2 * (size_t)j, make_float4(new_o.x, new_o.y, new_o.z, __int_as_float(face)),
+                    make_float4(new_d.x, new_d.y, new_d.z, pdf));
             }
         }
         // (the end of the CTA's first warp; behind the loop the same stamp made
@@ -1070,9 +1075,9 @@ __device__ __forceinline__ void finish_job(const FrameArgs &a, uint32_t b, uint3
     const float mis = 0.3f;
     const float q = nee * mis + (1.0f - mis) * inv2pi;
     const float w = pdf / q;
-    const size_t rb = (size_t)b * 2 * a.P;
-    reinterpret_cast<float *>(a.rec + rb + p)[3] = w;
-    reinterpret_cast<float *>(a.rec + rb + a.P + p)[3] = q;
+    float4 *rec = a.rec + 2 * ((size_t)b * a.P + p);
+    rec[0].w = w;
+    rec[1].w = q;
 }
 
 // a job's hits in ascending key order
@@ -1152,8 +1157,10 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
                         root = V.sc.lamp_root;
                         extent = V.sc.extent;
                     }
-                    o = ld3(a.ajob[b & 1][2 * (size_t)idx]);
-                    d = ld3(a.ajob[b & 1][2 * (size_t)idx + 1]);
+                    float4 ro, rd;
+                    ld2(a.ajob[b & 1] + 2 * (size_t)idx, ro, rd);
+                    o = ld3(ro);
+                    d = ld3(rd);
                     inv = f3{slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)};
                     slab_offsets(o, inv, ray_margin(extent, o), oin, oif);
                     px = signbit(inv.x) ? 1 : 0;
@@ -1255,9 +1262,10 @@ __global__ void __launch_bounds__(128, 8) k_anyhit(const __grid_constant__ Frame
             const bool fits = hb + cnt <= a.hit_cap;
             if (!fits) atomicOr(err, ERR_LIGHT_LIST);
             for (uint32_t j = 0; j < cnt && hb + j < a.hit_cap; j++) {
-                a.hitbuf[2 * (size_t)(hb + j)] =
-                    make_uint4(p, (uint32_t)(hits.key[j] >> 32), (uint32_t)hits.key[j], __float_as_uint(hits.b1[j]));
-                a.hitbuf[2 * (size_t)(hb + j) + 1] = make_uint4(__float_as_uint(hits.b2[j]), idx, fits ? cnt : 0u, 0u);
+                st2(reinterpret_cast<float4 *>(a.hitbuf) + 2 * (size_t)(hb + j),
+                    as_float4(make_uint4(p, (uint32_t)(hits.key[j] >> 32), (uint32_t)hits.key[j],
+                                         __float_as_uint(hits.b1[j]))),
+                    as_float4(make_uint4(__float_as_uint(hits.b2[j]), idx, fits ? cnt : 0u, 0u)));
             }
             // the jobs with several hits, for the sum (a job past the hit
             // buffer's end has none to sum)
@@ -1280,10 +1288,13 @@ template <bool CAPTURE, bool BATCH>
 __global__ void __launch_bounds__(128) k_hit_eval(const __grid_constant__ FrameArgs a, uint32_t b) {
     const uint32_t n = min(a.counters[CNT_HITS + 2 * b], a.hit_cap);
     for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < n; h += gridDim.x * blockDim.x) {
-        const uint4 A = a.hitbuf[2 * (size_t)h], B = a.hitbuf[2 * (size_t)h + 1];
+        float4 h0, h1;
+        ld2(reinterpret_cast<const float4 *>(a.hitbuf) + 2 * (size_t)h, h0, h1);
+        const uint4 A = as_uint4(h0), B = as_uint4(h1);
         if (B.z == 0) continue;  // of a job that did not fit the hit buffer
         const uint32_t p = A.x;
-        const float4 ro = a.ajob[b & 1][2 * (size_t)B.y], rd = a.ajob[b & 1][2 * (size_t)B.y + 1];
+        float4 ro, rd;
+        ld2(a.ajob[b & 1] + 2 * (size_t)B.y, ro, rd);
         const DevScene &sc = view_of<BATCH>(a, p).sc;
         // the shading normal of the job's vertex: a voxel face's, or a mesh
         // triangle's, recomputed as its shading computed it

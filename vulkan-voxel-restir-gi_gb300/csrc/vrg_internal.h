@@ -264,7 +264,7 @@ struct Renderer {
     // and spatial passes, which run one frame after the other on the library
     // stream.
     struct FrameSet {
-        float4 *ray_o = nullptr, *ray_d = nullptr;
+        float4 *ray = nullptr;
         uint32_t *queue[2] = {nullptr, nullptr};
         uint32_t *counters = nullptr;          // CNT_* words of vrg_frame.cuh
         uint32_t *aqueue[2] = {nullptr, nullptr};  // light-pdf jobs by bounce parity
@@ -274,7 +274,7 @@ struct Renderer {
         float *hitval = nullptr;
         uint2 *jmeta = nullptr;
         uint8_t *nlive = nullptr;
-        float4 *rec = nullptr;                 // [nb][2][P]
+        float4 *rec = nullptr;                 // [nb][P][2]
         float4 *xv = nullptr, *xs = nullptr;
         float4 *ray_tab = nullptr;             // per view: W + H primary-ray terms (ViewDev::ray_x, ray_y)
     };
