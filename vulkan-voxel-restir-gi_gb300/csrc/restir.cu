@@ -58,7 +58,7 @@ __device__ __forceinline__ f3 vertex_normal(const float4 *faces, const float4 *t
         const float4 *q = tris + 3 * (size_t)((uint32_t)nw & 0x7FFFFFFFu);
         return tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2))).n;
     }
-    return ld3(__ldg(faces + 3 * nw));
+    return ld3(__ldg(faces + FACE_ROW * nw));
 }
 
 __device__ __forceinline__ uint8_t to_u8(float x) {

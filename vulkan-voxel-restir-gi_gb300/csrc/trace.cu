@@ -24,10 +24,10 @@
 
 namespace vrg {
 
-// Per (face, half): (normal, corner bits of the triangle's vertices: 3 x 3
-// bits), tangent, bitangent.  In global memory, not constant memory: the lanes
+// Per (face, half), FACE_ROW float4: (normal, corner bits of the triangle's
+// vertices: 3 x 3 bits), unused, tangent, bitangent.  In global memory, not constant memory: the lanes
 // of a warp shade different faces, and constant loads serialize over them.
-__device__ float4 d_faces[12 * 3];
+__device__ __align__(32) float4 d_faces[12 * FACE_ROW];
 
 namespace {
 
@@ -91,7 +91,9 @@ struct LightPair {
 template <bool NEE>
 __device__ __forceinline__ LightPair light_pair(const DevScene &sc, const ImpPt &P, uint32_t g) {
     const float4 *q = sc.light_pair + LIGHT_PAIR * (size_t)g;
-    const float4 a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
+    float4 a, b;
+    ldg2(q, a, b);
+    const float4 d = __ldg(q + 2);
     const float eps = NEE ? EPS_NEE : EPS_TRACE;
     const float2 half = make_float2(0.5f, 0.5f);
     const f3 point = P.point;
@@ -683,7 +685,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
             face = hv.y & 7;
             half = (hv.y >> 3) & 1;
             const int wx = rec_wx(rc), wy = rec_wy(rc), wz = rec_wz(rc);
-            ft = d_faces + 3 * (2 * face + half);
+            ft = d_faces + FACE_ROW * (2 * face + half);
             const float4 q = __ldg(ft);
             const uint32_t cb = __float_as_uint(q.w);
             fr.n = ld3(q);
@@ -764,8 +766,10 @@ __device__ __forceinline__ void shade_vertex(const DevScene &S, uint32_t nee_typ
                 const float vv = sqrtf(fmaxf(0.0f, 1.0f - uy * uy));
                 const f3 hs = f3{vv * c, uy, vv * s};
                 if (!MESH || ft) {
-                    fr.t = ld3(__ldg(ft + 1));
-                    fr.b = ld3(__ldg(ft + 2));
+                    float4 ta, bi;
+                    ldg2(ft + 2, ta, bi);
+                    fr.t = ld3(ta);
+                    fr.b = ld3(bi);
                 } else {  // (worked out again here, not carried through the descent)
                     const float4 *q = S.tri_rec + 3 * (size_t)((uint32_t)face & 0x7FFFFFFFu);
                     fr = tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2)));
@@ -1301,7 +1305,7 @@ __global__ void __launch_bounds__(128) k_hit_eval(const __grid_constant__ FrameA
         const int fw = __float_as_int(ro.w);
         f3 n3;
         if (fw >= 0) {
-            n3 = ld3(__ldg(d_faces + 6 * fw));
+            n3 = ld3(__ldg(d_faces + 2 * FACE_ROW * fw));
         } else {
             const float4 *q = sc.tri_rec + 3 * (size_t)((uint32_t)fw & 0x7FFFFFFFu);
             n3 = tri_frame(ld3(__ldg(q)), ld3(__ldg(q + 1)), ld3(__ldg(q + 2))).n;
@@ -1335,16 +1339,16 @@ __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameAr
 }  // namespace
 
 vrg_status upload_frames(cudaStream_t s, const float4 **table) {
-    float4 t[12 * 3];
+    float4 t[12 * FACE_ROW] = {};
     for (int f = 0; f < 6; f++)
         for (int h = 0; h < 2; h++) {
             const Frame fr = face_frame(f, h);
             const uint32_t bits = face_corner(f, h, 0) | face_corner(f, h, 1) << 3 | face_corner(f, h, 2) << 6;
-            float4 *q = t + 3 * (2 * f + h);
+            float4 *q = t + FACE_ROW * (2 * f + h);
             q[0] = make_float4(fr.n.x, fr.n.y, fr.n.z, 0.0f);
             memcpy(&q[0].w, &bits, 4);
-            q[1] = make_float4(fr.t.x, fr.t.y, fr.t.z, 0.0f);
-            q[2] = make_float4(fr.b.x, fr.b.y, fr.b.z, 0.0f);
+            q[2] = make_float4(fr.t.x, fr.t.y, fr.t.z, 0.0f);
+            q[3] = make_float4(fr.b.x, fr.b.y, fr.b.z, 0.0f);
         }
     VRG_CUDA_TRY(cudaMemcpyToSymbolAsync(d_faces, t, sizeof(t), 0, cudaMemcpyHostToDevice, s));
     VRG_CUDA_TRY(cudaGetSymbolAddress((void **)table, d_faces));

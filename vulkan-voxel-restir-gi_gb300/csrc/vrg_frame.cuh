@@ -29,6 +29,7 @@ constexpr int MAX_BOUNCES = 8;
 // record of a mesh triangle, or NORMAL_NONE (a miss).  (The two halves' normals
 // differ in the sign of zeros.)
 constexpr int NORMAL_NONE = 12;
+constexpr int FACE_ROW = 4;
 
 // The frame's stage times, written by its kernels: u64 nanoseconds of the
 // device's global timer from word CNT_STAMP on (0: the stage did not run).
@@ -133,7 +134,7 @@ struct FrameArgs {
     uint8_t *nlive;
     float4 *rec;                  // [nb][P][2]: (E.xyz, w), (R.xyz, q)
     float4 *xv, *xs;              // the first two vertices: position, normal word
-    const float4 *faces;          // face frames: normal, tangent, bitangent of 2 * face + half
+    const float4 *faces;          // face frames: FACE_ROW float4 per 2 * face + half, the normal first
     float4 *plain;                // L[0], for the views that show it (debug_view 0)
     float4 *res;                  // temporal ring slot [5][P]
     float4 *spatial;              // [5][P] (written when capture)
@@ -163,6 +164,12 @@ __device__ __forceinline__ void ld2(const float4 *p, float4 &a, float4 &b) {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                  : "l"(p));
+}
+// (of data no kernel running beside writes)
+__device__ __forceinline__ void ldg2(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
 }
 __device__ __forceinline__ uint4 as_uint4(float4 v) {
     return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
