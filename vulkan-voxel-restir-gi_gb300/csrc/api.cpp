@@ -19,6 +19,8 @@ vrg_status launch_frame_begin(cudaStream_t s, const FrameArgs &a, uint32_t max_e
 vrg_status launch_light_pdf(cudaStream_t s, const FrameArgs &a, uint32_t b, uint32_t max_rays);
 vrg_status launch_resolve(cudaStream_t s, const FrameArgs &a);
 vrg_status launch_spatial(cudaStream_t s, const FrameArgs &a, const CUtensorMap *res_map);
+vrg_status launch_ring_planes(cudaStream_t s, float4 *slot, uint32_t P, uint32_t p0, uint32_t n, float4 *planes,
+                              bool to_slot);
 vrg_status launch_train_targets(cudaStream_t s, const FrameArgs &a);
 void bounce_occupancy(bool batch, int occ[3], int *sms);
 
@@ -936,19 +938,22 @@ static EncodeTiledFn encode_tiled() {
     return fn;
 }
 
+// float4 from one ring slot to the next: 5 per pixel, each slot at a 32-byte boundary
+static size_t ring_stride(size_t P) { return (5 * P + 1) & ~(size_t)1; }
+
 // Tensor maps of the ring slots for the TMA-staged spatial pass: a single
-// view's slot [5 planes][H rows][W pixels x 4 floats], boxes of 32 pixels x 8
-// rows x 5 planes (the 16-byte aligned inner coordinate is 4 x the pixel)
+// view's slot, its pairs [2][H rows][W pixels x 8 floats], boxes of 32 pixels x
+// 8 rows x 2 (the 16-byte aligned inner coordinate is 8 x the pixel)
 static void make_res_maps(vrg_renderer *r) {
     r->res_map_ok = false;
     EncodeTiledFn enc = encode_tiled();
     if (!enc || r->n_views != 0 || r->W < 32 || r->H < 8 || r->ring_slots > 8) return;
     const cuuint64_t P = (cuuint64_t)r->P;
-    const cuuint64_t dims[3] = {4 * (cuuint64_t)r->W, r->H, 5};
-    const cuuint64_t strides[2] = {16 * (cuuint64_t)r->W, 16 * P};
-    const cuuint32_t box[3] = {4 * 32, 8, 5}, estr[3] = {1, 1, 1};
+    const cuuint64_t dims[3] = {8 * (cuuint64_t)r->W, r->H, 2};
+    const cuuint64_t strides[2] = {32 * (cuuint64_t)r->W, 32 * P};
+    const cuuint32_t box[3] = {8 * 32, 8, 2}, estr[3] = {1, 1, 1};
     for (uint32_t k = 0; k < r->ring_slots; k++)
-        if (enc(&r->res_map[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)(r->res + (size_t)k * 5 * P), dims,
+        if (enc(&r->res_map[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)(r->res + k * ring_stride(P)), dims,
                 strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return;
@@ -960,8 +965,8 @@ static vrg_status ensure_ring(vrg_renderer *r, uint32_t slots) {
     const size_t P = (size_t)r->P;
     cudaStream_t s = r->ctx->stream;
     DevBufPtr b;
-    VRG_TRY(dev_alloc(s, (size_t)slots * 5 * P * 16, b));
-    VRG_CUDA_TRY(cudaMemsetAsync(b->ptr, 0, (size_t)slots * 5 * P * 16, s));
+    VRG_TRY(dev_alloc(s, slots * ring_stride(P) * 16, b));
+    VRG_CUDA_TRY(cudaMemsetAsync(b->ptr, 0, slots * ring_stride(P) * 16, s));
     drop_graphs(r);
     r->res_buf = b;
     r->res = (float4 *)b->ptr;
@@ -1153,7 +1158,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.xs = F.xs;
     a.faces = r->ctx->faces;
     a.plain = r->plain;
-    a.res = r->res + (size_t)ring * 5 * P;
+    a.res = r->res + ring * ring_stride(P);
     a.spatial = r->spatial;
     a.final_t = r->final_t;
     a.bgra = r->bgra;
@@ -1367,7 +1372,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool pipelin
     // slot has its tensor map
     const CUtensorMap *res_map = nullptr;
     if (effective_tuning(r).spatial_staging == 1 && r->res_map_ok && !in_graph && r->ring_slots) {
-        const size_t slot = (size_t)(a.res - r->res) / (5 * (size_t)r->P);
+        const size_t slot = (size_t)(a.res - r->res) / ring_stride(r->P);
         if (slot < r->ring_slots) res_map = &r->res_map[slot];
     }
     VRG_TRY(launch_spatial(s, a, res_map));
@@ -1694,6 +1699,33 @@ VRG_API vrg_status vrg_renderer_state_size(vrg_renderer *r, uint64_t *bytes) {
     return VRG_OK;
 }
 
+// The ring slots to (save) or from the saved state's five planes per slot,
+// through at most 2^18 pixels of device scratch at a time.
+static vrg_status copy_ring(vrg_renderer *r, uint8_t *host, bool save) {
+    cudaStream_t s = r->ctx->stream;
+    const uint32_t P = (uint32_t)r->P, part = std::min<uint32_t>(P, 1u << 18);
+    if (!r->ring_slots) return VRG_OK;
+    DevBufPtr b;
+    VRG_TRY(dev_alloc(r->ctx, (size_t)part * 80, b));
+    float4 *planes = (float4 *)b->ptr;
+    for (uint32_t k = 0; k < r->ring_slots; k++) {
+        float4 *slot = r->res + k * ring_stride(P);
+        uint8_t *hk = host + (size_t)k * 5 * P * 16;
+        for (uint32_t p0 = 0; p0 < P; p0 += part) {
+            const uint32_t n = std::min(part, P - p0);
+            if (save) VRG_TRY(launch_ring_planes(s, slot, P, p0, n, planes, false));
+            for (int q = 0; q < 5; q++) {
+                uint8_t *h = hk + ((size_t)q * P + p0) * 16;
+                float4 *d = planes + (size_t)q * n;
+                if (save) VRG_CUDA_TRY(cudaMemcpyAsync(h, d, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
+                else VRG_CUDA_TRY(cudaMemcpyAsync(d, h, (size_t)n * 16, cudaMemcpyHostToDevice, s));
+            }
+            if (!save) VRG_TRY(launch_ring_planes(s, slot, P, p0, n, planes, true));
+        }
+    }
+    return VRG_OK;
+}
+
 VRG_API vrg_status vrg_renderer_state_save(vrg_renderer *r, void *dst, uint64_t bytes) {
     if (!r || !dst || bytes < state_bytes(r)) return VRG_ERR_INVALID_ARGUMENT;
     cudaStream_t s = r->ctx->stream;
@@ -1702,7 +1734,7 @@ VRG_API vrg_status vrg_renderer_state_save(vrg_renderer *r, void *dst, uint64_t 
     memcpy(d, &h, sizeof(h));
     d += sizeof(h);
     const size_t ring = (size_t)r->ring_slots * 5 * r->P * 16;
-    if (ring) VRG_CUDA_TRY(cudaMemcpyAsync(d, r->res, ring, cudaMemcpyDeviceToHost, s));
+    VRG_TRY(copy_ring(r, d, true));
     VRG_CUDA_TRY(cudaMemcpyAsync(d + ring, r->accum, (size_t)r->P * 24, cudaMemcpyDeviceToHost, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
     return VRG_OK;
@@ -1722,7 +1754,7 @@ VRG_API vrg_status vrg_renderer_state_load(vrg_renderer *r, const void *src, uin
     if (h.ring_slots) VRG_TRY(ensure_ring(r, h.ring_slots));
     cudaStream_t s = r->ctx->stream;
     const uint8_t *p = (const uint8_t *)src + sizeof(h);
-    if (ring) VRG_CUDA_TRY(cudaMemcpyAsync(r->res, p, ring, cudaMemcpyHostToDevice, s));
+    if (h.ring_slots) VRG_TRY(copy_ring(r, const_cast<uint8_t *>(p), false));
     VRG_CUDA_TRY(cudaMemcpyAsync(r->accum, p + ring, (size_t)r->P * 24, cudaMemcpyHostToDevice, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
     r->frame = h.frame;
@@ -1770,7 +1802,7 @@ VRG_API vrg_status vrg_renderer_autotune(vrg_renderer *r, vrg_scene *scene, cons
     VRG_TRY(scene_commit(scene));
     VRG_TRY(ensure_ring(r, slots));
     // state the tuning frames change: frame counter and reservoir history
-    const size_t ring_bytes = (size_t)slots * 5 * (size_t)r->P * 16;
+    const size_t ring_bytes = slots * ring_stride(r->P) * 16;
     DevBufPtr saved;
     VRG_TRY(dev_alloc(s, ring_bytes, saved));
     VRG_CUDA_TRY(cudaMemcpyAsync(saved->ptr, r->res, ring_bytes, cudaMemcpyDeviceToDevice, s));
@@ -1895,15 +1927,16 @@ VRG_API vrg_status vrg_debug_readback(vrg_renderer *r, uint32_t what, void *dst,
         VRG_CUDA_TRY(cudaStreamSynchronize(s));
         return VRG_OK;
     };
-    auto copy_res = [&](const float4 *planes) -> vrg_status {
+    auto copy_res = [&](const float4 *slot) -> vrg_status {
         if (bytes < P * 80) return VRG_ERR_INVALID_ARGUMENT;
         std::vector<float4> h(5 * P);
-        VRG_CUDA_TRY(cudaMemcpyAsync(h.data(), planes, 5 * P * 16, cudaMemcpyDeviceToHost, s));
+        VRG_CUDA_TRY(cudaMemcpyAsync(h.data(), slot, 5 * P * 16, cudaMemcpyDeviceToHost, s));
         VRG_CUDA_TRY(cudaStreamSynchronize(s));
         float *o = (float *)dst;
         for (size_t p = 0; p < P; p++) {
             float *d = o + 20 * p;
-            const float4 &a = h[p], &b = h[P + p], &c = h[2 * P + p], &e = h[3 * P + p], &l = h[4 * P + p];
+            const float4 &a = h[2 * p], &b = h[2 * p + 1], &c = h[2 * (P + p)], &l = h[2 * (P + p) + 1],
+                         &e = h[4 * P + p];
             d[0] = a.x; d[1] = a.y; d[2] = a.z;
             d[3] = b.x; d[4] = b.y; d[5] = b.z;
             d[6] = c.x; d[7] = c.y; d[8] = c.z;
@@ -1929,7 +1962,7 @@ VRG_API vrg_status vrg_debug_readback(vrg_renderer *r, uint32_t what, void *dst,
     case VRG_DBG_RADIANCE: return copy(r->c_L, nb * P * 12);
     case VRG_DBG_Q: return copy(r->c_q, nb * P * 4);
     case VRG_DBG_HIT: return copy(r->c_hit, nb * P * 16);
-    case VRG_DBG_TEMPORAL: return copy_res(r->res + (size_t)r->last_ring * 5 * P);
+    case VRG_DBG_TEMPORAL: return copy_res(r->res + r->last_ring * ring_stride(P));
     case VRG_DBG_SPATIAL: return copy_res(r->spatial);
     case VRG_DBG_FINAL: {
         if (bytes < P * 12) return VRG_ERR_INVALID_ARGUMENT;

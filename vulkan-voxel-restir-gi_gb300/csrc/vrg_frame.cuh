@@ -136,8 +136,8 @@ struct FrameArgs {
     float4 *xv, *xs;              // the first two vertices: position, normal word
     const float4 *faces;          // face frames: FACE_ROW float4 per 2 * face + half, the normal first
     float4 *plain;                // L[0], for the views that show it (debug_view 0)
-    float4 *res;                  // temporal ring slot [5][P]
-    float4 *spatial;              // [5][P] (written when capture)
+    float4 *res;                  // temporal ring slot (res_pair in restir.cu)
+    float4 *spatial;              // likewise (written when capture)
     float4 *final_t;              // [P] (written when capture)
     uint8_t *bgra;
     float *radiance;

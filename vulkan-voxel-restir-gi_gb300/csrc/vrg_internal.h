@@ -283,9 +283,9 @@ struct Renderer {
                                           // (2 -> 3: 1.264 -> 1.247 ms per 1080p frame)
     FrameSet fs[SETS];
     float4 *plain = nullptr;              // L[0] per pixel
-    float4 *res = nullptr;                // [ring][5][P] temporal reservoirs
+    float4 *res = nullptr;                // temporal reservoirs, ring_stride(P) per slot
     DevBufPtr res_buf;
-    float4 *spatial = nullptr;            // [5][P] spatial reservoirs (capture)
+    float4 *spatial = nullptr;            // spatial reservoirs (capture), laid out as a slot
     float4 *final_t = nullptr;            // restir final target (capture)
     uint8_t *bgra = nullptr;
     float *radiance = nullptr;            // [P*3]
