@@ -1408,6 +1408,9 @@ static vrg_status frame_stats(vrg_renderer *r, const FrameArgs &a, bool per_kern
         const uint32_t nb_main = (a.cache && !a.capture) ? a.nb_render : a.nb;
         double end = 0.0, main_end = 0.0;
         for (uint32_t b = 0; b < a.nb; b++) {
+            // (a forked cache frame's training bounces run beside the main
+            // stream, from the query bounce's light-pdf walk on)
+            if (b == nb_main) end = at(ST_WALK + nb_main - 1, 0.0);
             const double traced = at(ST_TRACED + b, end), shaded = at(ST_SHADED + b, traced);
             stats->ms_bounce[b] = (float)(shaded - end);
             stats->ms_trace[b] = (float)(traced - end);
