@@ -596,7 +596,8 @@ struct TrainArgs {
     __nv_bfloat16 *dZ;          // [6][n_pad][64] pre-activation gradients (layer 5: 16 used)
     size_t n_pad;               // rows per layer of H and dZ (the buffers' allocation, >= n)
     float2 *gtable;             // hash-grid gradients (fp32)
-    float *loss;                // summed loss
+    double *loss;               // summed loss (in 64 bits: as one 32-bit word its last digits
+                                // followed the order of the warps' adds)
     uint32_t *err;              // error word (ERR_COPY)
     float4 *pred;               // optional: the forward pass's prediction per sample
     const uint32_t *enc;        // tensor-core pass: the encoded input rows (k_nrc_encode layout)
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(NRC_WARPS * 32) k_nrc_train(TrainArgs a) {
     const uint32_t warps = gridDim.x * NRC_WARPS;
     const uint32_t n = a.n_dev ? min(*a.n_dev, a.n) : a.n;
     const float inv_n = n ? 1.0f / (float)n : 0.0f;
-    float loss_acc = 0.0f;
+    double loss_acc = 0.0;
     for (uint32_t base = (blockIdx.x * NRC_WARPS + w) * 32; base < n; base += warps * 32) {
         const uint32_t i = base + lane;
         uint32_t id = 0;
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(NRC_WARPS * 32) k_nrc_train(TrainArgs a) {
                     const float m = (yr[0] + yr[1] + yr[2]) * (1.0f / 3.0f);
                     const float den = m * m + 0.01f;
                     const float e0 = yr[0] - tg.x, e1 = yr[1] - tg.y, e2 = yr[2] - tg.z;
-                    loss_acc += (e0 * e0 + e1 * e1 + e2 * e2) / den * inv_n;
+                    loss_acc += (double)((e0 * e0 + e1 * e1 + e2 * e2) / den * inv_n);
                     yr[0] = 2.0f * e0 / den * inv_n;
                     yr[1] = 2.0f * e1 / den * inv_n;
                     yr[2] = 2.0f * e2 / den * inv_n;
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(NRC_WARPS * 32) k_nrc_train(TrainArgs a) {
         }
     }
     for (int o = 16; o; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-    if (lane == 0 && loss_acc != 0.0f) atomicAdd(a.loss, loss_acc);
+    if (lane == 0 && loss_acc != 0.0) atomicAdd(a.loss, loss_acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -835,7 +836,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_train_tc(TrainArgs a) {
                    wt_s = (uint32_t)__cvta_generic_to_shared(WTc);
     uint32_t phase = 0;
     bool failed = false;
-    float loss_acc = 0.0f;
+    double loss_acc = 0.0;
     // one MMA group (n_k K16 steps into this group's columns), then the wait
     auto mma_round = [&](uint32_t b_base, uint32_t nn, int n_k) {
         if (t == 0) {
@@ -924,7 +925,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_train_tc(TrainArgs a) {
                     const float m = (y0 + y1 + y2) * (1.0f / 3.0f);
                     const float den = m * m + 0.01f;
                     const float e0 = y0 - tg.x, e1 = y1 - tg.y, e2 = y2 - tg.z;
-                    loss_acc += (e0 * e0 + e1 * e1 + e2 * e2) / den * inv_n;
+                    loss_acc += (double)((e0 * e0 + e1 * e1 + e2 * e2) / den * inv_n);
                     d0 = 2.0f * e0 / den * inv_n;
                     d1 = 2.0f * e1 / den * inv_n;
                     d2 = 2.0f * e2 / den * inv_n;
@@ -989,7 +990,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_nrc_train_tc(TrainArgs a) {
         group_sync(grp);
     }
     for (int o = 16; o; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-    if (lane == 0 && loss_acc != 0.0f) atomicAdd(a.loss, loss_acc);
+    if (lane == 0 && loss_acc != 0.0) atomicAdd(a.loss, loss_acc);
     if (failed && t == 0) mbar_wait(bar, phase, TC_WAIT);  // the MMAs in flight, before their memory is freed
     tc_fence_before();
     __syncthreads();
@@ -1175,7 +1176,7 @@ struct Nrc {
     __half2 *table = nullptr;
     float *w_master = nullptr, *w_m = nullptr, *w_v = nullptr, *w_grad = nullptr;
     __nv_bfloat16 *wpack = nullptr;
-    float *loss = nullptr;
+    double *loss = nullptr;
     uint32_t *err = nullptr;  // error word of the host-array entry points
     DevBufPtr act;  // training activations
     size_t act_rows = 0;
@@ -1304,8 +1305,8 @@ vrg_status nrc_create(Context *ctx, const vrg_nrc_desc *d, Nrc **out) {
     N->w_v = (float *)(B + o_w2);
     N->w_grad = (float *)(B + o_wg);
     N->wpack = (__nv_bfloat16 *)(B + o_wp);
-    N->loss = (float *)(B + o_ls);
-    N->err = (uint32_t *)(B + o_ls + 4);
+    N->loss = (double *)(B + o_ls);
+    N->err = (uint32_t *)(B + o_ls + 8);
     VRG_CUDA_TRY(cudaMemsetAsync(B, 0, o, s));
     k_init_table<<<(uint32_t)((te + 255) / 256), 256, 0, s>>>(N->t_master, N->table, te, d->seed ^ 0x7ab1eull);
     // He-uniform hidden layers, Xavier-uniform output layer (rows 0..2)
@@ -1550,24 +1551,24 @@ vrg_status nrc_train_host(Nrc *N, uint32_t n, const float *pos, const float *nrm
     float4 *dp = (float4 *)b->ptr, *dd = dp + n, *dn = dd + n, *dt = dn + n;
     const float *src[4] = {pos, dir, nrm, target};
     VRG_TRY(stage_rows(s, n, src, 4, (float *)(dt + n), dp));
-    VRG_CUDA_TRY(cudaMemsetAsync(N->loss, 0, 8, s));  // loss and error word
+    VRG_CUDA_TRY(cudaMemsetAsync(N->loss, 0, 12, s));  // loss and error word
     if (N->pred_cap < n) {
         VRG_TRY(cache_alloc(N, s, (size_t)n * 16, false, N->pred_buf));
         N->pred_cap = n;
     }
     N->pred_n = n;
     VRG_TRY(nrc_train(N, s, n, nullptr, nullptr, dp, dd, dn, dt, update != 0, nullptr, (float4 *)N->pred_buf->ptr));
-    uint32_t res[2] = {0, 0};  // the loss's bits, the error word
-    VRG_CUDA_TRY(cudaMemcpyAsync(res, N->loss, 8, cudaMemcpyDeviceToHost, s));
+    uint32_t res[3] = {0, 0, 0};  // the loss's bits, the error word
+    VRG_CUDA_TRY(cudaMemcpyAsync(res, N->loss, 12, cudaMemcpyDeviceToHost, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
-    float l;
-    memcpy(&l, &res[0], 4);
-    const uint32_t err = res[1];
+    double l;
+    memcpy(&l, &res[0], 8);
+    const uint32_t err = res[2];
     if (err) {
         set_error("radiance cache kernel error flags 0x%x", err);
         return VRG_ERR_OVERFLOW;
     }
-    if (loss_out) *loss_out = l;
+    if (loss_out) *loss_out = (float)l;
     return VRG_OK;
 }
 
