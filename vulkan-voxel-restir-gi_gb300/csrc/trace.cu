@@ -13,9 +13,9 @@
 // Work distribution: the closest hit and the any-hit walk are persistent
 // warps in which each lane takes a new ray from the bounce's queue when its
 // walk ends; rays that continue, and light-pdf jobs, are compacted into the
-// next queues with one warp ballot + one atomic per warp.  State per pixel
-// stays in SoA float4 arrays; the per-bounce record (E, w=pdf/q) (R, q) feeds
-// the backward radiance recurrence of the resolve kernel.
+// next queues with one warp ballot + one atomic per warp.  A path's ray and its
+// per-bounce record (E, w=pdf/q) (R, q), which feeds the backward radiance
+// recurrence of the resolve kernel, are 32-byte entries.
 #include <cstring>
 #include <mutex>
 

@@ -281,9 +281,12 @@ struct InstDev {
 // transform applied to the node's min and max) and e = v111 - v000:
 //   0 (v000.x + v111.x L R, the same of y L R)  1 (the same of z L R, |e|^2 L R)
 //   2 (power L R, ref L R)  3..5 per axis (v000 L R, v111 L R)
-// A walk reads 0..2 and the axis of its normal: four 16-byte loads for both
-// children's importance, against ten 8-byte loads of two 40-byte nodes, and
-// packed arithmetic (f32x2) for the pair.  A ref >= 0 is an inner node; a leaf
+// A walk reads 0 and 1 in one 32-byte load, 2, and the axis of its normal for
+// both children's importance, against ten 8-byte loads of two 40-byte nodes, with
+// packed arithmetic (f32x2) for the pair.  (The tables' share of the L1 counts as
+// much as the loads: 128 bytes a pair, read by two 32-byte loads, took the 1080p
+// frame in flight from 863 to 878 us; 64 bytes, boxes only with the sums worked
+// out on the way, to 869, though 3840x2160 went from 4886 to 4860.)  A ref >= 0 is an inner node; a leaf
 // is ~instance in the top level, ~(BLAS node) below.  A top-level leaf's own
 // slot holds its instance's BLAS root as L.  light_par: parent << 1 | (is the
 // right child), INVALID at the top; a BLAS root's parent is its top-level

@@ -337,8 +337,8 @@ struct Renderer {
     CacheSet cs[SETS];
     int last_cache_set = -1;              // the set of the last cache frame (its targets)
     vrg_tuning tune{};                    // launch configuration (0 fields = defaults)
-    // per reservoir-ring slot: a 3-D tensor map (4*W floats x H rows x 5
-    // planes) for the TMA-staged spatial pass of a single view
+    // per reservoir-ring slot: a 3-D tensor map (8*W floats x H rows x 2
+    // pairs) for the TMA-staged spatial pass of a single view
     CUtensorMap res_map[8];
     bool res_map_ok = false;
 };
