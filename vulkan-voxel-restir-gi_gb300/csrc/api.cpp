@@ -976,17 +976,30 @@ static vrg_status ensure_ring(vrg_renderer *r, uint32_t slots) {
 }
 
 // the renderer's launch configuration with defaults resolved
-static vrg_tuning effective_tuning(const vrg_renderer *r) {
+// The launch configuration of a frame: the renderer's tuning, where it leaves a
+// field open (0) the default.  flight: the frame runs beside others (no stats,
+// capture, graph or cache).  Its persistent grids then leave part of each SM to
+// the stages of the other frames instead of queueing behind them, its walks
+// refill empty warps only, and its per-pixel passes run in smaller CTAs: in
+// flight at 1080p 800 -> 781 us, with 8 bounces 1692 -> 1649, at 957x541 265 ->
+// 259, 16 views 3159 -> 3057, 3840x2160 4673 -> 4645.  A frame alone fills the
+// SMs itself (64x64 with the smaller grids 106 -> 109, a replayed graph 854 ->
+// 868), and a cache frame's training chain loses more than it gains (1280 ->
+// 1285).
+static vrg_tuning effective_tuning(const vrg_renderer *r, bool flight) {
     int occ[3], sms = 1;
     bounce_occupancy(r->n_views != 0, occ, &sms);
     const vrg_tuning &t = r->tune;
+    auto grid = [&](uint32_t asked, int full, int beside) {
+        return asked ? std::min<uint32_t>(asked, full) : (uint32_t)(flight ? std::min(beside, full) : full);
+    };
     vrg_tuning e{};
-    e.trace_blocks_per_sm = t.trace_blocks_per_sm ? std::min<uint32_t>(t.trace_blocks_per_sm, occ[0]) : occ[0];
-    e.shade_blocks_per_sm = t.shade_blocks_per_sm ? std::min<uint32_t>(t.shade_blocks_per_sm, occ[1]) : occ[1];
-    e.anyhit_blocks_per_sm = t.anyhit_blocks_per_sm ? std::min<uint32_t>(t.anyhit_blocks_per_sm, occ[2]) : occ[2];
-    e.trace_refill = t.trace_refill ? t.trace_refill : 8;
+    e.trace_blocks_per_sm = grid(t.trace_blocks_per_sm, occ[0], 6);
+    e.shade_blocks_per_sm = grid(t.shade_blocks_per_sm, occ[1], 7);
+    e.anyhit_blocks_per_sm = grid(t.anyhit_blocks_per_sm, occ[2], 6);
+    e.trace_refill = t.trace_refill ? t.trace_refill : flight ? 32 : 8;
     e.anyhit_refill = t.anyhit_refill ? t.anyhit_refill : 8;
-    e.stream_block = t.stream_block ? t.stream_block : 256;
+    e.stream_block = t.stream_block ? t.stream_block : flight ? 128 : 256;
     // Per-thread loads unless TMA-staged tiles are asked for.  Staged tiles
     // make the spatial pass itself faster (0.113 against 0.117-0.119 ms per
     // 1080p frame), but the frame in flight slower (1.110-1.126 against
@@ -996,10 +1009,10 @@ static vrg_tuning effective_tuning(const vrg_renderer *r) {
     return e;
 }
 
-static void apply_tuning(const vrg_renderer *r, FrameArgs &a) {
+static void apply_tuning(const vrg_renderer *r, bool flight, FrameArgs &a) {
     int occ[3], sms = 1;
     bounce_occupancy(r->n_views != 0, occ, &sms);
-    const vrg_tuning e = effective_tuning(r);
+    const vrg_tuning e = effective_tuning(r, flight);
     a.refill_trace = e.trace_refill;
     a.refill_any = e.anyhit_refill;
     a.grid_trace = (uint32_t)sms * e.trace_blocks_per_sm;
@@ -1024,7 +1037,8 @@ static void set_tiles(ViewDev &d, uint32_t first) {
     d.tile_end = first + view_tiles(d.W, d.H);
 }
 
-static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool want_radiance, FrameArgs &a) {
+static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool want_radiance, bool flight,
+                              FrameArgs &a) {
     if (pr->num_bounces == 0 || pr->spatial_iterations > 64 || pr->nee_type > 2 || pr->mode > 1) {
         set_error("invalid render parameters");
         return VRG_ERR_INVALID_ARGUMENT;
@@ -1181,7 +1195,7 @@ static vrg_status frame_setup(vrg_renderer *r, const vrg_render_params *pr, bool
     a.c_L = r->c_L;
     a.c_q = r->c_q;
     a.c_hit = r->c_hit;
-    apply_tuning(r, a);
+    apply_tuning(r, flight && !capture && !cache, a);
     r->last_ring = ring;
     return VRG_OK;
 }
@@ -1371,7 +1385,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool pipelin
     // the TMA-staged spatial pass when the tuning asks for it and the ring
     // slot has its tensor map
     const CUtensorMap *res_map = nullptr;
-    if (effective_tuning(r).spatial_staging == 1 && r->res_map_ok && !in_graph && r->ring_slots) {
+    if (effective_tuning(r, false).spatial_staging == 1 && r->res_map_ok && !in_graph && r->ring_slots) {
         const size_t slot = (size_t)(a.res - r->res) / ring_stride(r->P);
         if (slot < r->ring_slots) res_map = &r->res_map[slot];
     }
@@ -1479,7 +1493,7 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
     VRG_TRY(scene_commit(scene));
     const size_t P = (size_t)r->P;
     FrameArgs a;
-    VRG_TRY(frame_setup(r, pr, out && out->radiance, a));
+    VRG_TRY(frame_setup(r, pr, out && out->radiance, stats == nullptr, a));
     if (a.cache && !scene->h_geo_tl.empty())
         nrc_set_bounds(r->cache, scene->h_geo_tl[0].min, scene->h_geo_tl[0].max);
     a.v0.sc = frame_scene(scene);
@@ -1575,7 +1589,7 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
     if (outs)
         for (uint32_t v = 0; v < n_views; v++) want_rad |= outs[v].radiance != nullptr;
     FrameArgs a;
-    VRG_TRY(frame_setup(r, pr, want_rad, a));
+    VRG_TRY(frame_setup(r, pr, want_rad, !graph && !stats, a));
     if (a.cache) {  // the cache spans every view's scene
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (uint32_t v = 0; v < n_views; v++) {
@@ -1782,7 +1796,7 @@ VRG_API vrg_status vrg_renderer_set_tuning(vrg_renderer *r, const vrg_tuning *t)
 
 VRG_API vrg_status vrg_renderer_get_tuning(vrg_renderer *r, vrg_tuning *t) {
     if (!r || !t) return VRG_ERR_INVALID_ARGUMENT;
-    *t = effective_tuning(r);
+    *t = effective_tuning(r, false);
     return VRG_OK;
 }
 
@@ -1853,7 +1867,7 @@ VRG_API vrg_status vrg_renderer_autotune(vrg_renderer *r, vrg_scene *scene, cons
         {&vrg_tuning::anyhit_blocks_per_sm, bpsm_candidates(occ[2])},
         {&vrg_tuning::stream_block, {64, 128, 256}},
     };
-    vrg_tuning cur = effective_tuning(r);
+    vrg_tuning cur = effective_tuning(r, !(params->flags & (VRG_RENDER_CAPTURE | VRG_RENDER_CACHE)));
     float cur_ms = 0.0f;
     vrg_status st = measure(cur, &cur_ms);
     for (int pass = 0; pass < 2 && st == VRG_OK; pass++) {
