@@ -213,14 +213,17 @@ VRG_API vrg_status vrg_material_table_set(vrg_context *ctx, const vrg_material *
         set_error("material table changed with uploads pending");
         return VRG_ERR_STATE;
     }
-    ctx->mats.assign(mats, mats + n);
+    // (the host's table and the device's change together: the device's second
+    // part, lambert_of, is found by the host's size)
+    std::vector<vrg_material> table(mats, mats + n);
+    DevBufPtr b;
+    VRG_TRY(upload_materials(ctx, table, b));
+    ctx->mats.swap(table);
+    ctx->d_mats = b;
     ctx->n_types = n / 6;
     ctx->d_atlas.reset();  // an atlas belongs to one table: set it again after a new table
     ctx->atlas_w = ctx->atlas_h = 0;
     ctx->d_srgb = nullptr;
-    DevBufPtr b;
-    VRG_TRY(upload_materials(ctx, ctx->mats, b));
-    ctx->d_mats = b;
     return VRG_OK;
 }
 
