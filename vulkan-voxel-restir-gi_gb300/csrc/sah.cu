@@ -23,7 +23,6 @@
 // of the serial two-pointer partition.
 #include <algorithm>
 #include <cfloat>
-#include <mutex>
 
 #include "vrg_internal.h"
 
@@ -698,14 +697,13 @@ __global__ void k_power_up(const SahTree *trees, vrg_bvh_node *nodes, uint32_t *
 
 }  // namespace
 
-// shared memory of k_sah_tree beyond the default 48 KB, asked for once
+// Shared memory of k_sah_tree beyond the default 48 KB.  The attribute belongs
+// to the context current at the call, so it is asked for before every build: a
+// process may build on several devices, reset one, or build under contexts of
+// its own (vrg_build_tl_bvh_noalloc).
 static vrg_status tree_smem_init() {
-    static std::once_flag once;
-    static cudaError_t err = cudaSuccess;
-    std::call_once(once, [] {
-        err = cudaFuncSetAttribute(k_sah_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem(TREE_MAX));
-    });
-    VRG_CUDA_TRY(err);
+    VRG_CUDA_TRY(cudaFuncSetAttribute(k_sah_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)tree_smem(TREE_MAX)));
     return VRG_OK;
 }
 
