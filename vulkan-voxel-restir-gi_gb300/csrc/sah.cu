@@ -149,8 +149,8 @@ __device__ __forceinline__ void best_plane(const Bins &B, int d, float &cost, in
     float l[3], h[3], rl[3], rh[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        l[k] = o2f(B.lo[bi][k]);
-        h[k] = o2f(B.hi[bi][k]);
+        l[k] = fminf(INFINITY, o2f(B.lo[bi][k]));  // (a bin whose bound is NaN has none)
+        h[k] = fmaxf(-INFINITY, o2f(B.hi[bi][k]));
         // the suffix past this lane: starts from the next lane's bin
         rl[k] = __shfl_down_sync(0xffffffffu, l[k], 1);
         rh[k] = __shfl_down_sync(0xffffffffu, h[k], 1);
@@ -261,7 +261,9 @@ __device__ uint32_t warp_partition(const float4 *cen, uint32_t *perm, uint32_t c
 // per (axis, prim) for the planes.  The planes between two occupied bins share
 // a cost, so the first minimum is at a prim's own bin (bin 0 always holds the
 // lowest centroid); each such plane takes the minima and maxima over the prims
-// on its sides straight from their boxes, without the 96 bins.
+// on its sides straight from their boxes, without the 96 bins.  Returns 0, with
+// nothing changed, for a node with a value that is not finite (raw prims may
+// hold one): its bounds and bins are those of the general path.
 constexpr uint32_t SMALL_NODE = 10;  // three axes' prims in a warp
 __device__ uint32_t warp_split_small(const Prims &Q, uint32_t *perm, uint32_t c, Bins &B, float nlo[3], float nhi[3]) {
     const uint32_t lane = threadIdx.x & 31;
@@ -271,6 +273,10 @@ __device__ uint32_t warp_split_small(const Prims &Q, uint32_t *perm, uint32_t c,
     float4 m = a;
     if (own) { a = Q.lo[p]; b = Q.hi[p]; m = Q.cen[p]; }
     const float lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z}, cc[3] = {m.x, m.y, m.z};
+    float zero = 0.0f;  // NaN once a value is not finite
+#pragma unroll
+    for (int k = 0; k < 3; k++) zero = __fmaf_rn(lo[k], 0.0f, __fmaf_rn(hi[k], 0.0f, __fmaf_rn(cc[k], 0.0f, zero)));
+    if (__any_sync(0xffffffffu, own && zero != 0.0f)) return 0;
     float clo[3], chi[3];
     uint32_t bins = 0;
 #pragma unroll
@@ -344,7 +350,10 @@ __device__ uint32_t warp_split_small(const Prims &Q, uint32_t *perm, uint32_t c,
 // build.rs:36-43) and the left child's count, the slice partitioned.  Bounds
 // and bins are order-independent minima and maxima.
 __device__ uint32_t warp_split(const Prims &Q, uint32_t *perm, uint32_t c, Bins &B, float nlo[3], float nhi[3]) {
-    if (c <= SMALL_NODE) return warp_split_small(Q, perm, c, B, nlo, nhi);
+    if (c <= SMALL_NODE) {
+        const uint32_t n_left = warp_split_small(Q, perm, c, B, nlo, nhi);
+        if (n_left) return n_left;
+    }
     const int lane = threadIdx.x & 31;
     float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     for (int k = 0; k < 3; k++) { nlo[k] = INFINITY; nhi[k] = -INFINITY; }
