@@ -79,7 +79,7 @@ void ctx_release(Context *c) {
     c->d_atlas.reset();
     cudaStreamSynchronize(c->stream);
     if (c->pool) cudaMemPoolDestroy(c->pool);
-    if (c->h_stage) cudaFreeHost(c->h_stage);
+    if (c->stage.ptr) cudaFreeHost(c->stage.ptr);
     cudaStreamDestroy(c->stream);
     delete static_cast<vrg_context *>(c);
 }

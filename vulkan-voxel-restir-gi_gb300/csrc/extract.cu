@@ -301,28 +301,23 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     const size_t in_bytes = (size_t)nc * CHUNK_BYTES, cnt_bytes = 16 * (size_t)nc;
     const size_t plan_bytes = nc * (16 + sizeof(ChunkTrees)), out_bytes = 2 * nc * sizeof(RootSummary) + 16;
     const size_t stage_bytes = in_bytes + cnt_bytes + plan_bytes + out_bytes;
-    if (ctx->h_stage_bytes < stage_bytes) {
-        if (ctx->h_stage) {
-            cudaStreamSynchronize(s);
-            cudaFreeHost(ctx->h_stage);
+    struct Pinned {
+        cudaStream_t s;
+        uint8_t *alloc(size_t n) {
+            void *p = nullptr;
+            if (cudaMallocHost(&p, n) == cudaSuccess) return (uint8_t *)p;
+            cudaGetLastError();
+            return nullptr;
         }
-        ctx->h_stage = nullptr;
-        ctx->h_stage_bytes = 0;
-        VRG_CUDA_TRY(cudaMallocHost(&ctx->h_stage, stage_bytes));
-        ctx->h_stage_bytes = stage_bytes;
+        void release(uint8_t *p) { cudaFreeHost(p); }
+        void wait() { cudaStreamSynchronize(s); }
+    };
+    StagingLease<Pinned> lease(ctx->stage, Pinned{s}, Context::STAGE_KEEP);
+    uint8_t *h_in = lease.take(stage_bytes);
+    if (!h_in) {
+        set_error("%zu bytes of page-locked staging are not to be had", stage_bytes);
+        return VRG_ERR_CUDA;
     }
-    // (given back after a flush of many chunks, also when it fails)
-    struct StageGuard {
-        Context *c;
-        ~StageGuard() {
-            if (c->h_stage_bytes <= Context::STAGE_KEEP) return;
-            cudaStreamSynchronize(c->stream);
-            cudaFreeHost(c->h_stage);
-            c->h_stage = nullptr;
-            c->h_stage_bytes = 0;
-        }
-    } guard{ctx};
-    uint8_t *h_in = ctx->h_stage;
     for (uint32_t c = 0; c < nc; c++) {
         memcpy(h_in + (size_t)c * CHUNK_BYTES, batch[c]->blocks.data(), VRG_CHUNK_BLOCKS);
         memcpy(h_in + (size_t)c * CHUNK_BYTES + VRG_CHUNK_BLOCKS, batch[c]->slabs.data(), 6 * 1024);
@@ -452,6 +447,7 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     const RootSummary *roots = (const RootSummary *)(h_in + in_bytes + cnt_bytes + plan_bytes);
     VRG_CUDA_TRY(cudaMemcpyAsync((void *)roots, d_roots, out_bytes, cudaMemcpyDeviceToHost, s));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    lease.settled();
     uint32_t lv_dev;
     memcpy(&lv_dev, roots + 2 * (size_t)nc, 4);
     levels = std::max(levels, lv_dev);

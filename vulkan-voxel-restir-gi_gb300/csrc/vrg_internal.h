@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/vrg.h"
+#include "staging.h"
 #include "vrg_device.cuh"
 #include "vrg_frame.cuh"
 
@@ -141,8 +142,7 @@ struct Context {
     cudaMemPool_t pool = nullptr;        // dev_alloc(Context *)
     // page-locked staging of a flush (guarded by mu), kept up to STAGE_KEEP bytes
     static constexpr size_t STAGE_KEEP = 16u << 20;
-    uint8_t *h_stage = nullptr;
-    size_t h_stage_bytes = 0;
+    Staging stage;
     // references: the handle, and every object, scene, renderer and cache made
     // from it (as the reference's Arc-shared queues and allocators): the
     // context, its stream and its buffers are freed when the last one is
