@@ -312,6 +312,7 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
         void release(uint8_t *p) { cudaFreeHost(p); }
         void wait() { cudaStreamSynchronize(s); }
     };
+    std::vector<SahTree> trees;  // (copied from here until the last synchronization: outlives the lease)
     StagingLease<Pinned> lease(ctx->stage, Pinned{s}, Context::STAGE_KEEP);
     uint8_t *h_in = lease.take(stage_bytes);
     if (!h_in) {
@@ -387,7 +388,6 @@ vrg_status extract_and_build(Context *ctx, std::vector<Object *> &batch) {
     // light trees (build_bl_bvh over light triangles).
     uint32_t *offs = (uint32_t *)(h_in + in_bytes + cnt_bytes);
     ChunkTrees *ct = (ChunkTrees *)(offs + 4 * (size_t)nc);
-    std::vector<SahTree> trees;
     uint64_t node_cursor = 0;
     uint32_t max_light_nodes = 0;
     for (int k = 0; k < 2; k++)

@@ -716,7 +716,7 @@ static vrg_status tree_smem_init() {
     return VRG_OK;
 }
 
-vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t total_prims, uint32_t total_nodes,
+vrg_status sah_build(Context *ctx, std::vector<SahTree> &trees, uint32_t total_prims, uint32_t total_nodes,
                      const SahInputs &in, const SahOutputs &out, uint32_t *levels, uint32_t *levels_dev) {
     cudaStream_t s = ctx->stream;
     if (trees.empty() || total_prims == 0) {
@@ -733,10 +733,9 @@ vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t t
     // a CTA each.  A CTA's shared memory is its launch's largest tree's, so
     // more trees than SMs go in launches by size; up to one per SM they go in
     // one, since launches of a few CTAs each would only follow one another.
-    std::vector<SahTree> by_size(trees);
-    std::stable_sort(by_size.begin(), by_size.end(), [](const SahTree &a, const SahTree &b) { return a.n > b.n; });
+    std::stable_sort(trees.begin(), trees.end(), [](const SahTree &a, const SahTree &b) { return a.n > b.n; });
     uint32_t n_large = 0;
-    while (n_large < nt && by_size[n_large].n > TREE_MAX) n_large++;
+    while (n_large < nt && trees[n_large].n > TREE_MAX) n_large++;
     // scratch: trees, counters, arrival flags; the level lists of large trees
     const size_t q_cap = n_large ? std::max<size_t>(n_large, (size_t)total_prims / 3 + 1) : 0;
     const size_t bytes = nt * sizeof(SahTree) + 2 * q_cap * sizeof(Item) + 64 + (size_t)total_nodes * 4;
@@ -748,26 +747,26 @@ vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t t
     Item *q1 = (Item *)p; p += q_cap * sizeof(Item);
     uint32_t *cnt = (uint32_t *)p; p += 64;
     uint32_t *arrive = (uint32_t *)p;
-    VRG_CUDA_TRY(cudaMemcpyAsync(d_trees, by_size.data(), nt * sizeof(SahTree), cudaMemcpyHostToDevice, s));
+    VRG_CUDA_TRY(cudaMemcpyAsync(d_trees, trees.data(), nt * sizeof(SahTree), cudaMemcpyHostToDevice, s));
     if (!levels_dev) VRG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 64, s));
     uint32_t *lv_dev = levels_dev ? levels_dev : cnt + 8;
-    for (uint32_t a = n_large; a < nt && by_size[a].n;) {
+    for (uint32_t a = n_large; a < nt && trees[a].n;) {
         uint32_t b = a;
-        const uint32_t n = by_size[a].n;
-        while (b < nt && by_size[b].n && (nt - n_large <= TREE_ONE_WAVE || 2 * by_size[b].n > n)) b++;
+        const uint32_t n = trees[a].n;
+        while (b < nt && trees[b].n && (nt - n_large <= TREE_ONE_WAVE || 2 * trees[b].n > n)) b++;
         k_sah_tree<<<b - a, TREE_THREADS, tree_smem(n), s>>>(d_trees + a, in, out, arrive, lv_dev);
         VRG_CUDA_TRY(cudaGetLastError());
         a = b;
     }
     uint32_t lv = 0, h_cnt = 0;
     if (n_large) {
-        const uint32_t max_n = by_size[0].n;
+        const uint32_t max_n = trees[0].n;
         std::vector<Item> roots;
-        for (uint32_t t = 0; t < n_large; t++) roots.push_back(Item{t, 0, 1, 0, by_size[t].n, INVALID});
+        for (uint32_t t = 0; t < n_large; t++) roots.push_back(Item{t, 0, 1, 0, trees[t].n, INVALID});
         uint32_t n_cur = n_large;
         // (the flags of the CTAs' trees are theirs: all before them is zeroed here)
         for (uint32_t t = 0; t < n_large; t++)
-            VRG_CUDA_TRY(cudaMemsetAsync(arrive + by_size[t].node_off, 0, (2 * (size_t)by_size[t].n - 1) * 4, s));
+            VRG_CUDA_TRY(cudaMemsetAsync(arrive + trees[t].node_off, 0, (2 * (size_t)trees[t].n - 1) * 4, s));
         VRG_CUDA_TRY(cudaMemcpyAsync(q0, roots.data(), roots.size() * sizeof(Item), cudaMemcpyHostToDevice, s));
         VRG_CUDA_TRY(cudaMemcpyAsync(cnt, &n_cur, 4, cudaMemcpyHostToDevice, s));
         k_perm_init<<<dim3(std::min(1024u, (max_n + 255) / 256), n_large), 256, 0, s>>>(d_trees, out.perm);

@@ -592,6 +592,7 @@ struct CommitPrep {
     std::vector<float> tl_in;        // [prims][10]: lo3 hi3 off3 power
     std::vector<uint32_t> tl_ids;
     std::vector<InstBuild> gb, lb;
+    std::vector<InstDev> idev;       // (as gb and lb: copied from here until the commit's last wait)
     uint64_t geo_recs = 0, light_recs = 0, tri_recs = 0, n_geo_wide = 0, n_light_nodes_all = 0;
     uint64_t blk_cursor = 0;
     uint32_t max_levels = 0;
@@ -776,6 +777,9 @@ vrg_status commit_top_levels(Context *ctx, std::vector<CommitPrep> &cps, uint32_
     }
     *tl_levels = 0;
     std::vector<vrg_bvh_node> h_nodes(n_nodes + 1, vrg_bvh_node{});  // (the last: the trees' levels)
+    std::vector<float> tin;  // (copied from here until the wait below, as the trees)
+    std::vector<uint32_t> tid;
+    std::vector<SahTree> trees;
     if (n_prims) {
         auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
         uint64_t o = 0;
@@ -791,11 +795,8 @@ vrg_status commit_top_levels(Context *ctx, std::vector<CommitPrep> &cps, uint32_
         DevBufPtr sb;
         VRG_TRY(dev_alloc(ctx, o, sb));
         uint8_t *S = (uint8_t *)sb->ptr;
-        std::vector<float> tin;
-        std::vector<uint32_t> tid;
         tin.reserve((size_t)n_prims * 10);
         tid.reserve(n_prims);
-        std::vector<SahTree> trees;
         for (auto &cp : cps) {
             tin.insert(tin.end(), cp.tl_in.begin(), cp.tl_in.end());
             tid.insert(tid.end(), cp.tl_ids.begin(), cp.tl_ids.end());
@@ -852,7 +853,8 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
     const uint32_t ni = cp.ni;
     uint8_t *B = cp.B;
     // instance table (prim2node, scene.rs:282-287)
-    std::vector<InstDev> idev(ni);
+    std::vector<InstDev> &idev = cp.idev;
+    idev.resize(ni);
     for (uint32_t i = 0; i < ni; i++) {
         const Object *ob = sc->inst_objs[i];
         const bool xf_light = !sc->inst_tonly[i] && ob->sum.n_light;  // (its light nodes carry the transform)
@@ -942,8 +944,10 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
 
 // all scenes' lamp-block trees in one SAH build
 // (their number of lamps is known from the objects, so nothing is read back but
-// the tree levels, which arrive at the commit's end: *levels)
-vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, uint32_t *levels, uint32_t *levels_copy) {
+// the tree levels, which arrive at the commit's end: *levels; the trees are
+// copied from where they are until then)
+vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, std::vector<SahTree> &trees, uint32_t *levels,
+                        uint32_t *levels_copy) {
     cudaStream_t s = ctx->stream;
     uint64_t L = 0;
     for (auto &cp : cps) {
@@ -1001,7 +1005,6 @@ vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, uint32_t *le
         D.lamp_rec = lamp;
         D.lamp_table = table;
     }
-    std::vector<SahTree> trees;
     for (auto &cp : cps)
         if (cp.n_lamps) trees.push_back(SahTree{cp.n_lamps, (uint32_t)cp.lamp_off, 2 * (uint32_t)cp.lamp_off, 0});
     SahInputs in{(const float4 *)(S + o_lo), (const float4 *)(S + o_hi), (const float4 *)(S + o_cen),
@@ -1065,7 +1068,8 @@ vrg_status scene_commit_many(Scene *const *scs, uint32_t n) {
     VRG_TRY(commit_top_levels(ctx, cps, &tl_levels));
     for (auto &cp : cps) VRG_TRY(commit_layouts(s, cp, (const vrg_bvh_node *)(cp.B + cp.o_tln)));
     uint32_t lamp_levels = 0, lamp_levels_dev = 0;
-    VRG_TRY(commit_lamps(ctx, cps, &lamp_levels, &lamp_levels_dev));
+    std::vector<SahTree> lamp_trees;
+    VRG_TRY(commit_lamps(ctx, cps, lamp_trees, &lamp_levels, &lamp_levels_dev));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
     lamp_levels = std::max(lamp_levels, lamp_levels_dev);
     for (auto &cp : cps) {

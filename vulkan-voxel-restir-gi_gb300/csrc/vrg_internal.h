@@ -79,11 +79,13 @@ struct SahOutputs {
     uint32_t *leaf_prim;  // per node: local prim index of a leaf, INVALID for internal nodes
 };
 // Builds every tree on the context's stream; trees with n == 0 are skipped.
+// Sorts the trees, largest first, and copies them to the device from where they
+// are: the caller keeps them until it has waited for the stream.
 // *levels receives the number of level passes (an upper bound on depth - 2).
 // With levels_dev (a zeroed device word) the call does not synchronize for it:
 // the bound is then the larger of *levels and that word after the build.
-vrg_status sah_build(Context *ctx, const std::vector<SahTree> &trees, uint32_t total_prims,
-                     uint32_t total_nodes, const SahInputs &in, const SahOutputs &out, uint32_t *levels, uint32_t *levels_dev = nullptr);
+vrg_status sah_build(Context *ctx, std::vector<SahTree> &trees, uint32_t total_prims, uint32_t total_nodes,
+                     const SahInputs &in, const SahOutputs &out, uint32_t *levels, uint32_t *levels_dev = nullptr);
 
 // ---- chunk extraction ---------------------------------------------------
 struct ChunkSummary {      // per chunk, copied to the host after a flush
