@@ -943,11 +943,11 @@ vrg_status commit_layouts(cudaStream_t s, CommitPrep &cp, const vrg_bvh_node *d_
 }
 
 // all scenes' lamp-block trees in one SAH build
-// (their number of lamps is known from the objects, so nothing is read back but
-// the tree levels, which arrive at the commit's end: *levels; the trees are
-// copied from where they are until then)
+// (their number of lamps is known from the objects, so nothing is waited for
+// here: the lamps counted per scene and the trees' levels arrive in `back` at
+// the commit's end, and the trees are copied from where they are until then)
 vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, std::vector<SahTree> &trees, uint32_t *levels,
-                        uint32_t *levels_copy) {
+                        std::vector<uint32_t> &back) {
     cudaStream_t s = ctx->stream;
     uint64_t L = 0;
     for (auto &cp : cps) {
@@ -955,6 +955,7 @@ vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, std::vector<
         L += cp.light_recs;
         cp.dev.lamp_root = EMPTY_ROOT;
     }
+    back.assign(cps.size() + 1, 0);
     if (L == 0) return VRG_OK;
     if (2 * L >= 0x7FFFFFFFull) {
         set_error("too many light triangles in one commit");
@@ -1013,7 +1014,7 @@ vrg_status commit_lamps(Context *ctx, std::vector<CommitPrep> &cps, std::vector<
     uint32_t *leaf = (uint32_t *)(S + o_leaf);
     SahOutputs out{nodes, (uint32_t *)(S + o_perm), leaf};
     VRG_TRY(sah_build(ctx, trees, (uint32_t)L, (uint32_t)(2 * L), in, out, levels, tot + nc));
-    VRG_CUDA_TRY(cudaMemcpyAsync(levels_copy, tot + nc, 4, cudaMemcpyDeviceToHost, s));
+    VRG_CUDA_TRY(cudaMemcpyAsync(back.data(), tot, (size_t)nc * 4 + 4, cudaMemcpyDeviceToHost, s));
     for (auto &cp : cps) {
         if (!cp.n_lamps) continue;
         DevScene &D = cp.dev;
@@ -1067,11 +1068,17 @@ vrg_status scene_commit_many(Scene *const *scs, uint32_t n) {
     uint32_t tl_levels = 0;
     VRG_TRY(commit_top_levels(ctx, cps, &tl_levels));
     for (auto &cp : cps) VRG_TRY(commit_layouts(s, cp, (const vrg_bvh_node *)(cp.B + cp.o_tln)));
-    uint32_t lamp_levels = 0, lamp_levels_dev = 0;
+    uint32_t lamp_levels = 0;
     std::vector<SahTree> lamp_trees;
-    VRG_TRY(commit_lamps(ctx, cps, lamp_trees, &lamp_levels, &lamp_levels_dev));
+    std::vector<uint32_t> lamp_words;
+    VRG_TRY(commit_lamps(ctx, cps, lamp_trees, &lamp_levels, lamp_words));
     VRG_CUDA_TRY(cudaStreamSynchronize(s));
-    lamp_levels = std::max(lamp_levels, lamp_levels_dev);
+    lamp_levels = std::max(lamp_levels, lamp_words.back());
+    for (size_t c = 0; c < cps.size(); c++)
+        if (cps[c].n_lamps != lamp_words[c]) {  // (the chunks' extraction and k_lamp_flags count by one rule)
+            set_error("scene has %u lamps, its objects %u", lamp_words[c], cps[c].n_lamps);
+            return VRG_ERR_STATE;
+        }
     for (auto &cp : cps) {
         // the 4-wide walks push up to 3 refs per 4-wide level (half the binary depth)
         const uint32_t lamp_depth = cp.n_lamps ? 3 * ((lamp_levels + 2 + 1) / 2) + 1 : 0;
