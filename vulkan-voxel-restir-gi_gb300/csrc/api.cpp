@@ -1720,14 +1720,17 @@ VRG_API vrg_status vrg_renderer_state_size(vrg_renderer *r, uint64_t *bytes) {
 }
 
 // The ring slots to (save) or from the saved state's five planes per slot,
-// through at most 2^18 pixels of device scratch at a time.
+// through the bounce records of the renderer's first array set, as many pixels
+// at a time as fit: 80 bytes each of the set's 32 per pixel and bounce, in at
+// least 256 bytes.  The records are between frames here: a frame writes them
+// before it reads them, every frame so far has read them before the library
+// stream gets here, and the callers wait for the stream before they return.
 static vrg_status copy_ring(vrg_renderer *r, uint8_t *host, bool save) {
     cudaStream_t s = r->ctx->stream;
-    const uint32_t P = (uint32_t)r->P, part = std::min<uint32_t>(P, 1u << 18);
-    if (!r->ring_slots) return VRG_OK;
-    DevBufPtr b;
-    VRG_TRY(dev_alloc(r->ctx, (size_t)part * 80, b));
-    float4 *planes = (float4 *)b->ptr;
+    const uint32_t P = (uint32_t)r->P;
+    const size_t room = ((size_t)P * 32 * r->nb_max + 255) & ~(size_t)255;
+    const uint32_t part = (uint32_t)std::min<size_t>(P, room / 80);
+    float4 *planes = r->fs[0].rec;
     for (uint32_t k = 0; k < r->ring_slots; k++) {
         float4 *slot = r->res + k * ring_stride(P);
         uint8_t *hk = host + (size_t)k * 5 * P * 16;
