@@ -385,11 +385,15 @@ typedef struct vrg_tuning {
                                        0 = 2.  The autotuner keeps the value it is given: staged tiles
                                        speed up the spatial pass alone but slow frames in flight, whose
                                        walks beside it lose L1 to the tile's shared memory */
-    uint32_t reserved[1];
+    uint32_t reserved[1];           /* 0, or as vrg_renderer_get_tuning gave it: bit k says that field k,
+                                       in the order above, is left open */
 } vrg_tuning;
 
 VRG_API vrg_status vrg_renderer_set_tuning(vrg_renderer *r, const vrg_tuning *t);
-/* The configuration in effect, defaults resolved to their values. */
+/* The configuration in effect for a frame alone, defaults resolved to their
+ * values, and in reserved[0] which fields are defaults.  Set again, those that
+ * still have the value given here stay open, for frames in flight too; with
+ * reserved[0] = 0 every value that is not 0 holds for all frames. */
 VRG_API vrg_status vrg_renderer_get_tuning(vrg_renderer *r, vrg_tuning *t);
 /* Autotuner: renders frames of (scene, cam, params) under candidate launch
  * configurations, one field at a time over its candidate values (coordinate

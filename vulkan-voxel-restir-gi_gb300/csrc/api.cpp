@@ -978,9 +978,8 @@ static vrg_status ensure_ring(vrg_renderer *r, uint32_t slots) {
     return VRG_OK;
 }
 
-// the renderer's launch configuration with defaults resolved
-// The launch configuration of a frame: the renderer's tuning, where it leaves a
-// field open (0) the default.  flight: the frame runs beside others (no stats,
+// The launch configuration of a frame: the tuning t, where it leaves a field
+// open (0) the default.  flight: the frame runs beside others (no stats,
 // capture, graph or cache).  Its persistent grids then leave part of each SM to
 // the stages of the other frames instead of queueing behind them, its walks
 // refill empty warps only, and its per-pixel passes run in smaller CTAs: in
@@ -989,10 +988,9 @@ static vrg_status ensure_ring(vrg_renderer *r, uint32_t slots) {
 // SMs itself (64x64 with the smaller grids 106 -> 109, a replayed graph 854 ->
 // 868), and a cache frame's training chain loses more than it gains (1280 ->
 // 1285).
-static vrg_tuning effective_tuning(const vrg_renderer *r, bool flight) {
+static vrg_tuning effective_tuning(const vrg_renderer *r, const vrg_tuning &t, bool flight) {
     int occ[3], sms = 1;
     bounce_occupancy(r->n_views != 0, occ, &sms);
-    const vrg_tuning &t = r->tune;
     auto grid = [&](uint32_t asked, int full, int beside) {
         return asked ? std::min<uint32_t>(asked, full) : (uint32_t)(flight ? std::min(beside, full) : full);
     };
@@ -1015,7 +1013,7 @@ static vrg_tuning effective_tuning(const vrg_renderer *r, bool flight) {
 static void apply_tuning(const vrg_renderer *r, bool flight, FrameArgs &a) {
     int occ[3], sms = 1;
     bounce_occupancy(r->n_views != 0, occ, &sms);
-    const vrg_tuning e = effective_tuning(r, flight);
+    const vrg_tuning e = effective_tuning(r, r->tune, flight);
     a.refill_trace = e.trace_refill;
     a.refill_any = e.anyhit_refill;
     a.grid_trace = (uint32_t)sms * e.trace_blocks_per_sm;
@@ -1388,7 +1386,7 @@ static vrg_status frame_launch(vrg_renderer *r, const FrameArgs &a, bool pipelin
     // the TMA-staged spatial pass when the tuning asks for it and the ring
     // slot has its tensor map
     const CUtensorMap *res_map = nullptr;
-    if (effective_tuning(r, false).spatial_staging == 1 && r->res_map_ok && !in_graph && r->ring_slots) {
+    if (effective_tuning(r, r->tune, false).spatial_staging == 1 && r->res_map_ok && !in_graph && r->ring_slots) {
         const size_t slot = (size_t)(a.res - r->res) / ring_stride(r->P);
         if (slot < r->ring_slots) res_map = &r->res_map[slot];
     }
@@ -1785,6 +1783,13 @@ VRG_API vrg_status vrg_renderer_state_load(vrg_renderer *r, const void *src, uin
     return VRG_OK;
 }
 
+// the fields of vrg_tuning, in the order of their bits in its reserved word
+static constexpr uint32_t vrg_tuning::*TUNING[] = {
+    &vrg_tuning::trace_blocks_per_sm,  &vrg_tuning::trace_refill,  &vrg_tuning::shade_blocks_per_sm,
+    &vrg_tuning::anyhit_blocks_per_sm, &vrg_tuning::anyhit_refill, &vrg_tuning::stream_block,
+    &vrg_tuning::spatial_staging};
+static constexpr uint32_t TUNING_FIELDS = sizeof(TUNING) / sizeof(TUNING[0]);
+
 VRG_API vrg_status vrg_renderer_set_tuning(vrg_renderer *r, const vrg_tuning *t) {
     if (!r || !t) return VRG_ERR_INVALID_ARGUMENT;
     if (t->trace_refill > 32 || t->anyhit_refill > 32 || t->trace_blocks_per_sm > 64 ||
@@ -1795,14 +1800,20 @@ VRG_API vrg_status vrg_renderer_set_tuning(vrg_renderer *r, const vrg_tuning *t)
                   "spatial_staging 0/1/2)");
         return VRG_ERR_INVALID_ARGUMENT;
     }
+    // a field that get_tuning gave as open, with the value it gave, is open still
+    const vrg_tuning lone = effective_tuning(r, vrg_tuning{}, false);
     r->tune = *t;
+    for (uint32_t k = 0; k < TUNING_FIELDS; k++)
+        if ((t->reserved[0] >> k & 1u) && r->tune.*TUNING[k] == lone.*TUNING[k]) r->tune.*TUNING[k] = 0;
     memset(r->tune.reserved, 0, sizeof(r->tune.reserved));
     return VRG_OK;
 }
 
 VRG_API vrg_status vrg_renderer_get_tuning(vrg_renderer *r, vrg_tuning *t) {
     if (!r || !t) return VRG_ERR_INVALID_ARGUMENT;
-    *t = effective_tuning(r, false);
+    *t = effective_tuning(r, r->tune, false);
+    for (uint32_t k = 0; k < TUNING_FIELDS; k++)
+        if (r->tune.*TUNING[k] == 0) t->reserved[0] |= 1u << k;
     return VRG_OK;
 }
 
@@ -1873,7 +1884,7 @@ VRG_API vrg_status vrg_renderer_autotune(vrg_renderer *r, vrg_scene *scene, cons
         {&vrg_tuning::anyhit_blocks_per_sm, bpsm_candidates(occ[2])},
         {&vrg_tuning::stream_block, {64, 128, 256}},
     };
-    vrg_tuning cur = effective_tuning(r, !(params->flags & (VRG_RENDER_CAPTURE | VRG_RENDER_CACHE)));
+    vrg_tuning cur = effective_tuning(r, r->tune, !(params->flags & (VRG_RENDER_CAPTURE | VRG_RENDER_CACHE)));
     float cur_ms = 0.0f;
     vrg_status st = measure(cur, &cur_ms);
     for (int pass = 0; pass < 2 && st == VRG_OK; pass++) {
