@@ -369,8 +369,9 @@ VRG_API vrg_status vrg_renderer_state_load(vrg_renderer *r, const void *src, uin
 /* ---- launch configuration and autotuner (no reference counterpart) -----
  * Every field changes only how the frame's work is scheduled, never a result
  * (the tests render the same bits under any configuration).  0 = default:
- * given below for a frame alone; frames in flight (no stats, capture, graph or
- * cache) take 6, 7 and 6 CTAs per SM, trace_refill 32 and stream_block 128. */
+ * given below for a frame alone; frames in flight (no stats, capture, graph,
+ * cache or VRG_OUTPUT_HOST output) take 6, 7 and 6 CTAs per SM, trace_refill 32
+ * and stream_block 128. */
 typedef struct vrg_tuning {
     uint32_t trace_blocks_per_sm;   /* persistent closest-hit grid: CTAs of 128 threads per SM
                                        (default and maximum: full occupancy) */

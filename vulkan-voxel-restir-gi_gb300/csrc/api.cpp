@@ -980,7 +980,7 @@ static vrg_status ensure_ring(vrg_renderer *r, uint32_t slots) {
 
 // The launch configuration of a frame: the tuning t, where it leaves a field
 // open (0) the default.  flight: the frame runs beside others (no stats,
-// capture, graph or cache).  Its persistent grids then leave part of each SM to
+// capture, graph, cache or output that the call waits for).  Its persistent grids then leave part of each SM to
 // the stages of the other frames instead of queueing behind them, its walks
 // refill empty warps only, and its per-pixel passes run in smaller CTAs: in
 // flight at 1080p 800 -> 781 us, with 8 bounces 1692 -> 1649, at 957x541 265 ->
@@ -1494,7 +1494,8 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
     VRG_TRY(scene_commit(scene));
     const size_t P = (size_t)r->P;
     FrameArgs a;
-    VRG_TRY(frame_setup(r, pr, out && out->radiance, stats == nullptr, a));
+    const bool blocks = out && out->host == VRG_OUTPUT_HOST;  // the call waits for the frame: it runs alone
+    VRG_TRY(frame_setup(r, pr, out && out->radiance, !stats && !blocks, a));
     if (a.cache && !scene->h_geo_tl.empty())
         nrc_set_bounds(r->cache, scene->h_geo_tl[0].min, scene->h_geo_tl[0].max);
     a.v0.sc = frame_scene(scene);
@@ -1537,7 +1538,7 @@ VRG_API vrg_status vrg_render(vrg_renderer *r, vrg_scene *scene, const vrg_camer
     }
     VRG_TRY(frame_done(r, a, pr));
     if (stats) return frame_stats(r, a, true, stats);
-    if (out && out->host == VRG_OUTPUT_HOST) VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (blocks) VRG_CUDA_TRY(cudaStreamSynchronize(s));
     return VRG_OK;
 }
 
@@ -1586,11 +1587,14 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
         for (uint32_t v = 0; v < n_views; v++) scs[v] = views[v].scene;
         VRG_TRY(scene_commit_many(scs.data(), n_views));
     }
-    bool want_rad = false;
+    bool want_rad = false, blocks = false;  // blocks: the call waits for the frame, which runs alone
     if (outs)
-        for (uint32_t v = 0; v < n_views; v++) want_rad |= outs[v].radiance != nullptr;
+        for (uint32_t v = 0; v < n_views; v++) {
+            want_rad |= outs[v].radiance != nullptr;
+            blocks |= outs[v].host == VRG_OUTPUT_HOST && (outs[v].bgra8 || outs[v].radiance);
+        }
     FrameArgs a;
-    VRG_TRY(frame_setup(r, pr, want_rad, !graph && !stats, a));
+    VRG_TRY(frame_setup(r, pr, want_rad, !graph && !stats && !blocks, a));
     if (a.cache) {  // the cache spans every view's scene
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (uint32_t v = 0; v < n_views; v++) {
@@ -1677,7 +1681,6 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
         a.timed = stats ? 1u : 0u;
         VRG_TRY(frame_launch(r, a, stats == nullptr));
     }
-    bool host_out = false;
     if (outs) {
         for (uint32_t v = 0; v < n_views; v++) {
             const vrg_frame_output &o = outs[v];
@@ -1685,12 +1688,11 @@ VRG_API vrg_status vrg_render_batched(vrg_renderer *r, const vrg_view *views, ui
             const cudaMemcpyKind k = o.host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
             if (o.bgra8 && a.pack) VRG_CUDA_TRY(cudaMemcpyAsync(o.bgra8, r->bgra + 4 * off, n * 4, k, s));
             if (o.radiance) VRG_CUDA_TRY(cudaMemcpyAsync(o.radiance, r->radiance + 3 * off, n * 12, k, s));
-            host_out |= o.host == VRG_OUTPUT_HOST && (o.bgra8 || o.radiance);
         }
     }
     VRG_TRY(frame_done(r, a, pr));
     if (stats) return frame_stats(r, a, !graph, stats);
-    if (host_out) VRG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (blocks) VRG_CUDA_TRY(cudaStreamSynchronize(s));
     return VRG_OK;
 }
 
