@@ -178,8 +178,9 @@ typedef struct vrg_frame_stats {
     uint64_t rays_any;         /* light any-hit queries issued */
     uint32_t error_flags;      /* device-side error word (stack overflow etc.) */
     uint32_t reserved;
-    float ms_trace[8];         /* per bounce: k_trace, from the end of the stage before */
-    float ms_shade[8];         /* per bounce: k_shade, from the end of k_trace */
+    float ms_trace[8];         /* per bounce: k_trace, from the end of the stage before (waits for
+                                  an earlier light-pdf walk included) */
+    float ms_shade[8];         /* per bounce: k_shade, from the end of k_trace to its own */
     float ms_anyhit[8];        /* per bounce: the light-pdf walk (k_anyhit, k_hit_eval,
                                   k_hit_sum) on its stream */
     uint64_t nodes_visited;    /* closest-hit traversal: 4-wide inner nodes fetched (128 B each) */

@@ -1054,9 +1054,9 @@ __global__ void __launch_bounds__(128, 8) k_shade(const __grid_constant__ FrameA
                     make_float4(new_d.x, new_d.y, new_d.z, pdf));
             }
         }
-        // (the end of the CTA's first warp; behind the loop the same stamp made
-        // every shading 1% slower, written or not)
-        if (threadIdx.x == 0 && n_in - base <= warps * span) stamp_end(a, ST_SHADED + b);
+        // (the warp's end; behind the loop the same stamp made every shading 1%
+        // slower, written or not)
+        if (lane == 0 && n_in - base <= warps * span) stamp_end(a, ST_SHADED + b);
         __syncwarp();
     }
 }
@@ -1333,7 +1333,9 @@ __global__ void __launch_bounds__(128) k_hit_sum(const __grid_constant__ FrameAr
         finish_job(a, b, p, a.ajob[b & 1][2 * (size_t)idx + 1].w, nee);
         if (CAPTURE) a.c_nee[(size_t)b * a.P + p] = nee;
     }
-    if (threadIdx.x == 0) stamp_end(a, ST_WALKED + b);
+    // (of the warps that had a job, and the first)
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((threadIdx.x & 31u) == 0 && (first < n || first == 0)) stamp_end(a, ST_WALKED + b);
 }
 
 }  // namespace

@@ -34,7 +34,7 @@ constexpr int FACE_ROW = 4;
 // The frame's stage times, written by its kernels: u64 nanoseconds of the
 // device's global timer from word CNT_STAMP on (0: the stage did not run).
 // Starts are written by a kernel's first thread, ends are the latest of its
-// CTAs (of its CTAs' first warps in the shading and k_hit_sum; 0 for the
+// CTAs (of its warps that had work in the shading and k_hit_sum; 0 for the
 // shading of an empty queue).  About 20 timing events between the stages held
 // the frame up: with these times in their place a 64x64 frame with stats went
 // from 129 to 106 us, a 640x480 one from 287 to 260.
