@@ -1878,7 +1878,7 @@ VRG_API vrg_status vrg_renderer_autotune(vrg_renderer *r, vrg_scene *scene, cons
         uint32_t vrg_tuning::*m;
         std::vector<uint32_t> cand;
     };
-    const std::vector<Field> fields = {
+    std::vector<Field> fields = {
         {&vrg_tuning::trace_refill, refills},
         {&vrg_tuning::trace_blocks_per_sm, bpsm_candidates(occ[0])},
         {&vrg_tuning::shade_blocks_per_sm, bpsm_candidates(occ[1])},
@@ -1886,7 +1886,9 @@ VRG_API vrg_status vrg_renderer_autotune(vrg_renderer *r, vrg_scene *scene, cons
         {&vrg_tuning::anyhit_blocks_per_sm, bpsm_candidates(occ[2])},
         {&vrg_tuning::stream_block, {64, 128, 256}},
     };
-    vrg_tuning cur = effective_tuning(r, r->tune, !(params->flags & (VRG_RENDER_CAPTURE | VRG_RENDER_CACHE)));
+    vrg_tuning cur = effective_tuning(r, r->tune, true);
+    for (Field &fd : fields)  // (the search can return to where it began)
+        if (std::find(fd.cand.begin(), fd.cand.end(), cur.*(fd.m)) == fd.cand.end()) fd.cand.push_back(cur.*(fd.m));
     float cur_ms = 0.0f;
     vrg_status st = measure(cur, &cur_ms);
     for (int pass = 0; pass < 2 && st == VRG_OK; pass++) {
