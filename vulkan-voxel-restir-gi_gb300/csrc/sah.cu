@@ -36,7 +36,6 @@ struct Item {
 
 constexpr int TREE_THREADS = 512, TREE_WARPS = TREE_THREADS / 32;
 constexpr uint32_t TREE_BIG = 256;   // prims above which the whole CTA splits a node
-constexpr uint32_t TREE_ONE_WAVE = 152;  // trees of one launch: an SM each
 constexpr uint32_t TREE_MAX = 2560;  // prims of a tree one CTA builds (its arrays fill an SM's shared memory)
 constexpr int SAH_WARPS = 8;
 constexpr int NB = 32;
@@ -753,7 +752,7 @@ vrg_status sah_build(Context *ctx, std::vector<SahTree> &trees, uint32_t total_p
     for (uint32_t a = n_large; a < nt && trees[a].n;) {
         uint32_t b = a;
         const uint32_t n = trees[a].n;
-        while (b < nt && trees[b].n && (nt - n_large <= TREE_ONE_WAVE || 2 * trees[b].n > n)) b++;
+        while (b < nt && trees[b].n && (nt - n_large <= (uint32_t)ctx->num_sms || 2 * trees[b].n > n)) b++;
         k_sah_tree<<<b - a, TREE_THREADS, tree_smem(n), s>>>(d_trees + a, in, out, arrive, lv_dev);
         VRG_CUDA_TRY(cudaGetLastError());
         a = b;
@@ -899,16 +898,11 @@ extern "C" VRG_API vrg_status vrg_build_tl_bvh_noalloc(const float *aabbs, const
         uint32_t *arrive = (uint32_t *)(B + NOALLOC_OFF_ARRIVE);
         uint32_t *leaf = (uint32_t *)(B + NOALLOC_OFF_LEAF);
         const uint32_t n_nodes = 2 * n - 1;
-        // the array keeps the previous call's contents: reset what must start at zero
-        VRG_CUDA_TRY(cudaMemsetAsync(arrive, 0, (size_t)n_nodes * 4, s));
-        VRG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 256, s));
         // tree descriptor and root work item: copies of host stack values
         SahTree tree{n, 0, 0, SAH_POWER};
         Item root{0, 0, 1, 0, n, INVALID};
         uint32_t one = 1;
         VRG_CUDA_TRY(cudaMemcpyAsync(d_tree, &tree, sizeof(tree), cudaMemcpyHostToDevice, s));
-        VRG_CUDA_TRY(cudaMemcpyAsync(q0, &root, sizeof(root), cudaMemcpyHostToDevice, s));
-        VRG_CUDA_TRY(cudaMemcpyAsync(cnt, &one, 4, cudaMemcpyHostToDevice, s));
         k_noalloc_prep<<<(n + 255) / 256, 256, 0, s>>>(aabbs, power, n, lo, hi, cen);
         VRG_CUDA_TRY(cudaGetLastError());
         SahInputs in{lo, hi, cen, ids};
@@ -920,6 +914,12 @@ extern "C" VRG_API vrg_status vrg_build_tl_bvh_noalloc(const float *aabbs, const
             VRG_CUDA_TRY(cudaStreamSynchronize(s));
             return VRG_OK;
         }
+        // the array keeps the previous call's contents: reset what must start at
+        // zero (k_sah_tree resets its own)
+        VRG_CUDA_TRY(cudaMemsetAsync(arrive, 0, (size_t)n_nodes * 4, s));
+        VRG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 256, s));
+        VRG_CUDA_TRY(cudaMemcpyAsync(q0, &root, sizeof(root), cudaMemcpyHostToDevice, s));
+        VRG_CUDA_TRY(cudaMemcpyAsync(cnt, &one, 4, cudaMemcpyHostToDevice, s));
         k_perm_init<<<dim3(std::max(1u, (n + 255) / 256), 1), 256, 0, s>>>(d_tree, prim_order);
         VRG_CUDA_TRY(cudaGetLastError());
         uint32_t n_cur = 1, cur_slot = 0, lv = 0;
