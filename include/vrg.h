@@ -485,9 +485,10 @@ VRG_API vrg_status vrg_build_bl_bvh_batched(vrg_context *ctx, uint32_t count, co
  * (cudaGetSymbolAddress, which allocates nothing).  Every call shares the
  * array: calls that overlap on the GPU (other threads or streams) race and
  * must be serialized by the caller.  The call copies small host values to
- * the device, synchronizes `stream` once per BVH level (it reads each
- * level's work count back to the host) and returns after the build has
- * finished on `stream`; an error return also synchronizes `stream` first. */
+ * the device and returns after the build has finished on `stream`: up to 2560
+ * prims are one launch and one synchronization, more synchronize `stream` once
+ * per BVH level (each level's work count is read back to the host).  An error
+ * return also synchronizes `stream` first. */
 VRG_API vrg_status vrg_build_tl_bvh_noalloc(const float *aabbs, const float *power, const uint32_t *ids,
                                             uint32_t n, vrg_bvh_node *nodes, uint32_t *prim_order, void *stream);
 

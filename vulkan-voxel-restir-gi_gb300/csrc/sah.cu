@@ -9,18 +9,21 @@
 // `base` puts its left child at base, its right child at base+1, the left
 // child's children at base+2 and the right child's at base + 2*n_left (a
 // subtree of k leaves has 2k-1 nodes).  This builder runs the recursion
-// level by level over all trees of a batch at once, one warp per node,
-// carrying (node index, children base) so the node array comes out in the
-// reference's order without a renumbering pass.
+// level by level, carrying (node index, children base) so the node array comes
+// out in the reference's order without a renumbering pass: trees of up to
+// TREE_MAX prims by one CTA each, all levels in one launch (k_sah_tree), larger
+// ones in a launch per level over all of them (k_sah_level).
 //
-// Per node the warp: reduces the node AABB and centroid bounds
-// (order-independent min/max), bins prims per axis with shared-memory atomic
-// counts and ordered-integer atomic min/max (exact), evaluates the 93 plane
-// costs with the reference's float expression, takes the first minimum in
-// (axis, plane) order, and partitions the node's slice with a warp-parallel
-// two-sided (Hoare) pass: the k-th predicate-false element from the left is
-// swapped with the k-th predicate-true element from the right, the pairing
-// of the serial two-pointer partition.
+// A node is split by a warp, the largest of a CTA's tree by the whole CTA: it
+// reduces the node AABB and centroid bounds (order-independent min/max), bins
+// prims per axis with shared-memory atomic counts and ordered-integer atomic
+// min/max (exact), evaluates the 93 plane costs with the reference's float
+// expression, takes the first minimum in (axis, plane) order, and partitions
+// the node's slice in a parallel two-sided (Hoare) pass: the k-th
+// predicate-false element from the left is swapped with the k-th predicate-true
+// element from the right, the pairing of the serial two-pointer partition.  A
+// node of up to SMALL_NODE prims takes its plane costs from the prims' boxes,
+// without bins.
 #include <algorithm>
 #include <cfloat>
 

@@ -14,7 +14,7 @@
 //     conservative) and child references (>= 0 node, < 0 ~record), with
 //     top-level leaves linked straight to the object's BLAS root; and
 //     16-byte world-space records per surface block / light triangle;
-//   * the light any-hit layout: a 2-wide world-space BVH over lamp blocks.
+//   * the light any-hit layout: a 4-wide world-space BVH over lamp blocks.
 // Several scenes commit together with one SAH build for all their top-level
 // trees and one for all their lamp trees.
 #include <algorithm>
@@ -574,9 +574,9 @@ vrg_status standalone_sah(Context *ctx, bool tri, uint32_t count, const uint32_t
 // ---- scene commit ----------------------------------------------------------
 //
 // Several scenes commit together: their top-level trees (light and geometry)
-// are built by ONE level-synchronous SAH build, and so are their lamp-block
-// trees, so the per-level host round trips of the builder are paid once per
-// commit, not once per scene.  Each scene's result is the same as a commit of
+// are built by ONE SAH build, and so are their lamp-block trees, so the
+// builder's launches and waits are paid once per commit, not once per scene.
+// Each scene's result is the same as a commit of
 // that scene alone (the builder's trees are independent).
 //
 // The light any-hit walk (nee_pdf's candidate enumeration) runs over a
