@@ -904,6 +904,7 @@ static vrg_status ensure_capture(vrg_renderer *r) {
     DevBufPtr b;
     VRG_TRY(dev_alloc(r->ctx->stream, floats * 4, b));
     float *f = (float *)b->ptr;
+    r->c_hit = (uint32_t *)f; f += nb * P * 4;  // first: written 16 bytes at a time
     r->c_origin = f; f += (nb + 1) * P * 3;
     r->c_dir = f; f += (nb + 1) * P * 3;
     r->c_normal = f; f += nb * P * 3;
@@ -913,8 +914,7 @@ static vrg_status ensure_capture(vrg_renderer *r) {
     r->c_mis = f; f += nb * P;
     r->c_pdf = f; f += nb * P;
     r->c_nee = f; f += nb * P;
-    r->c_q = f; f += nb * P;
-    r->c_hit = (uint32_t *)f;
+    r->c_q = f;
     VRG_CUDA_TRY(cudaMemsetAsync(b->ptr, 0, floats * 4, r->ctx->stream));
     r->cap = b;
     return VRG_OK;
